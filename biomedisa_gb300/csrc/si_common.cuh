@@ -33,11 +33,8 @@ __device__ __forceinline__ U4 philox4x32_10(U4 c, uint32_t k0, uint32_t k1) {
       k0 += kPhiloxW0;
       k1 += kPhiloxW1;
     }
-    const uint32_t hi0 = __umulhi(kPhiloxM0, c.x);
-    const uint32_t lo0 = kPhiloxM0 * c.x;
-    const uint32_t hi1 = __umulhi(kPhiloxM1, c.z);
-    const uint32_t lo1 = kPhiloxM1 * c.z;
-    c = U4{hi1 ^ c.y ^ k0, lo1, hi0 ^ c.w ^ k1, lo0};
+    const uint64_t m0 = (uint64_t)kPhiloxM0 * c.x, m1 = (uint64_t)kPhiloxM1 * c.z;
+    c = U4{(uint32_t)(m1 >> 32) ^ c.y ^ k0, (uint32_t)m1, (uint32_t)(m0 >> 32) ^ c.w ^ k1, (uint32_t)m0};
   }
   return c;
 }
@@ -174,14 +171,19 @@ __device__ __forceinline__ uint64_t f2_negzero() {
 // Packed product RN(a*b) that is never fused into a later sum; nz = f2_negzero().
 __device__ __forceinline__ uint64_t f2_mul(uint64_t a, uint64_t b, uint64_t nz) { return f2_fma(a, b, nz); }
 
-// Weights of the two neighbours whose (B - I) differences are the lanes of d;
-// cc = {c, c}. Returns w_lo, w_hi equal to edge_weight(d_lo^2, c) and
-// edge_weight(d_hi^2, c).
-__device__ __forceinline__ void edge_weight_pair(uint64_t d, uint64_t cc, uint64_t nz, float& w_lo, float& w_hi) {
+// Weights of the two neighbours whose (B - I) differences are the lanes of d,
+// before the flush at kWeightYMax; cc = {c, c}; y_lo, y_hi receive d^2 * c.
+// edge_weight's operations but for one sign: r = magic - y holds -k where
+// magic + y holds k (the sum and the difference round alike: magic is even and
+// rounding is to the nearest even integer), so that the exponent field is
+// raised by bits(r) << 23 in one shift-and-add ((bits(magic) << 23) vanishes
+// modulo 2^32). Values with y >= kWeightYMax are meaningless.
+__device__ __forceinline__ void edge_weight_pair_raw(uint64_t d, uint64_t cc, uint64_t nz, float& w_lo, float& w_hi,
+                                                     float& y_lo, float& y_hi) {
   const uint64_t magic2 = f2_splat(kRoundMagic);
   const uint64_t y = f2_mul(f2_mul(d, d, nz), cc, nz);
-  const uint64_t r = f2_add(y, magic2);
-  const uint64_t g = f2_sub(f2_sub(r, magic2), y);
+  const uint64_t r = f2_sub(magic2, y);
+  const uint64_t g = f2_sub(f2_sub(magic2, r), y);
   uint64_t p = f2_fma(f2_splat(kP5), g, f2_splat(kP4));
   p = f2_fma(p, g, f2_splat(kP3));
   p = f2_fma(p, g, f2_splat(kP2));
@@ -190,12 +192,32 @@ __device__ __forceinline__ void edge_weight_pair(uint64_t d, uint64_t cc, uint64
   uint32_t p_lo, p_hi, r_lo, r_hi;
   u2_unpack(p, p_lo, p_hi);
   u2_unpack(r, r_lo, r_hi);
-  float y_lo, y_hi;
   f2_unpack(y, y_lo, y_hi);
-  // 2^-k through the exponent field: k = bits(r) - bits(1.5*2^23), and
-  // (bits(1.5*2^23) << 23) vanishes modulo 2^32, so k << 23 == bits(r) << 23.
-  w_lo = y_lo < kWeightYMax ? __uint_as_float(p_lo - (r_lo << 23)) : 0.0f;
-  w_hi = y_hi < kWeightYMax ? __uint_as_float(p_hi - (r_hi << 23)) : 0.0f;
+  w_lo = __uint_as_float(p_lo + (r_lo << 23));
+  w_hi = __uint_as_float(p_hi + (r_hi << 23));
+}
+
+// Largest of three; NaN when one is.
+__device__ __forceinline__ float max3_nan(float a, float b, float c) {
+  float r;
+  asm("max.NaN.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
+}
+
+// The six weights of a step from the differences (+z, -z), (+y, -y), (+x, -x);
+// w[k] equals edge_weight(d_k^2, c). The flush to zero is taken out of line:
+// two tests of the largest y (a NaN is flushed too), because few neighbours differ from the seed by so
+// much (instructions bound the walker: 6 selects and compares less per step).
+__device__ __forceinline__ void edge_weights(uint64_t dz, uint64_t dy, uint64_t dx, uint64_t cc, uint64_t nz,
+                                             float (&w)[6]) {
+  float y[6];
+  edge_weight_pair_raw(dz, cc, nz, w[0], w[1], y[0], y[1]);
+  edge_weight_pair_raw(dy, cc, nz, w[2], w[3], y[2], y[3]);
+  edge_weight_pair_raw(dx, cc, nz, w[4], w[5], y[4], y[5]);
+  if (!(max3_nan(y[0], y[1], y[2]) < kWeightYMax && max3_nan(y[3], y[4], y[5]) < kWeightYMax)) {
+#pragma unroll
+    for (int k = 0; k < 6; ++k) w[k] = y[k] < kWeightYMax ? w[k] : 0.0f;
+  }
 }
 
 // Per-seed weight constant c = RN(RN(1 / RN(2 var)) * log2e).
@@ -203,6 +225,26 @@ __device__ __forceinline__ float weight_constant(float var) {
   const float div1 = __fdiv_rn(1.0f, __fmul_rn(2.0f, var));
   return __fmul_rn(div1, kLog2e);
 }
+
+// Division of any 32-bit n by a fixed d > 0 with one high product (Granlund
+// and Montgomery, "Division by invariant integers using multiplication", PLDI
+// 1994, figure 4.1): the sort's keys take five divisions per walker, which as
+// divisions by variables were most of its instructions.
+struct FastDiv {
+  uint32_t m, s1, s2;
+  FastDiv() = default;
+  __host__ explicit FastDiv(uint32_t d) {
+    uint32_t l = 0;
+    while (l < 32u && (1ull << l) < d) ++l;
+    m = (uint32_t)(((1ull << 32) * ((1ull << l) - d)) / d + 1u);
+    s1 = l < 1u ? l : 1u;
+    s2 = l ? l - 1u : 0u;
+  }
+  __device__ __forceinline__ uint32_t operator()(uint32_t n) const {
+    const uint32_t t = __umulhi(m, n);
+    return (t + ((n - t) >> s1)) >> s2;
+  }
+};
 
 // ---------------------------------------------------------------------------
 // One walker start point. pos is the linear index in the working (cropped,
@@ -259,10 +301,9 @@ __device__ __forceinline__ WalkRec<true> load_rec<true>(const void* __restrict__
 // One step from voxel pos, whose record is rec, with the uniform variate u in
 // [0, 1) given.
 template <bool kFloat>
-__device__ __forceinline__ uint32_t step_from_rec(const WalkRec<kFloat>& rec, uint32_t pos, float u, float c,
-                                                  float bf, float b23, uint32_t* __restrict__ hl,
-                                                  const int32_t* s_delta, uint64_t nz) {
-  float w0, w1, w2, w3, w4, w5;
+__device__ __forceinline__ uint32_t move_from_rec(const WalkRec<kFloat>& rec, uint32_t pos, float u, float c,
+                                                  float bf, float b23, const int32_t* s_delta, uint64_t nz) {
+  float w[6];
   uint32_t mask;
   // The (B - I) differences are formed pairwise (+z,-z), (+y,-y), (+x,-x) and
   // weighted on the packed pipe; d = B - I is exact in both record kinds
@@ -270,31 +311,35 @@ __device__ __forceinline__ uint32_t step_from_rec(const WalkRec<kFloat>& rec, ui
   const uint64_t cc = f2_splat(c);
   if constexpr (kFloat) {
     const uint64_t bf2 = f2_splat(bf);
-    edge_weight_pair(f2_sub(bf2, f2_pack(rec.a.x, rec.a.y)), cc, nz, w0, w1);
-    edge_weight_pair(f2_sub(bf2, f2_pack(rec.a.z, rec.a.w)), cc, nz, w2, w3);
-    edge_weight_pair(f2_sub(bf2, f2_pack(rec.b.x, rec.b.y)), cc, nz, w4, w5);
+    edge_weights(f2_sub(bf2, f2_pack(rec.a.x, rec.a.y)), f2_sub(bf2, f2_pack(rec.a.z, rec.a.w)),
+                 f2_sub(bf2, f2_pack(rec.b.x, rec.b.y)), cc, nz, w);
     mask = __float_as_uint(rec.b.z);
   } else {
     const uint2 r = rec.r;
     const uint64_t b2 = f2_splat(b23);
-    edge_weight_pair(f2_sub(b2, f2_pack(byte_plus_2p23(r.x, 0), byte_plus_2p23(r.x, 1))), cc, nz, w0, w1);
-    edge_weight_pair(f2_sub(b2, f2_pack(byte_plus_2p23(r.x, 2), byte_plus_2p23(r.x, 3))), cc, nz, w2, w3);
-    edge_weight_pair(f2_sub(b2, f2_pack(byte_plus_2p23(r.y, 0), byte_plus_2p23(r.y, 1))), cc, nz, w4, w5);
+    edge_weights(f2_sub(b2, f2_pack(byte_plus_2p23(r.x, 0), byte_plus_2p23(r.x, 1))),
+                 f2_sub(b2, f2_pack(byte_plus_2p23(r.x, 2), byte_plus_2p23(r.x, 3))),
+                 f2_sub(b2, f2_pack(byte_plus_2p23(r.y, 0), byte_plus_2p23(r.y, 1))), cc, nz, w);
     mask = r.y >> 16;
   }
-  const float c1 = __fadd_rn(w0, w1);
-  const float c2 = __fadd_rn(c1, w2);
-  const float c3 = __fadd_rn(c2, w3);
-  const float c4 = __fadd_rn(c3, w4);
-  const float c5 = __fadd_rn(c4, w5);
+  const float c1 = __fadd_rn(w[0], w[1]);
+  const float c2 = __fadd_rn(c1, w[2]);
+  const float c3 = __fadd_rn(c2, w[3]);
+  const float c4 = __fadd_rn(c3, w[4]);
+  const float c5 = __fadd_rn(c4, w[5]);
   const float rnd = __fmul_rn(c5, u);
-  int dir = (int)(w0 <= rnd) + (int)(c1 <= rnd) + (int)(c2 <= rnd) + (int)(c3 <= rnd) + (int)(c4 <= rnd);
+  int dir = (int)(w[0] <= rnd) + (int)(c1 <= rnd) + (int)(c2 <= rnd) + (int)(c3 <= rnd) + (int)(c4 <= rnd);
   if (rnd == 0.0f) dir = 0;
-  if (!((mask >> dir) & 1u)) {
-    pos += (uint32_t)s_delta[dir];
-    atomicAdd(&hl[pos], 1u);
-  }
-  return pos;
+  return (mask >> dir) & 1u ? pos : pos + (uint32_t)s_delta[dir];
+}
+
+template <bool kFloat>
+__device__ __forceinline__ uint32_t step_from_rec(const WalkRec<kFloat>& rec, uint32_t pos, float u, float c,
+                                                  float bf, float b23, uint32_t* __restrict__ hl,
+                                                  const int32_t* s_delta, uint64_t nz) {
+  const uint32_t to = move_from_rec<kFloat>(rec, pos, u, c, bf, b23, s_delta, nz);
+  if (to != pos) atomicAdd(&hl[to], 1u);
+  return to;
 }
 
 // One step with the uniform variate u in [0, 1) given.
@@ -374,7 +419,17 @@ __device__ __forceinline__ void walk_steps_multi(const void* __restrict__ packed
     n = min(n, W[w].t_end - W[w].t);
   }
   if ((any_t & 3u) == 0u) {
-    n &= ~3u;
+    // a hit waits until the walker is somewhere else two steps later, and is
+    // then added with its returns: hit atomics bound the sweeps, and every fifth
+    // to sixth hit or so is a return. held/cnt: the two voxels (even, odd steps)
+    // and their counts, 16 bits each.
+    n = min(n, 0xFFFFu) & ~3u;
+    uint32_t held[N][2], cnt[N];
+#pragma unroll
+    for (int w = 0; w < N; ++w) {
+      held[w][0] = held[w][1] = W[w].pos;
+      cnt[w] = 0u;
+    }
     for (uint32_t k = 0; k < n; k += 4u) {
       U4 r[N];
 #pragma unroll
@@ -385,12 +440,26 @@ __device__ __forceinline__ void walk_steps_multi(const void* __restrict__ packed
 #pragma unroll
         for (int w = 0; w < N; ++w) q[w] = load_rec<kFloat>(packed_v, W[w].pos);
 #pragma unroll
-        for (int w = 0; w < N; ++w)
-          W[w].pos = step_from_rec<kFloat>(q[w], W[w].pos, u01_from_bits(philox_word(r[w], j)), W[w].c, W[w].bf,
-                                           W[w].b23, W[w].hl, s_delta, nz);
+        for (int w = 0; w < N; ++w) {
+          const uint32_t to = move_from_rec<kFloat>(q[w], W[w].pos, u01_from_bits(philox_word(r[w], j)), W[w].c,
+                                                    W[w].bf, W[w].b23, s_delta, nz);
+          const bool hit = to != W[w].pos;
+          if (hit && to != held[w][j & 1]) {
+            atomicAdd(&W[w].hl[held[w][j & 1]], j & 1 ? cnt[w] >> 16 : cnt[w] & 0xFFFFu);
+            held[w][j & 1] = to;
+            cnt[w] &= j & 1 ? 0xFFFFu : 0xFFFF0000u;
+          }
+          if (hit) cnt[w] += j & 1 ? 0x10000u : 1u;
+          W[w].pos = to;
+        }
       }
 #pragma unroll
       for (int w = 0; w < N; ++w) W[w].t += 4u;
+    }
+#pragma unroll
+    for (int w = 0; w < N; ++w) {
+      if (cnt[w] & 0xFFFFu) atomicAdd(&W[w].hl[held[w][0]], cnt[w] & 0xFFFFu);
+      if (cnt[w] >> 16) atomicAdd(&W[w].hl[held[w][1]], cnt[w] >> 16);
     }
   }
 #pragma unroll

@@ -1,0 +1,78 @@
+"""Sorted sweeps where their kernels can go wrong: hits held back over two steps
+(voxels next to the border, where moves are refused; sweeps longer than the
+held counts' 16 bits; walks that are not multiples of four steps), the flush of
+small weights (strong edges, variance one, values that are not numbers), the
+one-launch and the three-launch scan at the edges of their ranges, few and many
+walks. Hit maps equal the oracle's bit for bit."""
+import numpy as np
+import pytest
+
+import oracle as O
+from biomedisa_gb300 import _native as nat
+from biomedisa_gb300 import smart_interpolation, smart_interpolation_batch
+
+pytestmark = pytest.mark.gpu
+
+
+def _volume(shape, seed, every=3, noise=14.0):
+    rng = np.random.default_rng(seed)
+    truth = np.ones(shape, np.int32)
+    truth[:, shape[1] // 2:] = 2
+    img = rng.normal(70 + 60 * (truth == 2), noise).clip(0, 255).astype(np.uint8)
+    lab = np.zeros(shape, np.int32)
+    lab[::every] = truth[::every]
+    return img, lab
+
+
+@pytest.mark.parametrize("dtype", [np.uint8, np.float32], ids=["u8", "f32"])
+@pytest.mark.parametrize("shape,nbrw,sorw,sweep", [
+    ((3, 3, 3), 4, 37, 0),          # one interior voxel behind refused moves on every side
+    ((1, 5, 9), 3, 64, 0),          # a crop of three planes
+    ((14, 17, 19), 2, 1001, 0),     # a walk of 1001 steps: default sweeps of 128, unaligned second walk
+    ((9, 12, 11), 1, 999, 5),       # short sweeps
+    ((8, 9, 10), 1, 140_001, 140_001),  # one sweep, more steps than a held count holds
+], ids=str)
+def test_held_hits_equal_oracle(shape, nbrw, sorw, sweep, dtype, cuda):
+    img, lab = _volume(shape, sum(shape))
+    kw = dict(nbrw=nbrw, sorw=sorw, return_hits=True)
+    got = smart_interpolation(img.astype(dtype), lab, rng_seed=23, sweep_steps=sweep, **kw)
+    exp = O.smart_interpolation(img.astype(dtype), lab, key=23, **kw)
+    assert np.array_equal(got["hits"], exp["hits"]) and np.array_equal(got["regular"], exp["regular"])
+
+
+@pytest.mark.parametrize("noise", [0.0, 0.6, 40.0])
+def test_small_weights_equal_oracle(noise, cuda):
+    """Differences on both sides of the flush at d^2 c = 125."""
+    img, lab = _volume((20, 24, 22), 3, 4, noise)
+    img[:, ::3, ::5] = 255
+    kw = dict(nbrw=6, sorw=130, return_hits=True)
+    got = smart_interpolation(img, lab, rng_seed=2, **kw)
+    exp = O.smart_interpolation(img, lab, key=2, **kw)
+    assert np.array_equal(got["hits"], exp["hits"])
+
+
+@pytest.mark.parametrize("edge,device_loop", [(1, 1), (1, 0), (2, 1), (3, 0)], ids=str)
+def test_scans_of_few_and_many_buckets(edge, device_loop, cuda):
+    """29,406 (three launches), 4,095 (one launch, its tile one short) and 1,350
+    buckets of three labels over a 26 x 29 x 13 crop."""
+    img, lab = _volume((24, 27, 11), 6, 4)
+    kw = dict(nbrw=5, sorw=200, return_hits=True)
+    nat.call("si_walk_sorted_set_loop", device_loop)
+    try:
+        got = smart_interpolation(img, lab, rng_seed=5, sort_edge=edge, **kw)
+    finally:
+        nat.call("si_walk_sorted_set_loop", 1)
+    exp = O.smart_interpolation(img, lab, key=5, **kw)
+    assert np.array_equal(got["hits"], exp["hits"])
+
+
+def test_many_walks_in_one_sweep(cuda):
+    """More walks than small launches take, single and batched."""
+    img, lab = _volume((21, 60, 58), 8, 2)
+    kw = dict(nbrw=16, sorw=60, return_hits=True)  # 11 slices, 562 thousand walks
+    exp = O.smart_interpolation(img, lab, key=9, **kw)
+    got = smart_interpolation(img, lab, rng_seed=9, **kw)
+    both = smart_interpolation_batch([img, img.astype(np.uint16)], [lab, lab], rng_seed=9, autotune_params=False, **kw)
+    assert np.array_equal(got["hits"], exp["hits"]) and np.array_equal(both[0]["hits"], exp["hits"])
+    exp16 = O.smart_interpolation(img.astype(np.uint16), lab, key=9, **kw)
+    assert np.array_equal(both[1]["hits"], exp16["hits"])
