@@ -4,7 +4,7 @@ The walker's results do not depend on these parameters (integer hit sums), only
 its speed does: the sort-brick edge (walkers are bucketed by label and brick of
 edge^3 voxels between sweeps) and the sweep length (steps per sweep launch).
 The tuner times every candidate on the caller's own volumes with shortened
-walks (4 sweeps of every walk), keeps the fastest, and caches the choice per
+walks (2 sweeps of every walk), keeps the fastest, and caches the choice per
 workload signature in a JSON file ($SI_AUTOTUNE_CACHE or
 ~/.cache/biomedisa_gb300/autotune.json).
 """
@@ -22,7 +22,7 @@ import torch
 
 from . import _native as nat
 
-CANDIDATES = ((6, 32), (8, 32), (4, 32), (6, 24), (6, 48), (10, 32))
+CANDIDATES = ((6, 128), (8, 128), (6, 96), (6, 64))
 
 
 def cache_path() -> Path:
@@ -31,11 +31,12 @@ def cache_path() -> Path:
 
 
 def signature(vols, nbrw: int, sorw: int, walks: int) -> str:
-    """Workload class: device, record kind, walk counts and sizes (log2 bins)."""
+    """Workload class: device, candidates, record kind, walk counts and sizes
+    (log2 bins)."""
     dev = torch.cuda.get_device_name()
     kinds = sorted({int(v.work_is_float) for v in vols})
     vox = sum(v.Zc * v.Yc * v.Xc for v in vols)
-    return json.dumps([dev, kinds, len(vols), nbrw, sorw, int(math.log2(max(walks, 1))),
+    return json.dumps([dev, CANDIDATES, kinds, len(vols), nbrw, sorw, int(math.log2(max(walks, 1))),
                        int(math.log2(max(vox, 1)))])
 
 
@@ -88,7 +89,7 @@ def tune(vol_array, n_vols: int, hits: list, nbrw: int, sorw: int, key: int, wal
     stream = torch.cuda.current_stream()
     results = []
     for edge, steps in CANDIDATES:
-        probe = min(sorw, 4 * steps)
+        probe = min(sorw, 2 * steps)
         need = ctypes.c_ulonglong(0)
         nat.call("si_walk_sorted_batch_scratch", vol_array, n_vols, nbrw, edge, ctypes.byref(need))
         scratch = torch.empty(max(int(need.value), 1), dtype=torch.uint8, device="cuda")

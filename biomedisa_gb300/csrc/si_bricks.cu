@@ -39,6 +39,15 @@ constexpr int kAdvThreads = 512;
 constexpr uint32_t kChunk = 4096;  // sorted walkers per work ticket
 constexpr int kScanBlock = 1024;   // elements per scan block (256 threads x 4)
 
+// Device counters of a sorted walk.
+enum WalkCtr {
+  kCtrLive = 0,    // walkers live after the last scan = states of the next sweep
+  kCtrIn = 1,      // states the next scatter reads
+  kCtrSweeps = 2,  // sweeps that ran
+  kCtrOver = 3,    // round limit hit with live walkers
+  kCtrWords = 4
+};
+
 struct BrickGeom {
   int Zc, Yc, Xc;
   int edge;  // brick edge used for bucketing
@@ -46,6 +55,7 @@ struct BrickGeom {
   uint32_t nb;   // bricks per label
   uint32_t F;    // Yc * Xc
   uint32_t Xp;   // record row pitch (even)
+  FastDiv by_F, by_X, by_edge;
 };
 
 // Walker state: x = position (crop linear index), y = seed index,
@@ -53,17 +63,17 @@ struct BrickGeom {
 __device__ __forceinline__ bool live(const uint4& s) { return s.z != (s.w & 0xFFFFFFu); }
 
 __device__ __forceinline__ void coords(const BrickGeom& g, uint32_t pos, int& z, int& y, int& x) {
-  z = (int)(pos / g.F);
+  z = (int)g.by_F(pos);
   const uint32_t r = pos - (uint32_t)z * g.F;
-  y = (int)(r / (uint32_t)g.Xc);
+  y = (int)g.by_X(r);
   x = (int)(r - (uint32_t)y * (uint32_t)g.Xc);
 }
 
 __device__ __forceinline__ uint32_t bucket_of(const BrickGeom& g, const uint4& s) {
   int z, y, x;
   coords(g, s.x, z, y, x);
-  const uint32_t e = (uint32_t)g.edge;
-  const uint32_t brick = ((uint32_t)z / e * g.nby + (uint32_t)y / e) * g.nbx + (uint32_t)x / e;
+  const uint32_t brick = (g.by_edge((uint32_t)z) * (uint32_t)g.nby + g.by_edge((uint32_t)y)) * (uint32_t)g.nbx +
+                         g.by_edge((uint32_t)x);
   return (s.w >> 24) * g.nb + brick;
 }
 
@@ -83,7 +93,8 @@ __device__ __forceinline__ bool fetch_state(uint64_t i, uint64_t n, const uint4*
 }
 
 // Count (kScatter = false) or scatter (true) live walkers into buckets, with
-// warp aggregation of equal keys.
+// warp aggregation of equal keys. Scatter: counts are cursors relative to
+// offsets, or absolute ones (offsets null).
 template <bool kFirst, bool kScatter>
 __global__ void __launch_bounds__(256) bucket_kernel(const uint4* __restrict__ states_in, uint64_t n,
                                                      const SeedRec* __restrict__ seeds, uint32_t ns, int sorw,
@@ -93,25 +104,34 @@ __global__ void __launch_bounds__(256) bucket_kernel(const uint4* __restrict__ s
                                                      const uint32_t* __restrict__ n_dev = nullptr) {
   if (n_dev) n = *n_dev;  // the count lives on the device (device-side sweep loop)
   const int lane = threadIdx.x & 31;
+  // four states a thread, so that their loads and cursor atomics overlap (a
+  // walker's load, atomic and store one after the other bound this pass)
+  constexpr int N = 4;
   const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-  for (uint64_t base = (uint64_t)blockIdx.x * blockDim.x + (threadIdx.x & ~31u); base < n; base += stride) {
-    uint4 s;
-    const bool ok = fetch_state<kFirst>(base + lane, n, states_in, seeds, ns, sorw, s);
-    const uint32_t key = ok ? bucket_of(g, s) : 0u;
-    const uint32_t act = __ballot_sync(0xffffffffu, ok);
-    if (ok) {
-      const uint32_t peers = __match_any_sync(act, key);
-      const int leader = __ffs(peers) - 1;
-      const uint32_t cnt = __popc(peers);
-      if (!kScatter) {
-        if (lane == leader) atomicAdd(&counts[key], cnt);
-      } else {
-        uint32_t b = 0;
-        if (lane == leader) b = atomicAdd(&counts[key], cnt);
-        b = __shfl_sync(peers, b, leader);
-        const uint32_t rank = __popc(peers & ((1u << lane) - 1u));
-        states_out[offsets[key] + b + rank] = s;
+  for (uint64_t base = (uint64_t)blockIdx.x * blockDim.x + (threadIdx.x & ~31u); base < n; base += N * stride) {
+    uint4 s[N];
+    bool ok[N];
+    uint32_t key[N], peers[N], at[N];
+#pragma unroll
+    for (int k = 0; k < N; ++k)
+      ok[k] = fetch_state<kFirst>(base + k * stride + lane, n, states_in, seeds, ns, sorw, s[k]);
+#pragma unroll
+    for (int k = 0; k < N; ++k) {
+      key[k] = ok[k] ? bucket_of(g, s[k]) : 0u;
+      const uint32_t act = __ballot_sync(0xffffffffu, ok[k]);
+      at[k] = peers[k] = 0u;
+      if (ok[k]) {
+        peers[k] = __match_any_sync(act, key[k]);
+        if (lane == __ffs(peers[k]) - 1) at[k] = atomicAdd(&counts[key[k]], (uint32_t)__popc(peers[k]));
       }
+    }
+    if (kScatter) {
+#pragma unroll
+      for (int k = 0; k < N; ++k)
+        if (ok[k]) {
+          const uint32_t b = __shfl_sync(peers[k], at[k], __ffs(peers[k]) - 1);
+          states_out[(offsets ? offsets[key[k]] : 0u) + b + __popc(peers[k] & ((1u << lane) - 1u))] = s[k];
+        }
     }
   }
 }
@@ -379,11 +399,11 @@ __global__ void __launch_bounds__(kAdvThreads, 4) brick_advance_kernel(
 // aggregation of equal keys; walkers of a warp come from few buckets).
 template <bool kFloat>
 __global__ void __launch_bounds__(256) sweep_kernel(const void* __restrict__ packed, BrickGeom g,
-                                                    uint4* __restrict__ states, uint32_t n_live, uint32_t K,
+                                                    uint4* __restrict__ states, uint32_t K,
                                                     const SeedRec* __restrict__ seeds, uint32_t k0, uint32_t k1,
                                                     uint32_t* __restrict__ hits, uint32_t* __restrict__ next_counts,
-                                                    const uint32_t* __restrict__ live_dev) {
-  if (live_dev) n_live = *live_dev;  // the count lives on the device (device-side sweep loop)
+                                                    const uint32_t* __restrict__ ctrs) {
+  const uint32_t n_live = ctrs[kCtrLive];
   __shared__ int32_t s_delta[6];
   if (threadIdx.x < 6) {
     const int32_t F = (int32_t)g.F, X = g.Xc;
@@ -429,11 +449,10 @@ __global__ void __launch_bounds__(256) sweep_kernel(const void* __restrict__ pac
 // kMinBlocks CTAs of kThreads per SM.
 template <bool kFloat, int N, int kThreads, int kMinBlocks>
 __global__ void __launch_bounds__(kThreads, kMinBlocks)
-    sweep_multi_kernel(const void* __restrict__ packed, BrickGeom g, uint4* __restrict__ states, uint32_t n_live,
-                       uint32_t K, const SeedRec* __restrict__ seeds, uint32_t k0, uint32_t k1,
-                       uint32_t* __restrict__ hits, uint32_t* __restrict__ next_counts,
-                       const uint32_t* __restrict__ live_dev) {
-  if (live_dev) n_live = *live_dev;  // the count lives on the device (device-side sweep loop)
+    sweep_multi_kernel(const void* __restrict__ packed, BrickGeom g, uint4* __restrict__ states, uint32_t K,
+                       const SeedRec* __restrict__ seeds, uint32_t k0, uint32_t k1, uint32_t* __restrict__ hits,
+                       uint32_t* __restrict__ next_counts, const uint32_t* __restrict__ ctrs) {
+  const uint32_t n_live = ctrs[kCtrLive];
   __shared__ int32_t s_delta[6];
   if (threadIdx.x < 6) {
     const int32_t F = (int32_t)g.F, X = g.Xc;
@@ -469,8 +488,8 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks)
           st[w] = states[idx];
           const SeedRec sd = seeds[st[w].y];
           te[w] = st[w].w & 0xFFFFFFu;
-          W[w] = pair_walker(st[w].x, st[w].z, min(st[w].z + K, te[w]), sd.c, sd.b, sd.pos, seed_axis(sd.meta),
-                             seed_label(sd.meta), hits + (size_t)(st[w].w >> 24) * V);
+          W[w] = pair_walker(st[w].x, st[w].z, min(st[w].z + K, te[w]), sd.c, sd.b, sd.pos,
+                             seed_axis(sd.meta), seed_label(sd.meta), hits + (size_t)(st[w].w >> 24) * V);
         }
       }
       walk_steps_multi<kFloat, N>(packed, W, k0, k1, s_delta, nz);
@@ -539,6 +558,9 @@ BrickGeom make_geom(int Zc, int Yc, int Xc, int edge = kCore) {
   g.nb = (uint32_t)g.nbz * g.nby * g.nbx;
   g.F = (uint32_t)Yc * Xc;
   g.Xp = (uint32_t)((Xc + 1) & ~1);
+  g.by_F = FastDiv(g.F);
+  g.by_X = FastDiv((uint32_t)Xc);
+  g.by_edge = FastDiv((uint32_t)edge);
   return g;
 }
 
@@ -683,33 +705,145 @@ namespace si {
 namespace {
 constexpr uint64_t kBatchWalks = 1ull << 25;  // default walks per seed range of si_walk_sorted
 constexpr int kSortEdge = 6;
+// Default sweep length: 32 steps, 128 for walks of kLongWalk steps and more.
+// Longer sweeps share the sort's cost among more steps, but let the walkers
+// spread further between sorts. Walks of 4000 steps, 48 / 64 / 96 / 128 / 256
+// steps a sweep: 128^3 44.4 / 43.2 / 42.0 / 41.4 / 42.0 ms, 419x492x462 873 /
+// 855 / 838 / 834 / 843 ms.
+constexpr int kLongWalk = 1000;
+int default_sweep_steps(int sorw) { return sorw >= kLongWalk ? 128 : 32; }
 std::atomic<unsigned long long> g_range_walks{0};  // 0 = kBatchWalks (si_walk_sorted_set_range)
 std::atomic<int> g_sweep_pairs{1};  // sweep kernel mode (si_walk_sorted_set_pairs)
 std::atomic<int> g_device_loop{1};  // 1: device-side sweep loop (si_walk_sorted_set_loop)
 std::atomic<unsigned long long> g_round_limit{0};  // 0 = kRoundLimit (si_walk_sorted_set_round_limit)
 constexpr uint64_t kRoundLimit = 1ull << 24;
-constexpr int kCtrWords = 8;
 
 uint32_t round_limit() {
   const unsigned long long v = g_round_limit.load(std::memory_order_relaxed);
   return (uint32_t)std::min<uint64_t>(v ? v : kRoundLimit, 0xFFFFFFFFull);
 }
 
-// After a sweep: the states the next scatter reads are the ones this sweep
-// advanced (ctrs[0] of the scan before it); ctrs[4] counts sweeps that ran.
-__global__ void round_shift_kernel(uint32_t* __restrict__ ctrs) {
-  const uint32_t live = ctrs[0];
-  ctrs[3] = live;
-  if (live) ctrs[4] += 1u;
+// ---------------------------------------------------------------------------
+// Scan of the sorted walkers' bucket sizes: offsets receives every bucket's
+// first place (the scatter's cursors), counts is zeroed as it is read (the
+// sweep adds the next round's sizes), the counters move on to the next round.
+// With the memsets and the counter update inside, a round is three launches
+// for up to kScanOne buckets and five above; it was eight.
+// ---------------------------------------------------------------------------
+struct ScanArgs {
+  uint32_t* counts;
+  uint32_t n;
+  uint32_t* offsets;
+  uint32_t* ctrs;
+  uint32_t limit;                    // most sweeps (round_limit)
+  int cond;                          // 1: set the loop condition
+  cudaGraphConditionalHandle handle;
+};
+
+__device__ __forceinline__ uint32_t warp_inclusive(uint32_t v) {
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t u = __shfl_up_sync(0xffffffffu, v, o);
+    if (lane >= o) v += u;
+  }
+  return v;
 }
 
-// End of a loop iteration: continue while walkers are live and fewer than
-// `limit` sweeps ran; reaching the limit with live walkers sets ctrs[5].
-__global__ void round_cond_kernel(uint32_t* __restrict__ ctrs, cudaGraphConditionalHandle h, uint32_t limit) {
-  const uint32_t live = ctrs[0];
-  const bool over = live != 0u && ctrs[4] >= limit;
-  if (over) ctrs[5] = 1u;
-  cudaGraphSetConditional(h, (live != 0u && !over) ? 1u : 0u);
+// Exclusive scan over the CTA's threads (whole warps, at most 1024 threads);
+// total receives the sum. Two barriers.
+__device__ __forceinline__ uint32_t cta_exclusive(uint32_t v, uint32_t* s_warp, uint32_t& total) {
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  const uint32_t incl = warp_inclusive(v);
+  if (lane == 31) s_warp[wid] = incl;
+  __syncthreads();
+  const uint32_t w = warp_inclusive(lane < nw ? s_warp[lane] : 0u);
+  total = __shfl_sync(0xffffffffu, w, 31);
+  const uint32_t before = __shfl_sync(0xffffffffu, w, wid ? wid - 1 : 0);
+  __syncthreads();
+  return (wid ? before : 0u) + incl - v;
+}
+
+__device__ __forceinline__ uint4 load_counts(const ScanArgs& a, uint32_t i0) {
+  if (i0 + 4u <= a.n) return *reinterpret_cast<const uint4*>(a.counts + i0);
+  uint4 v = make_uint4(0u, 0u, 0u, 0u);
+  if (i0 < a.n) v.x = a.counts[i0];
+  if (i0 + 1u < a.n) v.y = a.counts[i0 + 1u];
+  if (i0 + 2u < a.n) v.z = a.counts[i0 + 2u];
+  return v;
+}
+
+// Places four buckets from i0 (a multiple of 4; offsets and counts are padded
+// to one), whose predecessors hold `run` walkers.
+__device__ __forceinline__ void place_buckets(const ScanArgs& a, uint32_t i0, const uint4& v, uint32_t run) {
+  if (i0 >= a.n) return;
+  *reinterpret_cast<uint4*>(a.offsets + i0) = make_uint4(run, run + v.x, run + v.x + v.y, run + v.x + v.y + v.z);
+  *reinterpret_cast<uint4*>(a.counts + i0) = make_uint4(0u, 0u, 0u, 0u);
+}
+
+// The sweep that just ran had ctrs[kCtrLive] states; the next has `live`.
+__device__ __forceinline__ void next_round(const ScanArgs& a, uint32_t live) {
+  const uint32_t prev = a.ctrs[kCtrLive];
+  const uint32_t sweeps = a.ctrs[kCtrSweeps] + (prev ? 1u : 0u);
+  a.ctrs[kCtrIn] = prev;
+  a.ctrs[kCtrSweeps] = sweeps;
+  a.ctrs[kCtrLive] = live;
+  if (a.cond) {
+    const bool over = live != 0u && sweeps >= a.limit;
+    if (over) a.ctrs[kCtrOver] = 1u;
+    cudaGraphSetConditional(a.handle, (live != 0u && !over) ? 1u : 0u);
+  }
+}
+
+// The whole scan in one CTA. Above kScanOne buckets its serial tiles of 4096
+// (about 1 us each) cost more than the two launches it saves.
+constexpr uint32_t kScanOne = 16384;
+__global__ void __launch_bounds__(1024) walk_scan_one_kernel(ScanArgs a) {
+  __shared__ uint32_t s_warp[32];
+  uint32_t carry = 0;
+  uint4 v = load_counts(a, threadIdx.x * 4u);
+  for (uint32_t b0 = 0; b0 < a.n; b0 += 4096u) {
+    const uint32_t i0 = b0 + threadIdx.x * 4u;
+    const uint4 next = load_counts(a, i0 + 4096u);  // the next tile's counts on their way
+    uint32_t tile;
+    place_buckets(a, i0, v, carry + cta_exclusive(v.x + v.y + v.z + v.w, s_warp, tile));
+    carry += tile;
+    v = next;
+  }
+  if (threadIdx.x == 0) next_round(a, carry);
+}
+
+// Three launches for many buckets: sums of 1024 buckets a CTA, their scan, the
+// places.
+__global__ void __launch_bounds__(256) walk_scan_sums_kernel(ScanArgs a, uint32_t* __restrict__ sums) {
+  __shared__ uint32_t s_warp[32];
+  const uint4 v = load_counts(a, blockIdx.x * kScanBlock + threadIdx.x * 4u);
+  uint32_t total;
+  cta_exclusive(v.x + v.y + v.z + v.w, s_warp, total);
+  if (threadIdx.x == 0) sums[blockIdx.x] = total;
+}
+
+__global__ void __launch_bounds__(1024) walk_scan_top_kernel(ScanArgs a, uint32_t* __restrict__ sums,
+                                                             uint32_t nblocks) {
+  __shared__ uint32_t s_warp[32];
+  uint32_t carry = 0;
+  for (uint32_t b0 = 0; b0 < nblocks; b0 += 1024u) {
+    const uint32_t b = b0 + threadIdx.x;
+    const uint32_t v = b < nblocks ? sums[b] : 0u;
+    uint32_t tile;
+    const uint32_t run = carry + cta_exclusive(v, s_warp, tile);
+    if (b < nblocks) sums[b] = run;
+    carry += tile;
+  }
+  if (threadIdx.x == 0) next_round(a, carry);
+}
+
+__global__ void __launch_bounds__(256) walk_scan_place_kernel(ScanArgs a, const uint32_t* __restrict__ sums) {
+  __shared__ uint32_t s_warp[32];
+  const uint32_t i0 = blockIdx.x * kScanBlock + threadIdx.x * 4u;
+  const uint4 v = load_counts(a, i0);
+  uint32_t total;
+  place_buckets(a, i0, v, sums[blockIdx.x] + cta_exclusive(v.x + v.y + v.z + v.w, s_warp, total));
 }
 
 // A stream of this device for capturing loop bodies (never executes work).
@@ -769,31 +903,125 @@ uint64_t range_walks() {
   return v ? (uint64_t)v : kBatchWalks;
 }
 
+// Scratch of a sorted walk (byte offsets).
 struct SortLayout {
-  size_t states0, states1, counts, counts2, offsets, sums, ctrs, total;
+  size_t vols, states0, states1, counts, offsets, sums, ctrs, total;
 };
 
-SortLayout sort_layout(const BrickGeom& g, uint64_t max_walks, int nol) {
+SortLayout sort_layout(uint64_t nbt, uint64_t max_walks, size_t vol_bytes) {
   SortLayout L{};
-  const uint64_t nbt = (uint64_t)g.nb * nol;
   const uint64_t nblocks = (nbt + kScanBlock - 1) / kScanBlock;
   size_t off = 0;
+  L.vols = off;
+  off = align_up(off + vol_bytes, 256);
   L.states0 = off;
   off = align_up(off + max_walks * sizeof(uint4), 256);
   L.states1 = off;
   off = align_up(off + max_walks * sizeof(uint4), 256);
   L.counts = off;
-  off = align_up(off + (nbt + 1) * sizeof(uint32_t), 256);
-  L.counts2 = off;
-  off = align_up(off + (nbt + 1) * sizeof(uint32_t), 256);
+  off = align_up(off + nbt * sizeof(uint32_t), 256);
   L.offsets = off;
-  off = align_up(off + (nbt + 1) * sizeof(uint32_t), 256);
+  off = align_up(off + nbt * sizeof(uint32_t), 256);
   L.sums = off;
-  off = align_up(off + (nblocks + 1) * sizeof(uint32_t), 256);
+  off = align_up(off + nblocks * sizeof(uint32_t), 256);
   L.ctrs = off;
   off = align_up(off + kCtrWords * sizeof(uint32_t), 256);
   L.total = off;
   return L;
+}
+
+struct WalkBuffers {
+  uint4* states[2];
+  uint32_t *counts, *offsets, *sums, *ctrs;
+  uint32_t nbt, nblocks;
+};
+
+WalkBuffers walk_buffers(void* scratch, const SortLayout& L, uint32_t nbt) {
+  uint8_t* b = static_cast<uint8_t*>(scratch);
+  WalkBuffers w{};
+  w.states[0] = reinterpret_cast<uint4*>(b + L.states0);
+  w.states[1] = reinterpret_cast<uint4*>(b + L.states1);
+  w.counts = reinterpret_cast<uint32_t*>(b + L.counts);
+  w.offsets = reinterpret_cast<uint32_t*>(b + L.offsets);
+  w.sums = reinterpret_cast<uint32_t*>(b + L.sums);
+  w.ctrs = reinterpret_cast<uint32_t*>(b + L.ctrs);
+  w.nbt = nbt;
+  w.nblocks = (nbt + kScanBlock - 1) / kScanBlock;
+  return w;
+}
+
+void walk_scan(cudaStream_t s, const WalkBuffers& w, const ScanArgs& a) {
+  if (w.nbt <= kScanOne) {
+    walk_scan_one_kernel<<<1, 1024, 0, s>>>(a);
+    return;
+  }
+  walk_scan_sums_kernel<<<w.nblocks, 256, 0, s>>>(a, w.sums);
+  walk_scan_top_kernel<<<1, 1024, 0, s>>>(a, w.sums, w.nblocks);
+  walk_scan_place_kernel<<<w.nblocks, 256, 0, s>>>(a, w.sums);
+}
+
+// One range of walks from their start to their end. first(s): counts the
+// virtual walks; start(s, out): scatters them; scatter(s, in, out): the live
+// states of the last sweep into the sorted order; sweep(s, states): K steps of
+// every state, the live ones counted. Device loop: the executable graph it
+// launches is added to execs (destroy it after the stream has run it).
+template <class First, class Start, class Scatter, class Sweep>
+int run_range(cudaStream_t st, const WalkBuffers& w, ScanArgs a, bool device_loop, const char* what,
+              std::vector<cudaGraphExec_t>& execs, First first, Start start, Scatter scatter, Sweep sweep) {
+  a.cond = 0;
+  first(st);
+  walk_scan(st, w, a);
+  start(st, w.states[0]);
+  if (device_loop) {
+    sweep(st, w.states[0]);
+    walk_scan(st, w, a);
+    int rc = check_launch(what);
+    if (rc) return rc;
+    // two rounds per loop iteration: states[0] -> states[1] -> states[0]
+    cudaGraphExec_t exec = nullptr;
+    rc = build_while_graph(
+        [&](cudaStream_t cs, cudaGraphConditionalHandle h) {
+          for (int half = 0; half < 2; ++half) {
+            scatter(cs, w.states[half], w.states[1 - half]);
+            sweep(cs, w.states[1 - half]);
+            ScanArgs b = a;
+            b.cond = half;
+            b.handle = h;
+            walk_scan(cs, w, b);
+          }
+        },
+        &exec);
+    if (rc) return rc;
+    execs.push_back(exec);
+    return cudaGraphLaunch(exec, st) == cudaSuccess ? SI_OK : set_error(SI_ERR_CUDA, "%s: graph launch failed", what);
+  }
+  for (int cur = 0;; cur = 1 - cur) {
+    uint32_t c[kCtrWords];
+    if (cudaMemcpyAsync(c, w.ctrs, sizeof(c), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
+        cudaStreamSynchronize(st) != cudaSuccess)
+      return set_error(SI_ERR_CUDA, "%s: %s", what, cudaGetErrorString(cudaGetLastError()));
+    if (c[kCtrLive] == 0) return SI_OK;
+    if (c[kCtrSweeps] >= a.limit) return set_error(SI_ERR_LIMIT, "%s: no convergence within %u sweeps", what, a.limit);
+    if (c[kCtrIn] != 0) scatter(st, w.states[1 - cur], w.states[cur]);
+    sweep(st, w.states[cur]);
+    walk_scan(st, w, a);
+    const int rc = check_launch(what);
+    if (rc) return rc;
+  }
+}
+
+// Waits for the walk and reads its counters.
+int finish_walk(cudaStream_t st, const WalkBuffers& w, std::vector<cudaGraphExec_t>& execs, uint32_t limit, int rc,
+                const char* what, int* rounds_out) {
+  uint32_t c[kCtrWords] = {};
+  if (cudaMemcpyAsync(c, w.ctrs, sizeof(c), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
+      cudaStreamSynchronize(st) != cudaSuccess)
+    rc = rc ? rc : set_error(SI_ERR_CUDA, "%s: %s", what, cudaGetErrorString(cudaGetLastError()));
+  for (cudaGraphExec_t e : execs) cudaGraphExecDestroy(e);
+  if (rc) return rc;
+  if (c[kCtrOver]) return set_error(SI_ERR_LIMIT, "%s: no convergence within %u sweeps", what, limit);
+  if (rounds_out) *rounds_out = (int)c[kCtrSweeps];
+  return check_launch(what);
 }
 }  // namespace
 }  // namespace si
@@ -803,7 +1031,8 @@ extern "C" int si_walk_sorted_scratch(int Zc, int Yc, int Xc, uint64_t max_walks
   clear_error();
   if (!bytes || Zc < 3 || Yc < 3 || Xc < 3 || nol < 1 || nol > 256 || sort_edge < 0 || sort_edge > 1024)
     return set_error(SI_ERR_ARG, "si_walk_sorted_scratch: bad arguments");
-  *bytes = sort_layout(make_geom(Zc, Yc, Xc, sort_edge > 0 ? sort_edge : kSortEdge), max_walks, nol).total;
+  const BrickGeom g = make_geom(Zc, Yc, Xc, sort_edge > 0 ? sort_edge : kSortEdge);
+  *bytes = sort_layout((uint64_t)g.nb * nol, max_walks, 0).total;
   return SI_OK;
 }
 
@@ -843,7 +1072,7 @@ extern "C" int si_walk_sorted(const void* packed, int work_is_float, int Zc, int
   if ((uint64_t)Zc * Yc * Xc > 0xFFFFFFFFull) return set_error(SI_ERR_LIMIT, "si_walk_sorted: volume above 2^32");
   if (nbrw < 0 || sorw < 0 || (uint64_t)nbrw * (uint64_t)sorw >= (1ull << 24))
     return set_error(SI_ERR_LIMIT, "si_walk_sorted: nbrw*sorw must be below 2^24");
-  if (sweep_steps <= 0) sweep_steps = 32;
+  if (sweep_steps <= 0) sweep_steps = default_sweep_steps(sorw);
   if (sort_edge <= 0) sort_edge = kSortEdge;
   if (sort_edge > 1024) return set_error(SI_ERR_ARG, "si_walk_sorted: sort_edge above 1024");
   cudaStream_t st = as_stream(stream);
@@ -858,24 +1087,16 @@ extern "C" int si_walk_sorted(const void* packed, int work_is_float, int Zc, int
   if (walks >= 0xFFFFFFFFull) return set_error(SI_ERR_LIMIT, "si_walk_sorted: more than 2^32 walks");
   const BrickGeom g = make_geom(Zc, Yc, Xc, sort_edge);
   if ((uint64_t)g.nb * (uint64_t)nol >= 0xFFFFFFFFull) return set_error(SI_ERR_LIMIT, "si_walk_sorted: too many buckets");
-  const SortLayout L = sort_layout(g, walks, nol);
+  const uint32_t nbt = g.nb * (uint32_t)nol;
+  const SortLayout L = sort_layout(nbt, walks, 0);
   if (scratch_bytes < L.total)
     return set_error(SI_ERR_ARG, "si_walk_sorted: scratch of %llu bytes, %llu needed", scratch_bytes,
                      (unsigned long long)L.total);
-  uint8_t* base = static_cast<uint8_t*>(scratch);
-  uint4* states[2] = {reinterpret_cast<uint4*>(base + L.states0), reinterpret_cast<uint4*>(base + L.states1)};
-  uint32_t* counts = reinterpret_cast<uint32_t*>(base + L.counts);     // this round's bucket sizes
-  uint32_t* counts2 = reinterpret_cast<uint32_t*>(base + L.counts2);   // the next round's, counted by the sweep
-  uint32_t* offsets = reinterpret_cast<uint32_t*>(base + L.offsets);
-  uint32_t* sums = reinterpret_cast<uint32_t*>(base + L.sums);
-  uint32_t* ctrs = reinterpret_cast<uint32_t*>(base + L.ctrs);
-  const uint32_t nbt = g.nb * (uint32_t)nol;
-  const uint32_t nblocks = (nbt + kScanBlock - 1) / kScanBlock;
+  const WalkBuffers w = walk_buffers(scratch, L, nbt);
   const SeedRec* sd_all = reinterpret_cast<const SeedRec*>(seeds);
   const int sms = sm_count();
   const int gb = sms * 8;
   const uint32_t k0 = (uint32_t)key, k1 = (uint32_t)(key >> 32);
-  const size_t count_bytes = (size_t)(nbt + 1) * sizeof(uint32_t);
   // Seeds are walked in consecutive ranges of about range_walks() walks, each
   // to completion. Seeds come in slice order, so a range is a compact slab and
   // a sweep's records and hit counters stay closer to L2 than when every seed
@@ -886,149 +1107,70 @@ extern "C" int si_walk_sorted(const void* packed, int work_is_float, int Zc, int
   const uint64_t nbatch = std::max<uint64_t>(1, (walks + per_range / 2) / per_range);
   // walkers per thread: mode 0 -> 1, 1 -> 2, 2 -> 3, 3 -> 4
   const int mode = g_sweep_pairs.load(std::memory_order_relaxed);
-  const int tpb = mode == 3 ? 128 : 256;
-  const uint64_t cap = (uint64_t)sms * (tpb == 128 ? 16 : 8);
-  // one sweep launch over states s_in (live count live_now, or *live_dev when
-  // the count stays on the device) into the next round's bucket sizes c_next
-  auto sweep = [&](cudaStream_t s, uint4* s_in, uint32_t live_now, const uint32_t* live_dev,
-                   const SeedRec* sd, uint32_t* c_next) {
+  const uint32_t limit = round_limit();
+  const bool device_loop = g_device_loop.load(std::memory_order_relaxed) != 0;
+  const ScanArgs a{w.counts, nbt, w.offsets, w.ctrs, limit, 0, {}};
+  const uint32_t K = (uint32_t)sweep_steps;
+  if (cudaMemsetAsync(w.ctrs, 0, kCtrWords * sizeof(uint32_t), st) != cudaSuccess ||
+      cudaMemsetAsync(w.counts, 0, ((size_t)nbt + 1) * sizeof(uint32_t), st) != cudaSuccess)
+    return set_error(SI_ERR_CUDA, "si_walk_sorted: memset failed");
+  std::vector<cudaGraphExec_t> execs;
+  int rc = SI_OK;
+  for (uint64_t bidx = 0; bidx < nbatch && rc == SI_OK; ++bidx) {
+    const uint32_t sa = (uint32_t)((uint64_t)ns * bidx / nbatch), se = (uint32_t)((uint64_t)ns * (bidx + 1) / nbatch);
+    if (se == sa) continue;
+    const SeedRec* sd = sd_all + sa;
+    const uint32_t ns_b = se - sa;
+    const uint64_t n0 = (uint64_t)ns_b * (uint64_t)nbrw;
+    // One group of walkers per thread: CTAs start in the sorted order, so that
+    // those running at any moment share a compact part of the volume. (A grid of
+    // 8 CTAs per SM that strides over the walkers: 419x492x462 915 ms, this one
+    // 857 ms; 176x224x208 with labels on all axes 370 and 332 ms.) Walks that
+    // do not fill the SMs once go out in small CTAs, spread more evenly:
+    // 40x36x33, 95 thousand walks, 4.5 and 4.2 ms.
     const uint64_t per = (uint64_t)mode + 1;
-    const uint64_t threads = live_dev ? cap * tpb : ((uint64_t)live_now + per - 1) / per;
-    const uint64_t want_blocks = (threads + tpb - 1) / tpb;
-    const uint32_t blocks = (uint32_t)(want_blocks < cap ? want_blocks : cap);
-#define SI_SWEEP(KERNEL) KERNEL<<<blocks, tpb, 0, s>>>(packed, g, s_in, live_now, (uint32_t)sweep_steps, sd, k0, k1, \
-                                                       hits, c_next, live_dev)
+    const bool few = mode == 1 && n0 <= (uint64_t)sms * 2 * 768;
+    const int tpb = few ? 64 : mode == 3 ? 128 : 256;
+    const uint32_t blocks = (uint32_t)(((n0 + per - 1) / per + tpb - 1) / tpb);
+    const uint32_t sort_blocks = (uint32_t)std::min<uint64_t>(gb, (n0 + 255) / 256);
+    auto sweep = [&](cudaStream_t s, uint4* states) {
+#define SI_SWEEP(KERNEL) KERNEL<<<blocks, tpb, 0, s>>>(packed, g, states, K, sd, k0, k1, hits, w.counts, w.ctrs)
 #define SI_SWEEPS(F)                                   \
   do {                                                 \
     if (mode == 3)                                     \
       SI_SWEEP((sweep_multi_kernel<F, 4, 128, 3>));    \
     else if (mode == 2)                                \
       SI_SWEEP((sweep_multi_kernel<F, 3, 256, 2>));    \
+    else if (few)                                      \
+      SI_SWEEP((sweep_multi_kernel<F, 2, 64, 12>));    \
     else if (mode == 1)                                \
       SI_SWEEP((sweep_multi_kernel<F, 2, 256, 3>));    \
     else                                               \
       SI_SWEEP(sweep_kernel<F>);                       \
   } while (0)
-    if (work_is_float)
-      SI_SWEEPS(true);
-    else
-      SI_SWEEPS(false);
+      if (work_is_float)
+        SI_SWEEPS(true);
+      else
+        SI_SWEEPS(false);
 #undef SI_SWEEPS
 #undef SI_SWEEP
-  };
-  auto scan = [&](cudaStream_t s, const uint32_t* c) {
-    scan_sums_kernel<<<nblocks, 256, 0, s>>>(c, nbt, sums);
-    scan_top_kernel<<<1, 1024, 0, s>>>(sums, nblocks);
-    scan_apply_kernel<<<nblocks, 256, 0, s>>>(c, nbt, sums, offsets, ctrs);
-  };
-  if (g_device_loop.load(std::memory_order_relaxed)) {
-    // Device-side sweep loop: no host round trip per sweep. ctrs: [0] live
-    // walkers after the last scan, [3] the states the next scatter reads,
-    // [4] sweeps run, [5] round limit hit.
-    const uint32_t limit = round_limit();
-    if (cudaMemsetAsync(ctrs, 0, kCtrWords * sizeof(uint32_t), st) != cudaSuccess)
-      return set_error(SI_ERR_CUDA, "si_walk_sorted: memset failed");
-    std::vector<cudaGraphExec_t> execs;
-    int rc = SI_OK;
-    uint32_t* C0 = counts;
-    uint32_t* C1 = counts2;
-    for (uint64_t bidx = 0; bidx < nbatch && rc == SI_OK; ++bidx) {
-      const uint32_t sa = (uint32_t)((uint64_t)ns * bidx / nbatch), se = (uint32_t)((uint64_t)ns * (bidx + 1) / nbatch);
-      if (se == sa) continue;
-      const SeedRec* sd = sd_all + sa;
-      const uint32_t ns_b = se - sa;
-      const uint64_t n0 = (uint64_t)ns_b * (uint64_t)nbrw;
-      // round 0 from the virtual (seed, walk) pairs into states[0]
-      cudaMemsetAsync(C0, 0, count_bytes, st);
-      bucket_kernel<true, false><<<gb, 256, 0, st>>>(nullptr, n0, sd, ns_b, sorw, g, C0, nullptr, nullptr);
-      scan(st, C0);
-      cudaMemsetAsync(C0, 0, count_bytes, st);
-      cudaMemsetAsync(C1, 0, count_bytes, st);
-      bucket_kernel<true, true><<<gb, 256, 0, st>>>(nullptr, n0, sd, ns_b, sorw, g, C0, offsets, states[0]);
-      sweep(st, states[0], 0u, ctrs, sd, C1);
-      round_shift_kernel<<<1, 1, 0, st>>>(ctrs);
-      scan(st, C1);
-      rc = check_launch("si_walk_sorted: round 0");
-      if (rc) break;
-      // later rounds: two per loop iteration (states[0] -> states[1] with
-      // counts C1 -> C0, then back), while walkers are live
-      cudaGraphExec_t exec = nullptr;
-      rc = build_while_graph(
-          [&](cudaStream_t cs, cudaGraphConditionalHandle h) {
-            for (int half = 0; half < 2; ++half) {
-              uint32_t* cur_c = half ? C0 : C1;  // scanned sizes -> scatter cursor
-              uint32_t* nxt_c = half ? C1 : C0;  // the sweep's counts of the round after
-              uint4* s_in = states[half];
-              uint4* s_out = states[1 - half];
-              cudaMemsetAsync(cur_c, 0, count_bytes, cs);
-              cudaMemsetAsync(nxt_c, 0, count_bytes, cs);
-              bucket_kernel<false, true><<<gb, 256, 0, cs>>>(s_in, 0, sd, ns_b, sorw, g, cur_c, offsets, s_out,
-                                                             ctrs + 3);
-              sweep(cs, s_out, 0u, ctrs, sd, nxt_c);
-              round_shift_kernel<<<1, 1, 0, cs>>>(ctrs);
-              scan(cs, nxt_c);
-            }
-            round_cond_kernel<<<1, 1, 0, cs>>>(ctrs, h, limit);
-          },
-          &exec);
-      if (rc) break;
-      execs.push_back(exec);
-      if (cudaGraphLaunch(exec, st) != cudaSuccess) rc = set_error(SI_ERR_CUDA, "si_walk_sorted: graph launch failed");
-    }
-    uint32_t host_ctrs[kCtrWords] = {};
-    if (cudaMemcpyAsync(host_ctrs, ctrs, sizeof(host_ctrs), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
-        cudaStreamSynchronize(st) != cudaSuccess)
-      rc = rc ? rc : set_error(SI_ERR_CUDA, "si_walk_sorted: %s", cudaGetErrorString(cudaGetLastError()));
-    for (cudaGraphExec_t e : execs) cudaGraphExecDestroy(e);
-    if (rc) return rc;
-    if (host_ctrs[5]) return set_error(SI_ERR_LIMIT, "si_walk_sorted: no convergence within %u sweeps", limit);
-    if (rounds_out) *rounds_out = (int)host_ctrs[4];
-    return check_launch("si_walk_sorted");
+    };
+    rc = run_range(
+        st, w, a, device_loop, "si_walk_sorted", execs,
+        [&](cudaStream_t s) {
+          bucket_kernel<true, false><<<sort_blocks, 256, 0, s>>>(nullptr, n0, sd, ns_b, sorw, g, w.counts, nullptr,
+                                                                 nullptr);
+        },
+        [&](cudaStream_t s, uint4* out) {
+          bucket_kernel<true, true><<<sort_blocks, 256, 0, s>>>(nullptr, n0, sd, ns_b, sorw, g, w.offsets, nullptr, out);
+        },
+        [&](cudaStream_t s, uint4* in, uint4* out) {
+          bucket_kernel<false, true><<<sort_blocks, 256, 0, s>>>(in, 0, sd, ns_b, sorw, g, w.offsets, nullptr, out,
+                                                                 w.ctrs + kCtrIn);
+        },
+        sweep);
   }
-  // Host-side sweep loop: the live count is read back after every scan.
-  int rounds = 0;
-  for (uint64_t bidx = 0; bidx < nbatch; ++bidx) {
-    const uint32_t sa = (uint32_t)((uint64_t)ns * bidx / nbatch), se = (uint32_t)((uint64_t)ns * (bidx + 1) / nbatch);
-    if (se == sa) continue;
-    const SeedRec* sd = sd_all + sa;
-    const uint32_t ns_b = se - sa;
-    int cur = 0;
-    uint64_t n_prev = (uint64_t)ns_b * (uint64_t)nbrw;
-    // round 0's bucket sizes come from a counting pass over the virtual
-    // (seed, walk) pairs; every later round's from the previous sweep
-    if (cudaMemsetAsync(counts, 0, count_bytes, st) != cudaSuccess)
-      return set_error(SI_ERR_CUDA, "si_walk_sorted: memset failed");
-    bucket_kernel<true, false><<<gb, 256, 0, st>>>(nullptr, n_prev, sd, ns_b, sorw, g, counts, nullptr, nullptr);
-    for (int batch_rounds = 0;; ++batch_rounds, ++rounds) {
-      const bool first = batch_rounds == 0;
-      scan(st, counts);
-      uint32_t live_now = 0;
-      if (cudaMemcpyAsync(&live_now, ctrs, sizeof(uint32_t), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
-          cudaStreamSynchronize(st) != cudaSuccess)
-        return set_error(SI_ERR_CUDA, "si_walk_sorted: round %d: %s", rounds, cudaGetErrorString(cudaGetLastError()));
-      if (live_now == 0) break;
-      if ((uint64_t)rounds >= round_limit()) return set_error(SI_ERR_LIMIT, "si_walk_sorted: no convergence");
-      // counts becomes the scatter's per-bucket cursor, counts2 the next round's sizes
-      if (cudaMemsetAsync(counts, 0, count_bytes, st) != cudaSuccess ||
-          cudaMemsetAsync(counts2, 0, count_bytes, st) != cudaSuccess)
-        return set_error(SI_ERR_CUDA, "si_walk_sorted: memset failed");
-      const int nxt = first ? 0 : 1 - cur;
-      if (first)
-        bucket_kernel<true, true><<<gb, 256, 0, st>>>(nullptr, n_prev, sd, ns_b, sorw, g, counts, offsets,
-                                                      states[nxt]);
-      else
-        bucket_kernel<false, true><<<gb, 256, 0, st>>>(states[cur], n_prev, sd, ns_b, sorw, g, counts, offsets,
-                                                       states[nxt]);
-      cur = nxt;
-      sweep(st, states[cur], live_now, nullptr, sd, counts2);
-      const int rc = check_launch("si_walk_sorted: sweep");
-      if (rc) return rc;
-      std::swap(counts, counts2);
-      n_prev = live_now;
-    }
-  }
-  if (rounds_out) *rounds_out = rounds;
-  return check_launch("si_walk_sorted");
+  return finish_walk(st, w, execs, limit, rc, "si_walk_sorted", rounds_out);
 }
 
 // ===========================================================================
@@ -1054,19 +1196,19 @@ struct VolDesc {
   uint64_t walk0;   // first global walk index of this volume (round 0)
   uint32_t ns;      // seeds
   int is_float;
+  FastDiv by_F, by_X;
 };
 
 __device__ __forceinline__ uint32_t bvol(const uint4& s) { return s.z >> 24; }
 __device__ __forceinline__ uint32_t bstep(const uint4& s) { return s.z & 0xFFFFFFu; }
 __device__ __forceinline__ bool blive(const uint4& s) { return bstep(s) != (s.w & 0xFFFFFFu); }
 
-__device__ __forceinline__ uint32_t bbucket(const VolDesc& v, int edge, const uint4& s) {
-  const uint32_t z = s.x / v.F;
+__device__ __forceinline__ uint32_t bbucket(const VolDesc& v, const FastDiv& by_edge, const uint4& s) {
+  const uint32_t z = v.by_F(s.x);
   const uint32_t r = s.x - z * v.F;
-  const uint32_t y = r / (uint32_t)v.Xc;
+  const uint32_t y = v.by_X(r);
   const uint32_t x = r - y * (uint32_t)v.Xc;
-  const uint32_t e = (uint32_t)edge;
-  const uint32_t brick = (z / e * (uint32_t)v.nby + y / e) * (uint32_t)v.nbx + x / e;
+  const uint32_t brick = (by_edge(z) * (uint32_t)v.nby + by_edge(y)) * (uint32_t)v.nbx + by_edge(x);
   return v.bucket0 + (s.w >> 24) * v.nb + brick;
 }
 
@@ -1094,31 +1236,37 @@ __device__ __forceinline__ bool bfetch(uint64_t i, uint64_t n, const uint4* __re
 template <bool kFirst, bool kScatter>
 __global__ void __launch_bounds__(256) bbucket_kernel(const uint4* __restrict__ states_in, uint64_t n,
                                                       const VolDesc* __restrict__ vols, int n_vols, int sorw,
-                                                      int edge, uint32_t* __restrict__ counts,
-                                                      const uint32_t* __restrict__ offsets,
+                                                      FastDiv edge, uint32_t* __restrict__ counts,
                                                       uint4* __restrict__ states_out,
                                                       const uint32_t* __restrict__ n_dev = nullptr) {
   if (n_dev) n = *n_dev;  // the count lives on the device (device-side sweep loop)
   const int lane = threadIdx.x & 31;
+  constexpr int N = 4;  // states a thread, as in bucket_kernel
   const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-  for (uint64_t base = (uint64_t)blockIdx.x * blockDim.x + (threadIdx.x & ~31u); base < n; base += stride) {
-    uint4 s;
-    const bool ok = bfetch<kFirst>(base + lane, n, states_in, vols, n_vols, sorw, s);
-    const uint32_t key = ok ? bbucket(vols[bvol(s)], edge, s) : 0u;
-    const uint32_t act = __ballot_sync(0xffffffffu, ok);
-    if (ok) {
-      const uint32_t peers = __match_any_sync(act, key);
-      const int leader = __ffs(peers) - 1;
-      const uint32_t cnt = __popc(peers);
-      if (!kScatter) {
-        if (lane == leader) atomicAdd(&counts[key], cnt);
-      } else {
-        uint32_t b = 0;
-        if (lane == leader) b = atomicAdd(&counts[key], cnt);
-        b = __shfl_sync(peers, b, leader);
-        const uint32_t rank = __popc(peers & ((1u << lane) - 1u));
-        states_out[offsets[key] + b + rank] = s;
+  for (uint64_t base = (uint64_t)blockIdx.x * blockDim.x + (threadIdx.x & ~31u); base < n; base += N * stride) {
+    uint4 s[N];
+    bool ok[N];
+    uint32_t key[N], peers[N], at[N];
+#pragma unroll
+    for (int k = 0; k < N; ++k)
+      ok[k] = bfetch<kFirst>(base + k * stride + lane, n, states_in, vols, n_vols, sorw, s[k]);
+#pragma unroll
+    for (int k = 0; k < N; ++k) {
+      key[k] = ok[k] ? bbucket(vols[bvol(s[k])], edge, s[k]) : 0u;
+      const uint32_t act = __ballot_sync(0xffffffffu, ok[k]);
+      at[k] = peers[k] = 0u;
+      if (ok[k]) {
+        peers[k] = __match_any_sync(act, key[k]);
+        if (lane == __ffs(peers[k]) - 1) at[k] = atomicAdd(&counts[key[k]], (uint32_t)__popc(peers[k]));
       }
+    }
+    if (kScatter) {
+#pragma unroll
+      for (int k = 0; k < N; ++k)
+        if (ok[k]) {
+          const uint32_t b = __shfl_sync(peers[k], at[k], __ffs(peers[k]) - 1);
+          states_out[b + __popc(peers[k] & ((1u << lane) - 1u))] = s[k];
+        }
     }
   }
 }
@@ -1129,11 +1277,11 @@ __global__ void __launch_bounds__(256) bbucket_kernel(const uint4* __restrict__ 
 // are formed here (warp-aggregated atomics into next_counts).
 template <bool kPair, int kMinBlocks>
 __global__ void __launch_bounds__(256, kMinBlocks) bsweep_kernel(const VolDesc* __restrict__ vols_g, int n_vols,
-                                                                 uint4* __restrict__ states, uint32_t n_live,
-                                                                 uint32_t K, uint32_t k0, uint32_t k1, int edge,
+                                                                 uint4* __restrict__ states, uint32_t K, uint32_t k0,
+                                                                 uint32_t k1, FastDiv edge,
                                                                  uint32_t* __restrict__ next_counts,
-                                                                 const uint32_t* __restrict__ live_dev) {
-  if (live_dev) n_live = *live_dev;  // the count lives on the device (device-side sweep loop)
+                                                                 const uint32_t* __restrict__ ctrs) {
+  const uint32_t n_live = ctrs[kCtrLive];
   __shared__ int32_t s_delta[256 * 6];  // move offsets of every volume
   __shared__ VolDesc vols[256];         // the volume table (at most 256 volumes)
   for (int i = threadIdx.x; i < n_vols; i += blockDim.x) vols[i] = vols_g[i];
@@ -1231,8 +1379,7 @@ struct BatchPlan {
   std::vector<si::VolDesc> vols;
   uint64_t walks = 0;
   uint32_t nbt = 0;
-  size_t off_vols = 0, off_states0 = 0, off_states1 = 0, off_counts = 0, off_counts2 = 0, off_offsets = 0,
-         off_sums = 0, off_ctrs = 0, total = 0;
+  si::SortLayout layout{};
 };
 
 int make_batch_plan(const si_volume_t* vols, int n_vols, int nbrw, int edge, const uint32_t* ns_host,
@@ -1262,6 +1409,8 @@ int make_batch_plan(const si_volume_t* vols, int n_vols, int nbrw, int edge, con
     d.walk0 = walk;
     d.ns = ns_host ? (ns_host[v] < in.max_seeds ? ns_host[v] : in.max_seeds) : in.max_seeds;
     d.is_float = in.work_is_float;
+    d.by_F = si::FastDiv(d.F);
+    d.by_X = si::FastDiv((uint32_t)in.Xc);
     bucket += (uint64_t)d.nb * in.nol;
     walk += (uint64_t)d.ns * (uint64_t)nbrw;
   }
@@ -1269,25 +1418,7 @@ int make_batch_plan(const si_volume_t* vols, int n_vols, int nbrw, int edge, con
   if (walk >= 0xFFFFFFFFull) return si::set_error(SI_ERR_LIMIT, "si_walk_sorted_batch: more than 2^32 walks");
   P.walks = walk;
   P.nbt = (uint32_t)bucket;
-  const uint64_t nblocks = (P.nbt + si::kScanBlock - 1) / si::kScanBlock;
-  size_t off = 0;
-  P.off_vols = off;
-  off = si::align_up(off + n_vols * sizeof(si::VolDesc), 256);
-  P.off_states0 = off;
-  off = si::align_up(off + P.walks * sizeof(uint4), 256);
-  P.off_states1 = off;
-  off = si::align_up(off + P.walks * sizeof(uint4), 256);
-  P.off_counts = off;
-  off = si::align_up(off + ((size_t)P.nbt + 1) * sizeof(uint32_t), 256);
-  P.off_counts2 = off;
-  off = si::align_up(off + ((size_t)P.nbt + 1) * sizeof(uint32_t), 256);
-  P.off_offsets = off;
-  off = si::align_up(off + ((size_t)P.nbt + 1) * sizeof(uint32_t), 256);
-  P.off_sums = off;
-  off = si::align_up(off + (nblocks + 1) * sizeof(uint32_t), 256);
-  P.off_ctrs = off;
-  off = si::align_up(off + si::kCtrWords * sizeof(uint32_t), 256);
-  P.total = off;
+  P.layout = si::sort_layout(P.nbt, P.walks, n_vols * sizeof(si::VolDesc));
   return SI_OK;
 }
 }  // namespace
@@ -1300,7 +1431,7 @@ extern "C" int si_walk_sorted_batch_scratch(const si_volume_t* vols, int n_vols,
   BatchPlan P;
   const int rc = make_batch_plan(vols, n_vols, nbrw, sort_edge > 0 ? sort_edge : kSortEdge, nullptr, P);
   if (rc) return rc;
-  *bytes = P.total;
+  *bytes = P.layout.total;
   return SI_OK;
 }
 
@@ -1311,7 +1442,7 @@ extern "C" int si_walk_sorted_batch(const si_volume_t* vols, int n_vols, int nbr
   if (!vols || !scratch || n_vols < 1 || n_vols > 256) return set_error(SI_ERR_ARG, "si_walk_sorted_batch: bad args");
   if (nbrw < 0 || sorw < 0 || (uint64_t)nbrw * (uint64_t)sorw >= (1ull << 24))
     return set_error(SI_ERR_LIMIT, "si_walk_sorted_batch: nbrw*sorw must be below 2^24");
-  if (sweep_steps <= 0) sweep_steps = 32;
+  if (sweep_steps <= 0) sweep_steps = default_sweep_steps(sorw);
   if (sort_edge <= 0) sort_edge = kSortEdge;
   if (sort_edge > 1024) return set_error(SI_ERR_ARG, "si_walk_sorted_batch: sort_edge above 1024");
   cudaStream_t st = as_stream(stream);
@@ -1331,132 +1462,48 @@ extern "C" int si_walk_sorted_batch(const si_volume_t* vols, int n_vols, int nbr
   BatchPlan Pmax;  // scratch is sized for max_seeds
   rc = make_batch_plan(vols, n_vols, nbrw, sort_edge, nullptr, Pmax);
   if (rc) return rc;
-  if (scratch_bytes < Pmax.total)
+  if (scratch_bytes < Pmax.layout.total)
     return set_error(SI_ERR_ARG, "si_walk_sorted_batch: scratch of %llu bytes, %llu needed", scratch_bytes,
-                     (unsigned long long)Pmax.total);
-  uint8_t* base = static_cast<uint8_t*>(scratch);
+                     (unsigned long long)Pmax.layout.total);
   // layout of the max-seed plan; the actual walks fit in it
-  VolDesc* d_vols = reinterpret_cast<VolDesc*>(base + Pmax.off_vols);
-  uint4* states[2] = {reinterpret_cast<uint4*>(base + Pmax.off_states0),
-                      reinterpret_cast<uint4*>(base + Pmax.off_states1)};
-  uint32_t* counts = reinterpret_cast<uint32_t*>(base + Pmax.off_counts);
-  uint32_t* offsets = reinterpret_cast<uint32_t*>(base + Pmax.off_offsets);
-  uint32_t* sums = reinterpret_cast<uint32_t*>(base + Pmax.off_sums);
-  uint32_t* ctrs = reinterpret_cast<uint32_t*>(base + Pmax.off_ctrs);
+  const WalkBuffers w = walk_buffers(scratch, Pmax.layout, P.nbt);
+  VolDesc* d_vols = reinterpret_cast<VolDesc*>(static_cast<uint8_t*>(scratch) + Pmax.layout.vols);
   if (cudaMemcpyAsync(d_vols, P.vols.data(), n_vols * sizeof(VolDesc), cudaMemcpyHostToDevice, st) != cudaSuccess)
     return set_error(SI_ERR_CUDA, "si_walk_sorted_batch: descriptor upload failed");
-  const uint32_t nbt = P.nbt;
-  const uint32_t nblocks = (nbt + kScanBlock - 1) / kScanBlock;
   const int sms = sm_count();
-  const int gb = sms * 8;
-  const uint32_t k0 = (uint32_t)key, k1 = (uint32_t)(key >> 32);
-  uint32_t* counts2 = reinterpret_cast<uint32_t*>(base + Pmax.off_counts2);
-  const size_t count_bytes = (size_t)(nbt + 1) * sizeof(uint32_t);
+  const uint32_t k0 = (uint32_t)key, k1 = (uint32_t)(key >> 32), K = (uint32_t)sweep_steps;
+  const FastDiv by_edge((uint32_t)sort_edge);
   // walker pairs unless mode 0
   const bool pairs = g_sweep_pairs.load(std::memory_order_relaxed) != 0;
-  const uint64_t bcap = (uint64_t)sms * 8;
-  auto sweep = [&](cudaStream_t s, uint4* s_in, uint32_t live_now, const uint32_t* live_dev, uint32_t* c_next) {
-    const uint64_t threads = live_dev ? bcap * 256 : (pairs ? ((uint64_t)live_now + 1) / 2 : (uint64_t)live_now);
-    const uint64_t want_blocks = (threads + 255) / 256;
-    const uint32_t blocks = (uint32_t)(want_blocks < bcap ? want_blocks : bcap);
+  // one group of walkers per thread, as in si_walk_sorted
+  const uint32_t blocks = (uint32_t)(((pairs ? (P.walks + 1) / 2 : P.walks) + 255) / 256);
+  const uint32_t sort_blocks = (uint32_t)std::min<uint64_t>((uint64_t)sms * 8, (P.walks + 255) / 256);
+  auto sweep = [&](cudaStream_t s, uint4* states) {
     if (pairs)  // measured: 2 CTAs of 256 per SM (no spills) beat 3
-      bsweep_kernel<true, 2><<<blocks, 256, 0, s>>>(d_vols, n_vols, s_in, live_now, (uint32_t)sweep_steps, k0, k1,
-                                                    sort_edge, c_next, live_dev);
+      bsweep_kernel<true, 2><<<blocks, 256, 0, s>>>(d_vols, n_vols, states, K, k0, k1, by_edge, w.counts, w.ctrs);
     else
-      bsweep_kernel<false, 5><<<blocks, 256, 0, s>>>(d_vols, n_vols, s_in, live_now, (uint32_t)sweep_steps, k0, k1,
-                                                     sort_edge, c_next, live_dev);
+      bsweep_kernel<false, 5><<<blocks, 256, 0, s>>>(d_vols, n_vols, states, K, k0, k1, by_edge, w.counts, w.ctrs);
   };
-  auto scan = [&](cudaStream_t s, const uint32_t* c) {
-    scan_sums_kernel<<<nblocks, 256, 0, s>>>(c, nbt, sums);
-    scan_top_kernel<<<1, 1024, 0, s>>>(sums, nblocks);
-    scan_apply_kernel<<<nblocks, 256, 0, s>>>(c, nbt, sums, offsets, ctrs);
-  };
-  if (g_device_loop.load(std::memory_order_relaxed)) {
-    // device-side sweep loop, as in si_walk_sorted
-    const uint32_t limit = round_limit();
-    uint32_t* C0 = counts;
-    uint32_t* C1 = counts2;
-    cudaMemsetAsync(ctrs, 0, kCtrWords * sizeof(uint32_t), st);
-    cudaMemsetAsync(C0, 0, count_bytes, st);
-    bbucket_kernel<true, false><<<gb, 256, 0, st>>>(nullptr, P.walks, d_vols, n_vols, sorw, sort_edge, C0, nullptr,
-                                                    nullptr);
-    scan(st, C0);
-    cudaMemsetAsync(C0, 0, count_bytes, st);
-    cudaMemsetAsync(C1, 0, count_bytes, st);
-    bbucket_kernel<true, true><<<gb, 256, 0, st>>>(nullptr, P.walks, d_vols, n_vols, sorw, sort_edge, C0, offsets,
-                                                   states[0]);
-    sweep(st, states[0], 0u, ctrs, C1);
-    round_shift_kernel<<<1, 1, 0, st>>>(ctrs);
-    scan(st, C1);
-    rc = check_launch("si_walk_sorted_batch: round 0");
-    if (rc) return rc;
-    cudaGraphExec_t exec = nullptr;
-    rc = build_while_graph(
-        [&](cudaStream_t cs, cudaGraphConditionalHandle h) {
-          for (int half = 0; half < 2; ++half) {
-            uint32_t* cur_c = half ? C0 : C1;  // scanned sizes -> scatter cursor
-            uint32_t* nxt_c = half ? C1 : C0;  // the sweep's counts of the round after
-            uint4* s_in = states[half];
-            uint4* s_out = states[1 - half];
-            cudaMemsetAsync(cur_c, 0, count_bytes, cs);
-            cudaMemsetAsync(nxt_c, 0, count_bytes, cs);
-            bbucket_kernel<false, true><<<gb, 256, 0, cs>>>(s_in, 0, d_vols, n_vols, sorw, sort_edge, cur_c, offsets,
-                                                            s_out, ctrs + 3);
-            sweep(cs, s_out, 0u, ctrs, nxt_c);
-            round_shift_kernel<<<1, 1, 0, cs>>>(ctrs);
-            scan(cs, nxt_c);
-          }
-          round_cond_kernel<<<1, 1, 0, cs>>>(ctrs, h, limit);
-        },
-        &exec);
-    if (rc) return rc;
-    if (cudaGraphLaunch(exec, st) != cudaSuccess) rc = set_error(SI_ERR_CUDA, "si_walk_sorted_batch: graph launch");
-    uint32_t host_ctrs[kCtrWords] = {};
-    if (cudaMemcpyAsync(host_ctrs, ctrs, sizeof(host_ctrs), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
-        cudaStreamSynchronize(st) != cudaSuccess)
-      rc = rc ? rc : set_error(SI_ERR_CUDA, "si_walk_sorted_batch: %s", cudaGetErrorString(cudaGetLastError()));
-    cudaGraphExecDestroy(exec);
-    if (rc) return rc;
-    if (host_ctrs[5]) return set_error(SI_ERR_LIMIT, "si_walk_sorted_batch: no convergence within %u sweeps", limit);
-    if (rounds_out) *rounds_out = (int)host_ctrs[4];
-    return check_launch("si_walk_sorted_batch");
-  }
-  int cur = 0, rounds = 0;
-  uint64_t n_prev = P.walks;
-  // round 0's bucket sizes come from a counting pass over the virtual
-  // (volume, seed, walk) triples; every later round's from the previous sweep
-  if (cudaMemsetAsync(counts, 0, count_bytes, st) != cudaSuccess)
+  const uint32_t limit = round_limit();
+  const ScanArgs a{w.counts, P.nbt, w.offsets, w.ctrs, limit, 0, {}};
+  if (cudaMemsetAsync(w.ctrs, 0, kCtrWords * sizeof(uint32_t), st) != cudaSuccess ||
+      cudaMemsetAsync(w.counts, 0, ((size_t)P.nbt + 1) * sizeof(uint32_t), st) != cudaSuccess)
     return set_error(SI_ERR_CUDA, "si_walk_sorted_batch: memset failed");
-  bbucket_kernel<true, false><<<gb, 256, 0, st>>>(nullptr, n_prev, d_vols, n_vols, sorw, sort_edge, counts, nullptr,
-                                                  nullptr);
-  for (;; ++rounds) {
-    const bool first = rounds == 0;
-    scan(st, counts);
-    uint32_t live_now = 0;
-    if (cudaMemcpyAsync(&live_now, ctrs, sizeof(uint32_t), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
-        cudaStreamSynchronize(st) != cudaSuccess)
-      return set_error(SI_ERR_CUDA, "si_walk_sorted_batch: round %d: %s", rounds,
-                       cudaGetErrorString(cudaGetLastError()));
-    if (live_now == 0) break;
-    if ((uint64_t)rounds >= round_limit()) return set_error(SI_ERR_LIMIT, "si_walk_sorted_batch: no convergence");
-    // counts becomes the scatter's per-bucket cursor, counts2 the next round's sizes
-    if (cudaMemsetAsync(counts, 0, count_bytes, st) != cudaSuccess ||
-        cudaMemsetAsync(counts2, 0, count_bytes, st) != cudaSuccess)
-      return set_error(SI_ERR_CUDA, "si_walk_sorted_batch: memset failed");
-    const int nxt = first ? 0 : 1 - cur;
-    if (first)
-      bbucket_kernel<true, true><<<gb, 256, 0, st>>>(nullptr, n_prev, d_vols, n_vols, sorw, sort_edge, counts, offsets,
-                                                     states[nxt]);
-    else
-      bbucket_kernel<false, true><<<gb, 256, 0, st>>>(states[cur], n_prev, d_vols, n_vols, sorw, sort_edge, counts,
-                                                      offsets, states[nxt]);
-    cur = nxt;
-    sweep(st, states[cur], live_now, nullptr, counts2);
-    rc = check_launch("si_walk_sorted_batch: sweep");
-    if (rc) return rc;
-    std::swap(counts, counts2);
-    n_prev = live_now;
-  }
-  if (rounds_out) *rounds_out = rounds;
-  return check_launch("si_walk_sorted_batch");
+  std::vector<cudaGraphExec_t> execs;
+  rc = run_range(
+      st, w, a, g_device_loop.load(std::memory_order_relaxed) != 0, "si_walk_sorted_batch", execs,
+      [&](cudaStream_t s) {
+        bbucket_kernel<true, false><<<sort_blocks, 256, 0, s>>>(nullptr, P.walks, d_vols, n_vols, sorw, by_edge,
+                                                                w.counts, nullptr);
+      },
+      [&](cudaStream_t s, uint4* out) {
+        bbucket_kernel<true, true><<<sort_blocks, 256, 0, s>>>(nullptr, P.walks, d_vols, n_vols, sorw, by_edge,
+                                                               w.offsets, out);
+      },
+      [&](cudaStream_t s, uint4* in, uint4* out) {
+        bbucket_kernel<false, true><<<sort_blocks, 256, 0, s>>>(in, 0, d_vols, n_vols, sorw, by_edge, w.offsets, out,
+                                                                w.ctrs + kCtrIn);
+      },
+      sweep);
+  return finish_walk(st, w, execs, limit, rc, "si_walk_sorted_batch", rounds_out);
 }

@@ -217,13 +217,15 @@ int si_walk_sorted_scratch(int Zc, int Yc, int Xc, uint64_t max_walks, int nol,
 
 /* Sorted-sweep walker: the same walk and the same uint32 hit maps as si_walk
  * over packed records (si_pack_neighbours), run as sweeps in which every live
- * walker advances min(sweep_steps, steps left) steps (default 32 when <= 0);
+ * walker advances min(sweep_steps, steps left) steps (default when <= 0: 128
+ * for walks of at least 1000 steps, else 32);
  * between sweeps the walkers are counting-sorted by (label slot, brick of
  * sort_edge^3 voxels; default 6 when <= 0),
  * so concurrently running walkers share a compact, cache-resident part of
  * the volume and of the hit maps. scratch: si_walk_sorted_scratch bytes;
  * rounds_out (nullable) receives the number of sweeps. nbrw * sorw must be
- * below 2^24. Synchronises `stream` once per sweep. */
+ * below 2^24. Synchronises `stream` before and after the walk (and once per
+ * sweep with the host loop, si_walk_sorted_set_loop). */
 int si_walk_sorted(const void* packed, int work_is_float, int Zc, int Yc,
                    int Xc, const si_seed_t* seeds, const uint32_t* n_seeds,
                    uint32_t max_seeds, int nbrw, int sorw, uint64_t key,
