@@ -39,6 +39,12 @@ constexpr int kAdvThreads = 512;
 constexpr uint32_t kChunk = 4096;  // sorted walkers per work ticket
 constexpr int kScanBlock = 1024;   // elements per scan block (256 threads x 4)
 
+// Threads of a CTA of float walker pairs, 3 CTAs per SM: a record is 8 registers
+// a walker, and at 256 threads (80 registers) they spill (117x141x133, walk of
+// 9.75e9 steps: 64.0 ms; 192 threads and 96 registers 57.8 ms, 128 x 5 60.4,
+// 256 x 2 59.3).
+constexpr int kFloatThreads = 192;
+
 // Device counters of a sorted walk.
 enum WalkCtr {
   kCtrLive = 0,    // walkers live after the last scan = states of the next sweep
@@ -1130,7 +1136,7 @@ extern "C" int si_walk_sorted(const void* packed, int work_is_float, int Zc, int
     // 40x36x33, 95 thousand walks, 4.5 and 4.2 ms.
     const uint64_t per = (uint64_t)mode + 1;
     const bool few = mode == 1 && n0 <= (uint64_t)sms * 2 * 768;
-    const int tpb = few ? 64 : mode == 3 ? 128 : 256;
+    const int tpb = few ? 64 : mode == 3 ? 128 : mode == 1 && work_is_float ? kFloatThreads : 256;
     const uint32_t blocks = (uint32_t)(((n0 + per - 1) / per + tpb - 1) / tpb);
     const uint32_t sort_blocks = (uint32_t)std::min<uint64_t>(gb, (n0 + 255) / 256);
     auto sweep = [&](cudaStream_t s, uint4* states) {
@@ -1142,9 +1148,9 @@ extern "C" int si_walk_sorted(const void* packed, int work_is_float, int Zc, int
     else if (mode == 2)                                \
       SI_SWEEP((sweep_multi_kernel<F, 3, 256, 2>));    \
     else if (few)                                      \
-      SI_SWEEP((sweep_multi_kernel<F, 2, 64, 12>));    \
+      SI_SWEEP((sweep_multi_kernel<F, 2, 64, F ? 9 : 12>)); \
     else if (mode == 1)                                \
-      SI_SWEEP((sweep_multi_kernel<F, 2, 256, 3>));    \
+      SI_SWEEP((sweep_multi_kernel<F, 2, F ? kFloatThreads : 256, 3>)); \
     else                                               \
       SI_SWEEP(sweep_kernel<F>);                       \
   } while (0)
@@ -1271,101 +1277,95 @@ __global__ void __launch_bounds__(256) bbucket_kernel(const uint4* __restrict__ 
   }
 }
 
-// One sweep of the batched walkers. kPair: a thread takes two consecutive
-// walkers and advances them together (walk_steps_multi) when they belong to
-// the same volume, else one after the other. The next sweep's bucket counts
-// are formed here (warp-aggregated atomics into next_counts).
-template <bool kPair, int kMinBlocks>
-__global__ void __launch_bounds__(256, kMinBlocks) bsweep_kernel(const VolDesc* __restrict__ vols_g, int n_vols,
+// One sweep of the batched walkers of the volumes of one record kind: every CTA
+// takes N * kThreads consecutive walkers of ONE volume, so that its geometry and
+// record pointer are the same for all threads, as in sweep_multi_kernel (a
+// kernel whose threads looked up their own walker's volume, record kind
+// included, took 106 registers, 2 CTAs per SM: 222 ms of sweeps for 6 uint16
+// volumes of 64..144 voxels an edge, this one 148 ms). After the scatter a
+// bucket's cursor stands at its end, so the cursor before a volume's first
+// bucket is where the volume's walkers start.
+template <bool kFloat, int N, int kThreads, int kMinBlocks>
+__global__ void __launch_bounds__(kThreads, kMinBlocks) bsweep_kernel(const VolDesc* __restrict__ vols, int n_vols,
+                                                                 uint32_t nbt, const uint32_t* __restrict__ cursors,
                                                                  uint4* __restrict__ states, uint32_t K, uint32_t k0,
                                                                  uint32_t k1, FastDiv edge,
-                                                                 uint32_t* __restrict__ next_counts,
-                                                                 const uint32_t* __restrict__ ctrs) {
-  const uint32_t n_live = ctrs[kCtrLive];
-  __shared__ int32_t s_delta[256 * 6];  // move offsets of every volume
-  __shared__ VolDesc vols[256];         // the volume table (at most 256 volumes)
-  for (int i = threadIdx.x; i < n_vols; i += blockDim.x) vols[i] = vols_g[i];
-  for (int i = threadIdx.x; i < n_vols * 6; i += blockDim.x) {
-    const VolDesc& d = vols_g[i / 6];
-    const int dir = i % 6;
-    const int32_t mag = dir < 2 ? (int32_t)d.F : (dir < 4 ? d.Xc : 1);
-    s_delta[i] = (dir & 1) ? -mag : mag;
+                                                                 uint32_t* __restrict__ next_counts) {
+  static_assert(kThreads >= 128, "two volumes a thread, at most 256");
+  constexpr uint32_t kSpan = (uint32_t)kThreads * (uint32_t)N;
+  __shared__ uint32_t s_warp[32];
+  __shared__ int32_t s_delta[6];
+  __shared__ VolDesc d;
+  __shared__ uint32_t s_first, s_n;
+  {
+    uint32_t beg[2], end[2], ctas[2];
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      const int v = 2 * (int)threadIdx.x + k;
+      beg[k] = end[k] = 0u;
+      if (v < n_vols && (vols[v].is_float != 0) == kFloat) {
+        beg[k] = v ? cursors[vols[v].bucket0 - 1u] : 0u;
+        end[k] = cursors[(v + 1 < n_vols ? vols[v + 1].bucket0 : nbt) - 1u];
+      }
+      ctas[k] = (end[k] - beg[k] + kSpan - 1u) / kSpan;
+    }
+    if (threadIdx.x == 0) s_n = 0u;
+    uint32_t total;
+    uint32_t before = cta_exclusive(ctas[0] + ctas[1], s_warp, total);
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      if (blockIdx.x >= before && blockIdx.x - before < ctas[k]) {
+        const uint32_t at = (blockIdx.x - before) * kSpan;
+        s_first = beg[k] + at;
+        s_n = min(kSpan, end[k] - beg[k] - at);
+        d = vols[2 * threadIdx.x + (unsigned)k];
+        const int32_t F = (int32_t)d.F;
+        s_delta[0] = F; s_delta[1] = -F; s_delta[2] = d.Xc; s_delta[3] = -d.Xc; s_delta[4] = 1; s_delta[5] = -1;
+      }
+      before += ctas[k];
+    }
+    __syncthreads();
   }
-  __syncthreads();
-  const uint32_t stride = gridDim.x * blockDim.x;
+  const uint32_t n = s_n;
+  if (n == 0u) return;  // beyond the last walker
   const int lane = threadIdx.x & 31;
   const uint64_t nz = f2_negzero();
-  constexpr uint32_t N = kPair ? 2u : 1u;
-  const uint32_t n_groups = (n_live + N - 1u) / N;
-  const uint32_t i_end = (n_groups + 31u) & ~31u;  // warp-uniform: the counting runs with full warps
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < i_end; i += stride) {
-    uint4 st[N];
-    bool alive[N];
+  const uint32_t first = s_first;
+  uint4 st[N];
+  bool alive[N];
+  uint32_t te[N];
+  PairWalker W[N];
 #pragma unroll
-    for (uint32_t w = 0; w < N; ++w) {
-      st[w] = make_uint4(0u, 0u, 0u, 0u);
-      alive[w] = false;
+  for (int w = 0; w < N; ++w) {
+    const uint32_t j = threadIdx.x * (uint32_t)N + (uint32_t)w;
+    st[w] = make_uint4(0u, 0u, 0u, 0u);
+    alive[w] = false;
+    te[w] = 0u;
+    W[w] = pair_walker(0u, 0u, 0u, 0.0f, 0.0f, 0u, 0u, 0u, nullptr);  // no steps without a walker
+    if (j < n) {
+      st[w] = states[first + j];
+      const SeedRec sd = d.seeds[st[w].y];
+      const uint32_t t = bstep(st[w]);
+      te[w] = st[w].w & 0xFFFFFFu;
+      W[w] = pair_walker(st[w].x, t, min(t + K, te[w]), sd.c, sd.b, sd.pos, seed_axis(sd.meta), seed_label(sd.meta),
+                         d.hits + (size_t)(st[w].w >> 24) * ((size_t)d.F * d.Zc));
     }
-    if (i < n_groups) {
-      PairWalker W[N];
-      uint32_t te[N], vol[N];
-      bool has[N];
+  }
+  walk_steps_multi<kFloat, N>(d.packed, W, k0, k1, s_delta, nz);
 #pragma unroll
-      for (uint32_t w = 0; w < N; ++w) {
-        const uint32_t idx = N * i + w;
-        has[w] = idx < n_live;
-        te[w] = 0u;
-        vol[w] = 0u;
-        W[w] = pair_walker(0u, 0u, 0u, 0.0f, 0.0f, 0u, 0u, 0u, nullptr);
-        if (has[w]) {
-          st[w] = states[idx];
-          vol[w] = bvol(st[w]);
-          const VolDesc& d = vols[vol[w]];
-          const SeedRec sd = d.seeds[st[w].y];
-          const uint32_t t = bstep(st[w]);
-          te[w] = st[w].w & 0xFFFFFFu;
-          W[w] = pair_walker(st[w].x, t, min(t + K, te[w]), sd.c, sd.b, sd.pos, seed_axis(sd.meta),
-                             seed_label(sd.meta), d.hits + (size_t)(st[w].w >> 24) * ((size_t)d.F * d.Zc));
-        }
-      }
-      const VolDesc& d0 = vols[vol[0]];
-      const int32_t* sdl0 = s_delta + 6 * vol[0];
-      if (kPair && has[N - 1] && vol[N - 1] == vol[0]) {
-        if (d0.is_float)
-          walk_steps_multi<true, N>(d0.packed, W, k0, k1, sdl0, nz);
-        else
-          walk_steps_multi<false, N>(d0.packed, W, k0, k1, sdl0, nz);
-      } else {
-#pragma unroll
-        for (uint32_t w = 0; w < N; ++w) {
-          if (!has[w]) continue;
-          const VolDesc& d = vols[vol[w]];
-          PairWalker& A = W[w];
-          if (d.is_float)
-            A.pos = walk_steps<true>(d.packed, A.pos, A.t, A.t_end, A.c, A.bf, A.seed_pos, A.axis, A.label, k0, k1,
-                                     A.hl, s_delta + 6 * vol[w], nz);
-          else
-            A.pos = walk_steps<false>(d.packed, A.pos, A.t, A.t_end, A.c, A.bf, A.seed_pos, A.axis, A.label, k0, k1,
-                                      A.hl, s_delta + 6 * vol[w], nz);
-        }
-      }
-#pragma unroll
-      for (uint32_t w = 0; w < N; ++w) {
-        if (!has[w]) continue;
-        st[w].x = W[w].pos;
-        st[w].z = W[w].t_end | (st[w].z & 0xFF000000u);
-        states[N * i + w] = st[w];
-        alive[w] = W[w].t_end != te[w];
-      }
+  for (int w = 0; w < N; ++w) {
+    const uint32_t j = threadIdx.x * (uint32_t)N + (uint32_t)w;
+    if (j < n) {
+      st[w].x = W[w].pos;
+      st[w].z = W[w].t_end | (st[w].z & 0xFF000000u);
+      states[first + j] = st[w];
+      alive[w] = W[w].t_end != te[w];
     }
-#pragma unroll
-    for (uint32_t w = 0; w < N; ++w) {
-      const uint32_t act = __ballot_sync(0xffffffffu, alive[w]);
-      if (alive[w]) {
-        const uint32_t key = bbucket(vols[bvol(st[w])], edge, st[w]);
-        const uint32_t peers = __match_any_sync(act, key);
-        if (lane == __ffs(peers) - 1) atomicAdd(&next_counts[key], (uint32_t)__popc(peers));
-      }
+    const uint32_t act = __ballot_sync(0xffffffffu, alive[w]);
+    if (alive[w]) {
+      const uint32_t key = bbucket(d, edge, st[w]);
+      const uint32_t peers = __match_any_sync(act, key);
+      if (lane == __ffs(peers) - 1) atomicAdd(&next_counts[key], (uint32_t)__popc(peers));
     }
   }
 }
@@ -1379,6 +1379,7 @@ struct BatchPlan {
   std::vector<si::VolDesc> vols;
   uint64_t walks = 0;
   uint32_t nbt = 0;
+  bool any_u8 = false, any_float = false;
   si::SortLayout layout{};
 };
 
@@ -1409,6 +1410,7 @@ int make_batch_plan(const si_volume_t* vols, int n_vols, int nbrw, int edge, con
     d.walk0 = walk;
     d.ns = ns_host ? (ns_host[v] < in.max_seeds ? ns_host[v] : in.max_seeds) : in.max_seeds;
     d.is_float = in.work_is_float;
+    (in.work_is_float ? P.any_float : P.any_u8) = true;
     d.by_F = si::FastDiv(d.F);
     d.by_X = si::FastDiv((uint32_t)in.Xc);
     bucket += (uint64_t)d.nb * in.nol;
@@ -1475,14 +1477,25 @@ extern "C" int si_walk_sorted_batch(const si_volume_t* vols, int n_vols, int nbr
   const FastDiv by_edge((uint32_t)sort_edge);
   // walker pairs unless mode 0
   const bool pairs = g_sweep_pairs.load(std::memory_order_relaxed) != 0;
-  // one group of walkers per thread, as in si_walk_sorted
-  const uint32_t blocks = (uint32_t)(((pairs ? (P.walks + 1) / 2 : P.walks) + 255) / 256);
   const uint32_t sort_blocks = (uint32_t)std::min<uint64_t>((uint64_t)sms * 8, (P.walks + 255) / 256);
   auto sweep = [&](cudaStream_t s, uint4* states) {
-    if (pairs)  // measured: 2 CTAs of 256 per SM (no spills) beat 3
-      bsweep_kernel<true, 2><<<blocks, 256, 0, s>>>(d_vols, n_vols, states, K, k0, k1, by_edge, w.counts, w.ctrs);
-    else
-      bsweep_kernel<false, 5><<<blocks, 256, 0, s>>>(d_vols, n_vols, states, K, k0, k1, by_edge, w.counts, w.ctrs);
+// every volume's last CTA may be partly filled
+#define SI_BSWEEP(F, N, T, MIN)                                                                                  \
+  bsweep_kernel<F, N, T, MIN><<<(uint32_t)((P.walks + N * T - 1) / (N * T)) + (uint32_t)n_vols, T, 0, s>>>(       \
+      d_vols, n_vols, P.nbt, w.offsets, states, K, k0, k1, by_edge, w.counts)
+    if (P.any_u8) {
+      if (pairs)
+        SI_BSWEEP(false, 2, 256, 3);
+      else
+        SI_BSWEEP(false, 1, 256, 5);
+    }
+    if (P.any_float) {
+      if (pairs)
+        SI_BSWEEP(true, 2, kFloatThreads, 3);
+      else
+        SI_BSWEEP(true, 1, 256, 5);
+    }
+#undef SI_BSWEEP
   };
   const uint32_t limit = round_limit();
   const ScanArgs a{w.counts, P.nbt, w.offsets, w.ctrs, limit, 0, {}};

@@ -76,3 +76,47 @@ def test_many_walks_in_one_sweep(cuda):
     assert np.array_equal(got["hits"], exp["hits"]) and np.array_equal(both[0]["hits"], exp["hits"])
     exp16 = O.smart_interpolation(img.astype(np.uint16), lab, key=9, **kw)
     assert np.array_equal(both[1]["hits"], exp16["hits"])
+
+
+@pytest.mark.parametrize("shift", [0, 16, 32])
+def test_float_records_aligned_to_16_bytes_only(shift, cuda):
+    """A record buffer that starts between two 32-byte boundaries."""
+    import torch
+
+    from biomedisa_gb300 import interpolation as I
+
+    img, lab = _volume((12, 15, 14), 4)
+    img = img.astype(np.float32)
+    ti, tl = I.upload(*I.normalize_host_dtypes(img, lab))
+    job = I.DeviceJob(ti, nat.SI_F32, tl, nat.SI_I32, nbrw=3, sorw=150, rng_seed=6)
+    assert job.analyze() is None
+    job.prepare()
+    cp = job.cplan
+    n = cp.voxels * 32
+    buf = torch.empty(n + 64, dtype=torch.uint8, device="cuda")
+    assert buf.data_ptr() % 64 == 0
+    packed = buf[shift:shift + n]
+    st = torch.cuda.current_stream().cuda_stream
+    nat.call("si_pack_neighbours", job.work.data_ptr(), 1, cp.Zc, cp.Yc, cp.Xc, packed.data_ptr(), st)
+    job.hits = torch.zeros((job.lplan.nol, cp.Zc, cp.Yc, cp.Xc), dtype=torch.int32, device="cuda")
+    I.walk_sorted(packed, True, cp.Zc, cp.Yc, cp.Xc, job.seeds, job.n_seeds, job.seed_capacity, 3, 150, 6, job.hits,
+                  job.lplan.nol)
+    exp = O.smart_interpolation(img, lab, key=6, nbrw=3, sorw=150, return_hits=True)
+    assert np.array_equal(job.hits_full().cpu().numpy(), exp["hits"])
+
+
+def test_batch_of_many_volumes(cuda):
+    """130 volumes (more than one per thread of a float CTA), some without a
+    walker of a kind, each equal to its own call."""
+    rng = np.random.default_rng(4)
+    imgs, labs = [], []
+    for k in range(130):
+        shape = tuple(int(v) for v in rng.integers(4, 10, 3))
+        img, lab = _volume(shape, k)
+        imgs.append(img if k % 3 else img.astype(np.float32))
+        labs.append(lab)
+    kw = dict(nbrw=2, sorw=70, return_hits=True, rng_seed=12)
+    got = smart_interpolation_batch(imgs, labs, autotune_params=False, **kw)
+    for img, lab, g in zip(imgs, labs, got):
+        one = smart_interpolation(img, lab, walker="packed", **kw)
+        assert np.array_equal(g["hits"], one["hits"])
