@@ -152,7 +152,7 @@ __global__ void __launch_bounds__(256) remap_kernel(uint8_t* __restrict__ out, P
 // tensor copies; the destination may have any row pitch.
 //
 // Schedule: a CTA of 256 threads owns a 64 x 8 column of voxels and marches
-// through kSZ planes in z. Planes arrive in a ring of four shared-memory slots
+// through `planes` planes in z (smooth_planes). Planes arrive in a ring of four shared-memory slots
 // by TMA (one 72 x 10 box per plane: x from x0 - 4 so the copy starts on 16
 // bytes, y from y0 - 1; out-of-volume parts read as zero), issued by one
 // thread two planes ahead of use and completed on per-slot mbarriers. Each
@@ -160,7 +160,10 @@ __global__ void __launch_bounds__(256) remap_kernel(uint8_t* __restrict__ out, P
 // the packed binary32 pipe (add/sub/mul.rn.f32x2: per lane the same IEEE
 // operation as the scalar form). Of the 19 stencil values a voxel needs, the
 // 10 of planes z-1 and z are carried in registers from the previous plane, so
-// a plane step loads 9 values per voxel from shared memory.
+// a plane step loads 9 values per voxel from shared memory. Instructions bound
+// it on large volumes (issue 79 % busy at 139 per voxel); unrolled by three, so
+// that the planes' registers change roles instead of being moved, 121 per voxel:
+// 402x514x514 441 -> 422 us dense, 373 -> 361 us on a hit map.
 //
 // Support box: values outside the box of non-(+0) source values grown by
 // one voxel per iteration are exactly +0 (all differences +0, kappa =
@@ -170,7 +173,7 @@ __global__ void __launch_bounds__(256) remap_kernel(uint8_t* __restrict__ out, P
 // ---------------------------------------------------------------------------
 // kP packed pairs per thread: the CTA's column is 64 * kP voxels wide
 // (voxels x0 + tx + 32 j, j < 2 kP; pair p = columns 2p and 2p + 1).
-constexpr int kSY = 8, kSZ = 32;
+constexpr int kSY = 8;
 template <int kP>
 struct SmoothTile {
   static constexpr int kSX = 64 * kP;
@@ -247,16 +250,25 @@ __global__ void __launch_bounds__(256, kP == 1 ? 3 : 2) smooth_tma_kernel(const 
                                                                          float* __restrict__ dst, int dst_pitch,
                                                                          int Zc, int Yc, int Xc,
                                                                          const int* __restrict__ box, int grow,
-                                                                         int write_outside, uint32_t wait_lim) {
+                                                                         int write_outside, int planes,
+                                                                         uint32_t wait_lim) {
   using T = SmoothTile<kP>;
   constexpr int kBoxX = T::kBoxX;
   __shared__ __align__(128) float pl[kSlots][T::kSlotFloats];
   __shared__ __align__(8) uint64_t bar[kSlots];
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-  const int x0 = blockIdx.x * T::kSX, y0 = blockIdx.y * kSY, zb = blockIdx.z * kSZ;
-  const int ze = min(zb + kSZ, Zc);
+  const int x0 = blockIdx.x * T::kSX, y0 = blockIdx.y * kSY, zb = blockIdx.z * planes;
+  const int ze = min(zb + planes, Zc);
   const int y = y0 + ty;
   const size_t dF = (size_t)Yc * dst_pitch;
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < kSlots; ++s) mbar_init(&bar[s], 1);
+    fence_barrier_init();
+  }
+  // the step before this one has written its maps and read this one's
+  // destination; the next step may be set up meanwhile
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   if (box_outside(box, grow, zb, ze - 1, y0, min(y0 + kSY, Yc) - 1, x0, min(x0 + T::kSX, Xc) - 1)) {
     if (write_outside && y < Yc) {
       for (int z = zb; z < ze; ++z) {
@@ -269,10 +281,6 @@ __global__ void __launch_bounds__(256, kP == 1 ? 3 : 2) smooth_tma_kernel(const 
     return;
   }
   const int nq = ze - zb + 2;  // planes zb-1 .. ze; plane zb-1+q sits in slot q & 3
-  if (threadIdx.x == 0) {
-    for (int s = 0; s < kSlots; ++s) mbar_init(&bar[s], 1);
-    fence_barrier_init();
-  }
   __syncthreads();
   int issued = 0;  // meaningful in thread 0 only
   if (threadIdx.x == 0) {
@@ -294,25 +302,33 @@ __global__ void __launch_bounds__(256, kP == 1 ? 3 : 2) smooth_tma_kernel(const 
   };
   auto wait_q = [&](int q) { return mbar_wait_bounded(&bar[q & 3], (uint32_t)(q >> 2) & 1u, wait_lim); };
 
-  uint64_t m_c[kP], m_xm[kP], m_xp[kP], m_ym[kP], m_yp[kP];  // plane z-1
-  uint64_t c_c[kP], c_xm[kP], c_xp[kP], c_ym[kP], c_yp[kP];  // plane z
+  // cross values of three planes; the roles z-1, z, z+1 rotate, the registers
+  // stay (steps are unrolled by three)
+  struct Cross {
+    uint64_t c[kP], xm[kP], xp[kP], ym[kP], yp[kP];
+  };
+  Cross S0, S1, S2;
 #pragma unroll
-  for (int p = 0; p < kP; ++p) m_c[p] = m_xm[p] = m_xp[p] = m_ym[p] = m_yp[p] = c_c[p] = c_xm[p] = c_xp[p] = c_ym[p] =
-      c_yp[p] = 0;
+  for (int p = 0; p < kP; ++p) {
+    S0.c[p] = S0.xm[p] = S0.xp[p] = S0.ym[p] = S0.yp[p] = 0;
+    S1 = S0;
+    S2 = S0;
+  }
   bool ok = wait_q(0);
   ok = ok && wait_q(1);
   if (ok) {
 #pragma unroll
     for (int p = 0; p < kP; ++p) {
-      cross(pl[0], p, m_c[p], m_xm[p], m_xp[p], m_ym[p], m_yp[p]);
-      cross(pl[1], p, c_c[p], c_xm[p], c_xp[p], c_ym[p], c_yp[p]);
+      cross(pl[0], p, S0.c[p], S0.xm[p], S0.xp[p], S0.ym[p], S0.yp[p]);
+      cross(pl[1], p, S1.c[p], S1.xm[p], S1.xp[p], S1.ym[p], S1.yp[p]);
     }
   }
-  const uint64_t two = f2_splat(2.0f), half = f2_splat(0.5f), quarter = f2_splat(0.25f);
+  const uint64_t half = f2_splat(0.5f), quarter = f2_splat(0.25f);
   const uint64_t eps = f2_splat(1e-10f), hundredth = f2_splat(0.01f);
   const uint64_t nz = f2_negzero();  // products as fma(a, b, -0): never fused into a later sum
   const bool row_in = y < Yc, row_interior = y > 0 && y < Yc - 1;
-  for (int k = 0; k < ze - zb; ++k) {
+  const int n = ze - zb;
+  auto step = [&](int k, Cross& M, Cross& Q, Cross& N) -> bool {  // planes z-1, z, z+1
     const int z = zb + k;
     ok = ok && wait_q(k + 2);
     if (ok) {
@@ -327,31 +343,31 @@ __global__ void __launch_bounds__(256, kP == 1 ? 3 : 2) smooth_tma_kernel(const 
         const uint64_t k_pp = f2_pack(C[ia + kBoxX + 1], C[ib + kBoxX + 1]);
         const uint64_t k_mp = f2_pack(C[ia - kBoxX + 1], C[ib - kBoxX + 1]);
         const uint64_t k_pm = f2_pack(C[ia + kBoxX - 1], C[ib + kBoxX - 1]);
-        uint64_t p_c, p_xm, p_xp, p_ym, p_yp;  // plane z+1
-        cross(Pn, p, p_c, p_xm, p_xp, p_ym, p_yp);
-        const uint64_t c2 = f2_mul(two, c_c[p], nz);
-        const uint64_t dx = f2_mul(f2_sub(c_xm[p], c_xp[p]), half, nz);
-        const uint64_t dxx = f2_add(f2_sub(c_xm[p], c2), c_xp[p]);
+        cross(Pn, p, N.c[p], N.xm[p], N.xp[p], N.ym[p], N.yp[p]);
+        const uint64_t c2 = f2_add(Q.c[p], Q.c[p]);  // 2 c, exact
+        const uint64_t dx = f2_mul(f2_sub(Q.xm[p], Q.xp[p]), half, nz);
+        const uint64_t dxx = f2_add(f2_sub(Q.xm[p], c2), Q.xp[p]);
         const uint64_t dx2 = f2_mul(dx, dx, nz);
-        const uint64_t dy = f2_mul(f2_sub(c_ym[p], c_yp[p]), half, nz);
-        const uint64_t dyy = f2_add(f2_sub(c_ym[p], c2), c_yp[p]);
+        const uint64_t dy = f2_mul(f2_sub(Q.ym[p], Q.yp[p]), half, nz);
+        const uint64_t dyy = f2_add(f2_sub(Q.ym[p], c2), Q.yp[p]);
         const uint64_t dy2 = f2_mul(dy, dy, nz);
-        const uint64_t dz = f2_mul(f2_sub(m_c[p], p_c), half, nz);
-        const uint64_t dzz = f2_add(f2_sub(m_c[p], c2), p_c);
+        const uint64_t dz = f2_mul(f2_sub(M.c[p], N.c[p]), half, nz);
+        const uint64_t dzz = f2_add(f2_sub(M.c[p], c2), N.c[p]);
         const uint64_t dz2 = f2_mul(dz, dz, nz);
         const uint64_t dxy = f2_mul(f2_sub(f2_sub(f2_add(k_mm, k_pp), k_mp), k_pm), quarter, nz);
-        const uint64_t dxz = f2_mul(f2_sub(f2_sub(f2_add(p_xm, m_xp[p]), p_xp), m_xm[p]), quarter, nz);
-        const uint64_t dyz = f2_mul(f2_sub(f2_sub(f2_add(p_ym, m_yp[p]), p_yp), m_ym[p]), quarter, nz);
+        const uint64_t dxz = f2_mul(f2_sub(f2_sub(f2_add(N.xm[p], M.xp[p]), N.xp[p]), M.xm[p]), quarter, nz);
+        const uint64_t dyz = f2_mul(f2_sub(f2_sub(f2_add(N.ym[p], M.yp[p]), N.yp[p]), M.ym[p]), quarter, nz);
         uint64_t num = f2_add(f2_mul(dxx, f2_add(dy2, dz2), nz), f2_mul(dyy, f2_add(dx2, dz2), nz));
         num = f2_add(num, f2_mul(dzz, f2_add(dx2, dy2), nz));
-        num = f2_sub(num, f2_mul(f2_mul(f2_mul(two, dx, nz), dy, nz), dxy, nz));
-        num = f2_sub(num, f2_mul(f2_mul(f2_mul(two, dx, nz), dz, nz), dxz, nz));
-        num = f2_sub(num, f2_mul(f2_mul(f2_mul(two, dy, nz), dz, nz), dyz, nz));
+        const uint64_t tx2 = f2_add(dx, dx);  // 2 dx, exact
+        num = f2_sub(num, f2_mul(f2_mul(tx2, dy, nz), dxy, nz));
+        num = f2_sub(num, f2_mul(f2_mul(tx2, dz, nz), dxz, nz));
+        num = f2_sub(num, f2_mul(f2_mul(f2_add(dy, dy), dz, nz), dyz, nz));
         const uint64_t den = f2_add(f2_add(f2_add(dx2, dy2), dz2), eps);
         float na, nb, da, db, ca, cb;
         f2_unpack(num, na, nb);
         f2_unpack(den, da, db);
-        f2_unpack(c_c[p], ca, cb);
+        f2_unpack(Q.c[p], ca, cb);
         // den >= 1e-10 > 0, so a zero numerator gives kappa = num (its sign
         // kept) exactly; flat neighbourhoods (zero regions of a hit map) skip
         // the division
@@ -365,13 +381,11 @@ __global__ void __launch_bounds__(256, kP == 1 ? 3 : 2) smooth_tma_kernel(const 
           oa = __double2float_rn(__dadd_rn((double)ca, __dmul_rn(0.01, (double)ka)));
           ob = __double2float_rn(__dadd_rn((double)cb, __dmul_rn(0.01, (double)kb)));
         } else {
-          f2_unpack(f2_add(c_c[p], f2_mul(hundredth, f2_pack(ka, kb), nz)), oa, ob);
+          f2_unpack(f2_add(Q.c[p], f2_mul(hundredth, f2_pack(ka, kb), nz)), oa, ob);
         }
         const int xa = x0 + tx + 64 * p, xb = xa + 32;
         if (row_in && xa < Xc) row[xa] = (z_int && row_interior && xa > 0 && xa < Xc - 1) ? oa : ca;
         if (row_in && xb < Xc) row[xb] = (z_int && row_interior && xb > 0 && xb < Xc - 1) ? ob : cb;
-        m_c[p] = c_c[p]; m_xm[p] = c_xm[p]; m_xp[p] = c_xp[p]; m_ym[p] = c_ym[p]; m_yp[p] = c_yp[p];
-        c_c[p] = p_c; c_xm[p] = p_xm; c_xp[p] = p_xp; c_ym[p] = p_ym; c_yp[p] = p_yp;
       }
     }
     if (__syncthreads_or(!ok)) {
@@ -382,7 +396,7 @@ __global__ void __launch_bounds__(256, kP == 1 ? 3 : 2) smooth_tma_kernel(const 
           mbar_wait_bounded(&bar[q & 3], (uint32_t)(q >> 2) & 1u, kDrainWaitLimit);
         atomicOr(&g_smooth_status, 1u);
       }
-      return;
+      return false;
     }
     // the slot of plane q = k was last read in step k - 1 (or the prologue): refill it
     if (threadIdx.x == 0 && issued < nq) {
@@ -391,7 +405,10 @@ __global__ void __launch_bounds__(256, kP == 1 ? 3 : 2) smooth_tma_kernel(const 
       tma_load_box(pl[issued & 3], &src, x0 - 4, y0 - 1, zb - 1 + issued, &bar[issued & 3]);
       ++issued;
     }
-  }
+    return k + 1 < n;
+  };
+  for (int k = 0;; k += 3)
+    if (!step(k, S0, S1, S2) || !step(k + 1, S1, S2, S0) || !step(k + 2, S2, S0, S1)) return;
 }
 
 __global__ void __launch_bounds__(256) u32_to_f32_kernel(const uint32_t* __restrict__ src, float* __restrict__ dst,
@@ -464,6 +481,37 @@ int encode_volume_map(CUtensorMap* map, float* base, int Zc, int Yc, int Xc, int
   return SI_OK;
 }
 
+// Planes a CTA marches through: 32, or fewer where that leaves fewer than five
+// waves of CTAs (3 per SM): a step then lasts as long as one column takes,
+// about 0.7 us a plane. Two planes more than it writes are read per CTA, so
+// large volumes keep long columns. One step on a hit map, 32 / 16 / 8 / 4
+// planes, each started after the one before it: 42x38x35 23.8 / 14.7 / 9.9 /
+// 7.8 us, 130^3 34.5 / 24.7 / 20.5 / 20.0, 178x226x210 53.5 / 47.9 / 45.9 / 47.6,
+// 402x514x514 375 / 375 / 386 / 420.
+int smooth_planes(int columns, int Zc) {
+  const int want = 5 * 3 * sm_count();
+  int planes = 32;
+  while (planes > 4 && (long long)columns * ((Zc + planes - 1) / planes) < want) planes /= 2;
+  return planes;
+}
+
+// One smoothing step, allowed to start while the step before it drains: its
+// CTAs set up their barriers and wait (griddepcontrol.wait) before they touch
+// the maps. 42x38x35 7.8 -> 5.4 us a step, 130^3 20.0 -> 17.2.
+template <class... Params, class... Args>
+cudaError_t launch_step(void (*kernel)(Params...), dim3 grid, cudaStream_t st, Args... args) {
+  cudaLaunchAttribute attr = {};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(256);
+  cfg.stream = st;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
+}
+
 // Smoothing of nol maps (uint32 hits when kSrcU32, else float32) of
 // Zc*Yc*Xc voxels; results as float32 in place. tmp0 holds the pitched
 // source of odd iterations, tmp1 its 64-float head (the support box) and the
@@ -487,7 +535,9 @@ int smooth_maps(void* maps, float* tmp0, float* tmp1, int nol, int Zc, int Yc, i
     rc = encode_volume_map(&map1, tmp1v, Zc, Yc, Xc, sx + 8, what);
     if (rc) return rc;
   }
-  const dim3 grid((Xc + sx - 1) / sx, (Yc + kSY - 1) / kSY, (Zc + kSZ - 1) / kSZ);
+  const int columns = ((Xc + sx - 1) / sx) * ((Yc + kSY - 1) / kSY);
+  const int planes = smooth_planes(columns, Zc);
+  const dim3 grid((Xc + sx - 1) / sx, (Yc + kSY - 1) / kSY, (Zc + planes - 1) / planes);
   const int cgrid = std::max(1, std::min(sm_count() * 8, (Zc * Yc + 7) / 8));
   const uint32_t wl = wait_limit();
   for (int l = 0; l < nol; ++l) {
@@ -508,18 +558,22 @@ int smooth_maps(void* maps, float* tmp0, float* tmp1, int nol, int Zc, int Yc, i
       // only iteration 1's destination (tmp1) may hold another map's values
       // outside the support; every later destination is +0 there already
       const int write_outside = (it == 1 && !last) ? 1 : 0;
-#define SI_SMOOTH(F64, P) \
-  smooth_tma_kernel<F64, P><<<grid, 256, 0, st>>>(sm, dst, pitch, Zc, Yc, Xc, box, it, write_outside, wl)
+#define SI_SMOOTH(F64, P)                                                                                          \
+  if (launch_step(smooth_tma_kernel<F64, P>, grid, st, sm, dst, pitch, Zc, Yc, Xc, box, it, write_outside, planes, \
+                  wl) != cudaSuccess)                                                                              \
+  return check_launch(what)
       if (update) {
-        if (kp == 2)
+        if (kp == 2) {
           SI_SMOOTH(true, 2);
-        else
+        } else {
           SI_SMOOTH(true, 1);
+        }
       } else {
-        if (kp == 2)
+        if (kp == 2) {
           SI_SMOOTH(false, 2);
-        else
+        } else {
           SI_SMOOTH(false, 1);
+        }
       }
 #undef SI_SMOOTH
     }
