@@ -23,8 +23,12 @@ def _scratch(shape, device):
 
 def present_labels(labels: torch.Tensor) -> list[int]:
     """Ascending label values present in a uint8 volume (the reference's unique())."""
-    counts = torch.bincount(labels.reshape(-1).to(torch.int64), minlength=256)
-    return [int(v) for v in torch.nonzero(counts).flatten().tolist()]
+    if not labels.is_cuda:
+        return [int(v) for v in torch.nonzero(torch.bincount(labels.reshape(-1).to(torch.int64))).flatten().tolist()]
+    labels = labels.contiguous()
+    hist = torch.zeros(258, dtype=torch.int64, device=labels.device)
+    nat.call("si_label_histogram", labels.data_ptr(), nat.SI_U8, labels.numel(), hist.data_ptr(), _stream())
+    return [v for v, n in enumerate(hist[:256].tolist()) if n]
 
 
 def clean(labels: torch.Tensor, threshold: float = 0.1) -> torch.Tensor:
