@@ -173,8 +173,6 @@ constexpr int kBoxP = kTileP + 7, kBoxQ = kTileQ + 3, kBoxR = kTileR + 1;
 constexpr int kBoxCells = kBoxP * kBoxQ * kBoxR;
 constexpr int kTileThreads = kTileQ * kTileR;
 constexpr size_t kTileSmem = 2 * sizeof(float) * kBoxCells;
-constexpr int kStageBatch = 8;
-constexpr int kStageRounds = (kBoxCells + kTileThreads - 1) / kTileThreads;  // cells per thread, rounded up
 
 struct GeoTiling {
   int s;             // +1 forward, -1 backward
@@ -197,6 +195,22 @@ __host__ __device__ inline GeoTiling geo_tiling(int Z, int Y, int X, int fwd) {
   g.ntq = (qmax - qmin + kTileQ) / kTileQ;
   g.ntr = (g.zhi - g.zlo + kTileR) / kTileR;
   return g;
+}
+
+// Tiles iq of row ir that can hold voxels of the domain on tile-wavefront S:
+// [*lo, *hi], empty when *hi < *lo. With u = q - 2 r = s y and v = p - 2 q = s x
+// in [1, Y - 2] and [1, X - 2] (negated on the backward pass), the tile's q and p
+// ranges have to meet those of its r and q.
+__host__ __device__ inline void geo_tile_row(const GeoTiling& g, int Y, int X, int S, int ir, int* lo, int* hi) {
+  const int r0 = g.rb + ir * kTileR, r1 = imin(r0 + kTileR - 1, g.rb + g.zhi - g.zlo);
+  const int ulo = g.s > 0 ? 1 : -(Y - 2), uhi = g.s > 0 ? Y - 2 : -1;
+  const int vlo = g.s > 0 ? 1 : -(X - 2), vhi = g.s > 0 ? X - 2 : -1;
+  const int t = g.pb + (S - ir) * kTileP - 2 * g.qb;  // p0 - 2 q0 at iq = 0
+  constexpr int step = kTileP + 2 * kTileQ;           // and what it loses per tile
+  *lo = imax(imax(0, S - ir - (g.ntp - 1)),
+             imax(floor_div(2 * r0 + ulo - g.qb, kTileQ), ceil_div(t - 2 * (kTileQ - 1) - vhi, step)));
+  *hi = imin(imin(g.ntq - 1, S - ir), imin(floor_div(2 * r1 + uhi - g.qb, kTileQ),
+                                           floor_div(t + kTileP - 1 - vlo, step)));
 }
 
 // Volume coordinates of transformed (p, q, r).
@@ -224,87 +238,172 @@ inline int geo_box_offset(int n) {
   return geo_box_cell(dx + 2 * dy + 4 * dz, dy + 2 * dz, dz);
 }
 
+// Asynchronous copy of one float to shared memory.
+__device__ __forceinline__ void copy_async_f32(float* dst, const float* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src)
+               : "memory");
+}
+
+// Starts the copies of one box of a volume: a warp takes box rows of equal
+// (q, r), which run along x; from one q to the next the row moves by one y and
+// two x. Cells outside the volume are left as they are: no voxel of the domain
+// has a neighbour there.
+__device__ __forceinline__ void geo_stage_box(const GeoScanArgs& a, const GeoTiling& g, const float* vol, float* box,
+                                              int p0, int q0, int r0) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  constexpr int kWarps = kTileThreads / 32;
+  const long long dq = (long long)kWarps * g.s * (a.X - 2);
+  for (int br = 0; br < kBoxR; ++br) {
+    int z, y, x;
+    geo_unskew(g, p0, q0 + warp, r0 + br, &z, &y, &x);
+    if (z < 0 || z >= a.Z) continue;
+    x += g.s * lane;
+    const float* src = vol + ((long long)z * a.Y + y) * a.X + x;
+    float* dst = box + (br * kBoxQ + warp) * kBoxP + lane;
+#pragma unroll
+    for (int bq = warp; bq < kBoxQ; bq += kWarps) {
+      const bool in = y >= 0 && y < a.Y;
+      if (in && x >= 0 && x < a.X) copy_async_f32(dst, src);
+      const int x2 = x + 32 * g.s;
+      if (in && lane < kBoxP - 32 && x2 >= 0 && x2 < a.X) copy_async_f32(dst + 32, src + 32 * g.s);
+      y += g.s * kWarps;
+      x -= 2 * g.s * kWarps;
+      src += dq;
+      dst += kWarps * kBoxP;
+    }
+  }
+}
+
+// What bounds it: a scan is a chain of tile-wavefronts (416 on 120x131x125),
+// each as long as one tile takes. A tile's 32 planes follow one another behind
+// a CTA barrier, so a plane keeps only three of the 13 costs behind it: those
+// of the neighbours updated in the plane before (its own column, and the columns
+// q-1 of r and r-1). A column's y and z are fixed and x runs along p, so the
+// other ten neighbours are values that moved through registers (three per
+// neighbour column, one new load per column and plane); their minimum is formed
+// before the barrier. Boxes come by asynchronous copies, the image's while the
+// wavefront before still runs (programmatic launch). 23.5 us per tile-wavefront
+// with 26 loads and the index arithmetic of every voxel behind the barrier.
 template <bool kLamb1>
-__global__ void __launch_bounds__(kTileThreads) geo_tile_kernel(GeoScanArgs a, GeoTiling g, int S) {
+__global__ void __launch_bounds__(kTileThreads) geo_tile_kernel(GeoScanArgs a, GeoTiling g, int S, int ir0) {
   extern __shared__ float smem[];
   float* sc = smem;              // distances of the box
   float* si = smem + kBoxCells;  // image of the box
-  const int iq = blockIdx.x % g.ntq, ir = blockIdx.x / g.ntq;
+  const int ir = ir0 + (int)blockIdx.y;
+  int iq, iq_hi;
+  geo_tile_row(g, a.Y, a.X, S, ir, &iq, &iq_hi);
+  iq += (int)blockIdx.x;
+  if (iq > iq_hi) return;  // uniform over the CTA
   const int ip = S - iq - ir;
-  if (ip < 0 || ip >= g.ntp || ir >= g.ntr) return;  // uniform over the CTA
-  float* cl = a.c + (long long)blockIdx.y * a.V;
+  float* cl = a.c + (long long)blockIdx.z * a.V;
   const int cq = threadIdx.x % kTileQ, cr = threadIdx.x / kTileQ;
-  bool any = false;
-  for (int k = 0; k < kTileP; ++k) {
-    int z, y, x;
-    any = any || geo_tile_voxel(g, a.Y, a.X, ip, iq, ir, cq, cr, k, &z, &y, &x);
-  }
-  if (!__syncthreads_or(any)) return;  // no voxel of the domain in this tile
+  // steps of this column inside the domain: x = x0 + s k in [1, X - 2]
+  int z, y, x0;
+  geo_unskew(g, g.pb + ip * kTileP, g.qb + iq * kTileQ + cq, g.rb + ir * kTileR + cr, &z, &y, &x0);
+  int k_lo = g.s > 0 ? 1 - x0 : x0 - (a.X - 2), k_hi = g.s > 0 ? a.X - 2 - x0 : x0 - 1;
+  k_lo = imax(k_lo, 0);
+  k_hi = imin(k_hi, kTileP - 1);
+  if (z < g.zlo || z > g.zhi || y < 1 || y > a.Y - 2) k_hi = -1;
+  if (!__syncthreads_or(k_lo <= k_hi)) return;  // no voxel of the domain in this tile
   const int p0 = g.pb + ip * kTileP - 7, q0 = g.qb + iq * kTileQ - 3, r0 = g.rb + ir * kTileR - 1;
-  // staging in batches of kStageBatch cells per thread: all loads of a batch
-  // are issued before the first shared-memory store waits for one
-  for (int b = 0; b < kStageRounds; b += kStageBatch) {
-    float vc[kStageBatch], vi[kStageBatch];
-#pragma unroll
-    for (int u = 0; u < kStageBatch; ++u) {
-      const int cell = threadIdx.x + (b + u) * kTileThreads;
-      vc[u] = __uint_as_float(0x7f800000u);
-      vi[u] = 0.0f;
-      if (cell < kBoxCells) {
-        const int bp = cell % kBoxP, bq = (cell / kBoxP) % kBoxQ, br = cell / (kBoxP * kBoxQ);
-        int z, y, x;
-        geo_unskew(g, p0 + bp, q0 + bq, r0 + br, &z, &y, &x);
-        if (z >= 0 && z < a.Z && y >= 0 && y < a.Y && x >= 0 && x < a.X) {
-          const long long v = ((long long)z * a.Y + y) * a.X + x;
-          vc[u] = cl[v];
-          vi[u] = a.img[v];
-        }
-      }
-    }
-#pragma unroll
-    for (int u = 0; u < kStageBatch; ++u) {
-      const int cell = threadIdx.x + (b + u) * kTileThreads;
-      if (cell < kBoxCells) {
-        sc[cell] = vc[u];
-        si[cell] = vi[u];
-      }
-    }
-  }
+  geo_stage_box(a, g, a.img, si, p0, q0, r0);
+  // the wavefront before has written its distances; the next may start on its image
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  geo_stage_box(a, g, cl, sc, p0, q0, r0);
+  asm volatile("cp.async.wait_all;" ::: "memory");
   __syncthreads();
-  for (int k = 0; k < kTileP; ++k) {
-    int z, y, x;
-    if (geo_tile_voxel(g, a.Y, a.X, ip, iq, ir, cq, cr, k, &z, &y, &x)) {
-      const int own = geo_box_cell(k + 7, cq + 3, cr + 1);
-      const float iv = si[own];
-      if (kLamb1) {
-        float best = sc[own];
+  const int own = geo_box_cell(7, cq + 3, cr + 1);
+  if constexpr (kLamb1) {
+    // neighbour columns and the steps they are read at, relative to this one:
+    // B (q-1, r) and E (q-1, r-1) at -3, -2, -1, C (q-3, r-1) at -7, -6, -5,
+    // D (q-2, r-1) at -5, -4, -3, and the own column at -1
+    const int B = geo_box_cell(7, cq + 2, cr + 1), C = geo_box_cell(7 - 4, cq, cr), D = geo_box_cell(7 - 2, cq + 1, cr),
+              E = geo_box_cell(7, cq + 2, cr);
+    float bc[3], bi[3], cc[3], ci[3], dc[3], di[3], ec[3], ei[3];  // [j]: step k - 3 + j of the (shifted) column
+#pragma unroll
+    for (int j = 0; j < 3; ++j) {
+      bi[j] = si[B - 3 + j];
+      ci[j] = si[C - 3 + j];
+      di[j] = si[D - 3 + j];
+      ei[j] = si[E - 3 + j];
+      cc[j] = sc[C - 3 + j];
+      dc[j] = sc[D - 3 + j];
+      bc[j] = j < 2 ? sc[B - 3 + j] : 0.0f;
+      ec[j] = j < 2 ? sc[E - 3 + j] : 0.0f;
+    }
+    float iv = si[own], li = si[own - 1], lc = sc[own - 1], oc = sc[own];
+    auto sq = [&](float i) {
+      const float d = __fsub_rn(iv, i);
+      return __fmul_rn(d, d);
+    };
+    // costs of a plane before its barrier: the ten older neighbours (a NaN cost
+    // is never taken and fminf drops it; an own NaN stays, no comparison with it
+    // being true; no cost is -0, squares being +0 or more)
+    auto older = [&]() {
+      float m = fminf(fminf(__fadd_rn(bc[0], sq(bi[0])), __fadd_rn(bc[1], sq(bi[1]))),
+                      fminf(__fadd_rn(ec[0], sq(ei[0])), __fadd_rn(ec[1], sq(ei[1]))));
+#pragma unroll
+      for (int j = 0; j < 3; ++j) {
+        m = fminf(m, fminf(__fadd_rn(cc[j], sq(ci[j])), __fadd_rn(dc[j], sq(di[j]))));
+      }
+      return m;
+    };
+    float pre = older(), sb = sq(bi[2]), se = sq(ei[2]), sl = sq(li);
+#pragma unroll 3
+    for (int k = 0; k < kTileP; ++k) {
+      bc[2] = sc[B + k - 1];
+      ec[2] = sc[E + k - 1];
+      const float m = fminf(fminf(pre, __fadd_rn(lc, sl)), fminf(__fadd_rn(bc[2], sb), __fadd_rn(ec[2], se)));
+      const bool in = k >= k_lo && k <= k_hi;
+      lc = in && m < oc ? m : oc;
+      if (in) sc[own + k] = lc;
+      // the next plane (its loads end inside the box: k + 1 <= 32 of 39 - 7)
+      if (k + 1 < kTileP) {
+        li = iv;
+        iv = si[own + k + 1];
+        oc = sc[own + k + 1];
+        bc[0] = bc[1]; bc[1] = bc[2];
+        ec[0] = ec[1]; ec[1] = ec[2];
+        bi[0] = bi[1]; bi[1] = bi[2]; bi[2] = si[B + k];
+        ei[0] = ei[1]; ei[1] = ei[2]; ei[2] = si[E + k];
+        ci[0] = ci[1]; ci[1] = ci[2]; ci[2] = si[C + k];
+        di[0] = di[1]; di[1] = di[2]; di[2] = si[D + k];
+        cc[0] = cc[1]; cc[1] = cc[2]; cc[2] = sc[C + k];
+        dc[0] = dc[1]; dc[1] = dc[2]; dc[2] = sc[D + k];
+        pre = older();
+        sb = sq(bi[2]);
+        se = sq(ei[2]);
+        sl = sq(li);
+      }
+      __syncthreads();
+    }
+  } else {
+    for (int k = 0; k < kTileP; ++k) {
+      if (k >= k_lo && k <= k_hi) {
+        const int at = own + k;
+        const float iv = si[at];
+        double best = (double)sc[at];
 #pragma unroll
         for (int n = 0; n < 13; ++n) {
-          const int nb = own + a.box_off[n];
-          const float diff = __fsub_rn(iv, si[nb]);
-          const float cost = __fadd_rn(sc[nb], __fmul_rn(diff, diff));
-          if (cost < best) best = cost;
-        }
-        sc[own] = best;
-      } else {
-        double best = (double)sc[own];
-#pragma unroll
-        for (int n = 0; n < 13; ++n) {
-          const int nb = own + a.box_off[n];
+          const int nb = at + a.box_off[n];
           const float diff = __fsub_rn(iv, si[nb]);
           const double sq = (double)__fmul_rn(diff, diff);
           const double cost = __dadd_rn(__dadd_rn((double)sc[nb], a.w[n]), __dmul_rn(a.lamb, sq));
           if (cost < best) best = cost;
         }
-        sc[own] = __double2float_rn(best);
+        sc[at] = __double2float_rn(best);
       }
+      __syncthreads();
     }
-    __syncthreads();
   }
-  for (int k = 0; k < kTileP; ++k) {
-    int z, y, x;
-    if (geo_tile_voxel(g, a.Y, a.X, ip, iq, ir, cq, cr, k, &z, &y, &x))
-      cl[((long long)z * a.Y + y) * a.X + x] = sc[geo_box_cell(k + 7, cq + 3, cr + 1)];
+  // a warp writes its plane's columns one after the other, along x
+  const int lane = threadIdx.x & 31;
+#pragma unroll 4
+  for (int j = 0; j < kTileQ; ++j) {
+    geo_unskew(g, g.pb + ip * kTileP + lane, g.qb + iq * kTileQ + j, g.rb + ir * kTileR + cr, &z, &y, &x0);
+    if (z >= g.zlo && z <= g.zhi && y >= 1 && y <= a.Y - 2 && x0 >= 1 && x0 <= a.X - 2)
+      cl[((long long)z * a.Y + y) * a.X + x0] = sc[geo_box_cell(7 + lane, j + 3, cr + 1)];
   }
 }
 
@@ -599,17 +698,39 @@ int geo_tile_prepare() {
 // (tiled) or one per wavefront.
 int geo_launch_scan(const GeoScanArgs& a, bool lamb1, int iterations, bool tiled, cudaStream_t st) {
   if (tiled) {
+    bool first = true;
     for (int it = 0; it < iterations; ++it)
       for (int fwd = 1; fwd >= 0; --fwd) {
         const GeoTiling g = geo_tiling(a.Z, a.Y, a.X, fwd);
-        const long long ncta = (long long)g.ntq * g.ntr;
-        if (ncta > 0x7fffffffLL) return set_error(SI_ERR_LIMIT, "si_geo_scan: too many tiles");
-        const dim3 grid((unsigned)ncta, (unsigned)a.nol);
         for (int S = 0; S <= g.ntp + g.ntq + g.ntr - 3; ++S) {
-          if (lamb1)
-            geo_tile_kernel<true><<<grid, kTileThreads, kTileSmem, st>>>(a, g, S);
-          else
-            geo_tile_kernel<false><<<grid, kTileThreads, kTileSmem, st>>>(a, g, S);
+          // rows of tiles with voxels on this wavefront, and the longest of them
+          int ir0 = g.ntr, ir1 = -1, width = 0;
+          for (int ir = 0; ir < g.ntr; ++ir) {
+            int lo, hi;
+            geo_tile_row(g, a.Y, a.X, S, ir, &lo, &hi);
+            if (hi < lo) continue;
+            ir0 = imin(ir0, ir);
+            ir1 = ir;
+            width = imax(width, hi - lo + 1);
+          }
+          if (ir1 < 0) continue;  // no voxel of the domain
+          if (ir1 - ir0 >= 65535) return set_error(SI_ERR_LIMIT, "si_geo_scan: too many tiles");
+          // The first launch follows whatever wrote the image in full; the
+          // others may read the image before the wavefront before has ended.
+          cudaLaunchAttribute attr = {};
+          attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+          attr.val.programmaticStreamSerializationAllowed = 1;
+          cudaLaunchConfig_t cfg = {};
+          cfg.gridDim = dim3((unsigned)width, (unsigned)(ir1 - ir0 + 1), (unsigned)a.nol);
+          cfg.blockDim = dim3(kTileThreads);
+          cfg.dynamicSmemBytes = kTileSmem;
+          cfg.stream = st;
+          cfg.attrs = &attr;
+          cfg.numAttrs = first ? 0 : 1;
+          first = false;
+          if ((lamb1 ? cudaLaunchKernelEx(&cfg, geo_tile_kernel<true>, a, g, S, ir0)
+                     : cudaLaunchKernelEx(&cfg, geo_tile_kernel<false>, a, g, S, ir0)) != cudaSuccess)
+            return check_launch("si_geo_scan (tile launch)");
         }
       }
     return SI_OK;
