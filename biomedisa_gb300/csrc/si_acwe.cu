@@ -85,6 +85,40 @@ __device__ __forceinline__ EvoKey evo_key(const float* mean, int l, float f, con
   return l == 0 ? k0 : EvoKey{fabsf(__fsub_rn(mean[l], f)), 0};
 }
 
+// Stages the planes of a tile (with its halo of one voxel) for a CTA that
+// marches in z: a thread's cells stay the same from plane to plane, and a plane
+// is fetched into registers one step before it is stored, so that its latency
+// passes under the step before it.
+template <typename T>
+struct PlaneLoader {
+  static constexpr int kCells = (kPlaneB + kTX * kTY - 1) / (kTX * kTY);
+  const T* at[kCells];
+  bool in[kCells];
+  T v[kCells], outside;
+  int tid, Z;
+  size_t plane;
+  __device__ __forceinline__ PlaneLoader(const T* src, int tid_, int x0, int y0, int Z_, int Y, int X, T outside_)
+      : outside(outside_), tid(tid_), Z(Z_), plane((size_t)Y * X) {
+#pragma unroll
+    for (int k = 0; k < kCells; ++k) {
+      const int i = tid + k * kTX * kTY, r = i / kRowB, c = i - r * kRowB;
+      const int gy = y0 - 1 + r, gx = x0 - 1 + c;
+      in[k] = i < kPlaneB && (unsigned)gy < (unsigned)Y && (unsigned)gx < (unsigned)X;
+      at[k] = src + ((ptrdiff_t)gy * X + gx);
+      v[k] = outside;
+    }
+  }
+  __device__ __forceinline__ void fetch(int z) {
+#pragma unroll
+    for (int k = 0; k < kCells; ++k) v[k] = in[k] && (unsigned)z < (unsigned)Z ? at[k][(size_t)z * plane] : outside;
+  }
+  __device__ __forceinline__ void store(T* slot) const {
+#pragma unroll
+    for (int k = 0; k < kCells; ++k)
+      if (tid + k * kTX * kTY < kPlaneB) slot[tid + k * kTX * kTY] = v[k];
+  }
+};
+
 // One pass of a 27-point stencil over the crop (Z, Y, X); dst must not alias
 // src. kEvolution reads img and the label sums; kErosion / kDilation act on
 // `label`.
@@ -107,26 +141,40 @@ __global__ void __launch_bounds__(kTX* kTY) acwe_stencil_kernel(const uint8_t* _
       mean[k] = cnt ? __double2float_rn(__ddiv_rn((double)sums[256 + k], (double)cnt)) : 0.0f;
     }
   }
-  auto load_plane = [&](int z, int slot) {
-    for (int i = tid; i < kPlaneB; i += kTX * kTY) {
-      const int r = i / kRowB, c = i - r * kRowB;
-      const int gy = y0 - 1 + r, gx = x0 - 1 + c;
-      uint8_t v = 0;
-      if ((unsigned)z < (unsigned)Z && (unsigned)gy < (unsigned)Y && (unsigned)gx < (unsigned)X)
-        v = src[((size_t)z * Y + gy) * X + gx];
-      s[slot][i] = v;
-    }
-  };
-  load_plane(zs - 1, 0);
-  load_plane(zs, 1);
+  PlaneLoader<uint8_t> ld(src, tid, x0, y0, Z, Y, X, 0);
+  ld.fetch(zs - 1);
+  ld.store(s[0]);
+  ld.fetch(zs);
+  ld.store(s[1]);
+  ld.fetch(zs + 1);
   const int x = x0 + tx, y = y0 + ty;
   const bool in_xy = x < X && y < Y;
   const bool int_xy = x >= 1 && x <= X - 2 && y >= 1 && y <= Y - 2;
   const int cpos = (ty + 1) * kRowB + tx + 1;
   int sm = 0, sc = 1, sp = 2;
-  for (int z = zs; z < ze; ++z) {
-    load_plane(z + 1, sp);
+  // The label that all nine voxels of a plane around the column hold, or -1:
+  // evolution looks for voxels inside one label with 9 loads a plane, the
+  // planes z - 1 and z keeping their answer (27 loads: 201 us a pass on a
+  // 194x258x252 crop, 126 then, 102 with PlaneLoader's prefetch).
+  auto nine = [&](int slot) -> int {
+    const uint8_t* p = s[slot] + cpos;
+    const int t = p[0];
+    int diff = 0;
+#pragma unroll
+    for (int i = 0; i < 9; ++i) diff |= p[(i / 3 - 1) * kRowB + i % 3 - 1] ^ t;
+    return diff ? -1 : t;
+  };
+  int nm = -1, nc = -1;
+  if (kOp == kEvolution) {
     __syncthreads();
+    nm = nine(0);
+    nc = nine(1);
+  }
+  for (int z = zs; z < ze; ++z) {
+    ld.store(s[sp]);
+    ld.fetch(z + 2);
+    __syncthreads();
+    const int np = kOp == kEvolution ? nine(sp) : -1;
     if (in_xy) {
       const size_t v = ((size_t)z * Y + y) * X + x;
       const int c = s[sc][cpos];
@@ -134,11 +182,7 @@ __global__ void __launch_bounds__(kTX* kTY) acwe_stencil_kernel(const uint8_t* _
       if (int_xy && z >= 1 && z <= Z - 2) {
         const uint8_t* pl[3] = {s[sm], s[sc], s[sp]};
         if (kOp == kEvolution) {
-          uint32_t same = 0;
-#pragma unroll
-          for (int i = 0; i < 27; ++i)
-            same |= (uint32_t)(pl[i / 9][cpos + ((i / 3) % 3 - 1) * kRowB + (i % 3 - 1)] == c) << i;
-          if (same != kAll27) {  // a voxel inside one label keeps it
+          if (nm != c || nc != c || np != c) {  // a voxel inside one label keeps it
             const float f = (float)img[v];
             const EvoKey k0 = zero_key(mean, f, alpha);
             EvoKey ref = evo_key(mean, c, f, k0);
@@ -179,6 +223,8 @@ __global__ void __launch_bounds__(kTX* kTY) acwe_stencil_kernel(const uint8_t* _
       dst[v] = (uint8_t)out;
     }
     __syncthreads();
+    nm = nc;
+    nc = np;
     const int t = sm;
     sm = sc;
     sc = sp;
@@ -487,51 +533,55 @@ __global__ void __launch_bounds__(kTX* kTY) acwe_chamfer_pass_kernel(const float
   const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * kTX + tx;
   const int x0 = blockIdx.x * kTX, y0 = blockIdx.y * kTY, zs = blockIdx.z * kZChunk;
   const int ze = min(zs + kZChunk, Z);
-  auto load_plane = [&](int z, int slot) {
-    for (int i = tid; i < kPlaneF; i += kTX * kTY) {
-      const int r = i / kRowF, c = i - r * kRowF;
-      const int gy = y0 - 1 + r, gx = x0 - 1 + c;
-      float v = 11.0f;
-      if ((unsigned)z < (unsigned)Z && (unsigned)gy < (unsigned)Y && (unsigned)gx < (unsigned)X)
-        v = src[((size_t)z * Y + gy) * X + gx];
-      s[slot][i] = v;
-    }
-  };
-  load_plane(zs - 1, 0);
-  load_plane(zs, 1);
+  PlaneLoader<float> ld(src, tid, x0, y0, Z, Y, X, 11.0f);
+  ld.fetch(zs - 1);
+  ld.store(s[0]);
+  ld.fetch(zs);
+  ld.store(s[1]);
+  ld.fetch(zs + 1);
   const int x = x0 + tx, y = y0 + ty;
   const bool in_xy = x < X && y < Y;
   const bool int_xy = x >= 1 && x <= X - 2 && y >= 1 && y <= Y - 2;
   const int cpos = (ty + 1) * kRowF + tx + 1;
   const float w1 = 1.0f, w2 = 1.41421356f, w3 = 1.73205081f;
-  int sm = 0, sc = 1, sp = 2;
+  // A column's centre, the minimum of its four edge and of its four corner
+  // neighbours in a plane: 9 loads per voxel instead of 27, because the planes
+  // z - 1 and z keep theirs in registers, and one addition per weight, because
+  // the rounded sums of a minimum's operands are in its operands' order
+  // (194x258x252 crop: 91 -> 62 us a pass, 40 with PlaneLoader's prefetch).
+  struct Col {
+    float c, e, d;
+  };
+  auto column = [&](int slot) {
+    const float* p = s[slot] + cpos;
+    return Col{p[0], fminf(fminf(p[-1], p[1]), fminf(p[-kRowF], p[kRowF])),
+               fminf(fminf(p[-kRowF - 1], p[-kRowF + 1]), fminf(p[kRowF - 1], p[kRowF + 1]))};
+  };
+  __syncthreads();
+  const Col none{INFINITY, INFINITY, INFINITY};  // planes outside the crop do not relax
+  Col cm = zs > 0 ? column(0) : none, cc = column(1);
+  int sp = 2;  // the slot of plane z + 1; the next plane goes to slot (sp + 1) % 3
   for (int z = zs; z < ze; ++z) {
-    load_plane(z + 1, sp);
+    ld.store(s[sp]);
+    ld.fetch(z + 2);
     __syncthreads();
+    const Col cp = z + 1 < Z ? column(sp) : none;
     if (in_xy) {
-      float best = s[sc][cpos];
+      float best = cc.c;
       if (int_xy) {  // every plane of the crop relaxes (see above); rows/columns 0 and n-1 keep their values
-        const float* pl[3] = {s[sm], s[sc], s[sp]};
-#pragma unroll
-        for (int i = 0; i < 27; ++i) {
-          const int dz = i / 9 - 1, dy = (i / 3) % 3 - 1, dx = i % 3 - 1;
-          const int nzero = (dz != 0) + (dy != 0) + (dx != 0);
-          if (nzero == 0 || (z + dz) < 0 || (z + dz) >= Z) continue;
-          const float w = nzero == 1 ? w1 : (nzero == 2 ? w2 : w3);
-          best = fminf(best, __fadd_rn(pl[dz + 1][cpos + dy * kRowF + dx], w));
-        }
+        best = fminf(best, __fadd_rn(fminf(cc.e, fminf(cm.c, cp.c)), w1));
+        best = fminf(best, __fadd_rn(fminf(cc.d, fminf(cm.e, cp.e)), w2));
+        best = fminf(best, __fadd_rn(fminf(cm.d, cp.d), w3));
         best = fminf(best, 11.0f);
       }
       dst[((size_t)z * Y + y) * X + x] = best;
     }
-    __syncthreads();
-    const int t = sm;
-    sm = sc;
-    sc = sp;
-    sp = t;
+    // three slots: the plane loaded next was last read one barrier ago
+    cm = cc;
+    cc = cp;
+    sp = sp == 2 ? 0 : sp + 1;
   }
 }
-
 
 __global__ void __launch_bounds__(256) acwe_dist_init_kernel(const uint8_t* __restrict__ L, uint64_t n,
                                                              float* __restrict__ dist) {
