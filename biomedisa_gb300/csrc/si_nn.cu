@@ -10,6 +10,9 @@
 // Channel counts are multiples of 16 (padding channels carry zeros).
 #include <cuda_bf16.h>
 
+#include <algorithm>
+#include <atomic>
+
 #include "si_common.cuh"
 #include "si_internal.h"
 
@@ -299,7 +302,8 @@ __global__ void __launch_bounds__(128) conv3d_wgrad_kernel(const __nv_bfloat16* 
 }
 
 // ---------------------------------------------------------------------------
-// 16 x 16 weight gradient. A block of 4 warps walks a run of 64-voxel x-rows;
+// 16 x 16 weight gradient for dilations that wgrad16_rows_kernel's rows do not
+// hold. A block of 4 warps walks a run of 64-voxel x-rows;
 // per row the dY row is staged once in shared memory, and each warp handles
 // the taps w, w + 4, ... : it stages the shifted X row (zeros outside the
 // volume) and runs dW[tap] += dY^T X on the tensor cores, with both operands
@@ -410,6 +414,199 @@ __global__ void __launch_bounds__(128) wgrad16_kernel(const __nv_bfloat16* __res
   }
 }
 
+// ---------------------------------------------------------------------------
+// 16 x 16 weight and bias gradient, dilation up to kWgMaxDil. A CTA of nine
+// warps walks a run of 64-voxel x-rows of dY; warp j takes the input row at
+// (dz, dy) = (j / 3, j % 3) - 1 and its three taps along x, which read the same
+// staged row (64 voxels and the dilation on both sides) at shifted addresses. Rows
+// are staged two steps ahead by asynchronous copies in a ring of three slots, with
+// one CTA barrier per row. What bounds it: with a copy of every tap's row through
+// registers and no copy in flight across rows (wgrad16_kernel) the global loads'
+// latency did, 306 us on 8 x 64^3 voxels (94 TFLOP/s); this one takes 123 us (236
+// TFLOP/s), its shared-memory operand loads and mma.sync issue. The bias
+// gradient's sums are taken from the staged dY rows (37 us as a pass of its own).
+// ---------------------------------------------------------------------------
+constexpr int kWgMaxDil = 8, kWgWarps = 9, kWgStages = 3;
+constexpr int kWgRow = (64 + 2 * kWgMaxDil) * 32;          // bytes of a staged input row
+constexpr int kWgStage = 64 * 32 + kWgWarps * kWgRow;      // dY row, input rows
+constexpr int kWgSmem = kWgStages * kWgStage;
+constexpr int kWgOut = 27 * 256 + 16;                      // sums of a block: weights, bias
+
+// 16 bytes to shared memory; zeros where !ok (src is not read then).
+__device__ __forceinline__ void copy_async16(uint32_t dst, const void* src, bool ok) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(ok ? 16 : 0) : "memory");
+}
+
+__global__ void __launch_bounds__(kWgWarps * 32, 3)
+    wgrad16_rows_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ dy,
+                        float* __restrict__ dw, float* __restrict__ db, float* __restrict__ partials, Vol5 g, int dil,
+                        int xchunks, int64_t rows_per_block) {
+  extern __shared__ __align__(128) uint8_t smem[];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int64_t rows = (int64_t)g.N * g.D * g.H * xchunks;
+  const int64_t r0 = (int64_t)blockIdx.x * rows_per_block;
+  const int64_t r1 = r0 + rows_per_block < rows ? r0 + rows_per_block : rows;
+  const uint32_t base = (uint32_t)__cvta_generic_to_shared(smem);
+  const int dz = (warp / 3 - 1) * dil, dyo = (warp % 3 - 1) * dil;
+  const int chunks = (64 + 2 * dil) * 2;  // 16-byte pieces of an input row
+  // position of the next row to stage; whether this warp's input row exists
+  int xc, yy, zz, n;
+  {
+    int64_t t = r0;
+    xc = (int)(t % xchunks);
+    t /= xchunks;
+    yy = (int)(t % g.H);
+    t /= g.H;
+    zz = (int)(t % g.D);
+    n = (int)(t / g.D);
+  }
+  unsigned exists = 0u;  // bit s: slot s holds an input row
+  auto stage = [&](int64_t row, int slot) {
+    if (row < r1) {
+      const uint32_t at = base + slot * kWgStage;
+      const int xb = xc * 64;
+      const int64_t vox = (((int64_t)n * g.D + zz) * g.H + yy) * g.W;
+      if (warp < 4) {  // 128 threads x 16 bytes of dY
+        const int v = threadIdx.x >> 1, h = threadIdx.x & 1;
+        const bool ok = xb + v < g.W;
+        copy_async16(at + swz(v, h), dy + (vox + (ok ? xb + v : 0)) * 16 + h * 8, ok);
+      }
+      const int zi = zz + dz, yi = yy + dyo;
+      const bool zy = (unsigned)zi < (unsigned)g.D && (unsigned)yi < (unsigned)g.H;
+      exists = (exists & ~(1u << slot)) | ((unsigned)zy << slot);
+      if (zy) {
+        const __nv_bfloat16* xrow = x + (((int64_t)n * g.D + zi) * g.H + yi) * g.W * 16;
+        const uint32_t to = at + 64 * 32 + warp * kWgRow;
+#pragma unroll
+        for (int k = 0; k < (64 + 2 * kWgMaxDil) * 2 / 32; ++k) {
+          const int q = lane + 32 * k, v = q >> 1, h = q & 1;
+          const int xi = xb - dil + v;
+          const bool ok = (unsigned)xi < (unsigned)g.W;
+          if (q < chunks) copy_async16(to + swz(v, h), xrow + (int64_t)(ok ? xi : 0) * 16 + h * 8, ok);
+        }
+      }
+      if (++xc == xchunks) {
+        xc = 0;
+        if (++yy == g.H) {
+          yy = 0;
+          if (++zz == g.D) {
+            zz = 0;
+            ++n;
+          }
+        }
+      }
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  float acc[3][2][4];
+#pragma unroll
+  for (int i = 0; i < 3; ++i)
+#pragma unroll
+    for (int j = 0; j < 2; ++j) acc[i][j][0] = acc[i][j][1] = acc[i][j][2] = acc[i][j][3] = 0.0f;
+  float bias = 0.0f, lost = 0.0f;  // thread t < 256: channel t % 16, voxels 4 (t / 16) .. + 3 of every row
+  const int bc = threadIdx.x & 15, bv = (threadIdx.x >> 4) * 4;
+  // ldmatrix row addresses as in wgrad16_kernel
+  const int q = lane >> 3, i8 = lane & 7;
+  const int va = i8 + ((q >> 1) << 3), ha = q & 1;
+  const int vb = i8 + ((q & 1) << 3), hb = q >> 1;
+  stage(r0, 0);
+  stage(r0 + 1, 1);
+  int slot = 0;
+  for (int64_t row = r0; row < r1; ++row) {
+    asm volatile("cp.async.wait_group 1;" ::: "memory");
+    __syncthreads();  // the row has landed; the slot staged below was last read one row ago
+    stage(row + 2, slot == 0 ? 2 : slot - 1);
+    const uint32_t sdy = base + slot * kWgStage, sx = sdy + 64 * 32 + warp * kWgRow;
+    if ((exists >> slot) & 1u) {
+#pragma unroll
+      for (int ks = 0; ks < 4; ++ks) {
+        uint32_t a[4];
+        ldsm_x4_trans(a, sdy + swz(ks * 16 + va, ha));
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+          uint32_t b[4];
+          ldsm_x4_trans(b, sx + swz(ks * 16 + vb + i * dil, hb));
+          mma_bf16(acc[i][0], a, b[0], b[1]);
+          mma_bf16(acc[i][1], a, b[2], b[3]);
+        }
+      }
+    }
+    if (db && threadIdx.x < 256) {
+      float t[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+        t[k] = __bfloat162float(*reinterpret_cast<const __nv_bfloat16*>(smem + slot * kWgStage +
+                                                                       swz(bv + k, bc >> 3) + (bc & 7) * 2));
+      // compensated (Kahan): the sum of a block's rows is as good as one rounding
+      const float add = __fsub_rn((t[0] + t[1]) + (t[2] + t[3]), lost), sum = __fadd_rn(bias, add);
+      lost = __fsub_rn(__fsub_rn(sum, bias), add);
+      bias = sum;
+    }
+    slot = slot == 2 ? 0 : slot + 1;
+  }
+  asm volatile("cp.async.wait_all;" ::: "memory");
+  const int grp = lane >> 2, tig = lane & 3;
+  float* out = partials ? partials + (int64_t)blockIdx.x * kWgOut : dw;
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    const int tap = warp * 3 + i;
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      float* d = out + tap * 256 + grp * 16 + j * 8 + tig * 2;
+      if (partials) {  // deterministic: this block's sums, reduced in block order afterwards
+        *reinterpret_cast<float2*>(d) = make_float2(acc[i][j][0], acc[i][j][1]);
+        *reinterpret_cast<float2*>(d + 128) = make_float2(acc[i][j][2], acc[i][j][3]);
+      } else {
+        atomicAdd(d, acc[i][j][0]);
+        atomicAdd(d + 1, acc[i][j][1]);
+        atomicAdd(d + 128, acc[i][j][2]);
+        atomicAdd(d + 129, acc[i][j][3]);
+      }
+    }
+  }
+  if (db) {  // the 16 threads of a channel, pairwise
+    __syncthreads();
+    float* s = reinterpret_cast<float*>(smem);
+    if (threadIdx.x < 256) s[threadIdx.x] = bias;
+    __syncthreads();
+    if (threadIdx.x < 16) {
+      float u[16];
+      for (int k = 0; k < 16; ++k) u[k] = s[16 * k + threadIdx.x];
+      for (int o = 8; o; o >>= 1)
+        for (int k = 0; k < o; ++k) u[k] += u[k + o];
+      const float t = u[0];
+      if (partials)
+        out[27 * 256 + threadIdx.x] = t;
+      else
+        atomicAdd(&db[threadIdx.x], t);
+    }
+  }
+}
+
+// dw[i] += sum_b partials[b][i], db likewise, in the order of
+// reduce_partials_kernel: 32 sums over the blocks b = l, l + 32, ..., combined
+// pairwise. A CTA takes 32 outputs, so that its loads are coalesced.
+__global__ void __launch_bounds__(1024) reduce_wgrad_kernel(const float* __restrict__ partials, int nb,
+                                                            float* __restrict__ dw, float* __restrict__ db) {
+  __shared__ float s[32][32];
+  const int lane = threadIdx.x & 31, l = threadIdx.x >> 5, i = blockIdx.x * 32 + lane;
+  float t = 0.0f;
+  if (i < kWgOut)
+#pragma unroll 8
+    for (int b = l; b < nb; b += 32) t += partials[(int64_t)b * kWgOut + i];
+  s[l][lane] = t;
+  for (int o = 16; o; o >>= 1) {
+    __syncthreads();
+    if (l < o) s[l][lane] += s[l + o][lane];
+  }
+  if (l == 0 && i < kWgOut) {
+    if (i < 27 * 256)
+      dw[i] += s[0][lane];
+    else if (db)
+      db[i - 27 * 256] += s[0][lane];
+  }
+}
+
 // W'[tap][ci][co] = W[26 - tap][co][ci]
 __global__ void flip_weights_kernel(const __nv_bfloat16* __restrict__ w, __nv_bfloat16* __restrict__ wf, int cout,
                                     int cin) {
@@ -471,15 +668,33 @@ __global__ void __launch_bounds__(256) reduce_partials_kernel(const float* __res
   }
 }
 
-// g *= (y > 0); optionally also out = g_masked + add
+// g *= (y > 0); optionally also out = g_masked + add. Eight values a thread
+// where all pointers are aligned to 16 bytes (3 x 67 MB: 72 us one by one, 26 so).
+__device__ __forceinline__ __nv_bfloat16 relu_bwd_one(__nv_bfloat16 g, __nv_bfloat16 y, bool has, __nv_bfloat16 a) {
+  float v = __bfloat162float(y) > 0.0f ? __bfloat162float(g) : 0.0f;
+  if (has) v += __bfloat162float(a);
+  return __float2bfloat16(v);
+}
+
 __global__ void __launch_bounds__(256) relu_bwd_kernel(__nv_bfloat16* __restrict__ g,
                                                        const __nv_bfloat16* __restrict__ y,
-                                                       const __nv_bfloat16* __restrict__ add, int64_t n) {
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    float v = __bfloat162float(y[i]) > 0.0f ? __bfloat162float(g[i]) : 0.0f;
-    if (add) v += __bfloat162float(add[i]);
-    g[i] = __float2bfloat16(v);
+                                                       const __nv_bfloat16* __restrict__ add, int64_t n, int64_t n8) {
+  const int64_t stride = (int64_t)gridDim.x * blockDim.x, first = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  union Eight {
+    uint4 q;
+    __nv_bfloat16 v[8];
+  };
+  for (int64_t i = first; i < n8; i += stride) {
+    Eight a, b, c;
+    a.q = reinterpret_cast<const uint4*>(g)[i];
+    b.q = reinterpret_cast<const uint4*>(y)[i];
+    c.q = add ? reinterpret_cast<const uint4*>(add)[i] : make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+    for (int k = 0; k < 8; ++k) a.v[k] = relu_bwd_one(a.v[k], b.v[k], add != nullptr, c.v[k]);
+    reinterpret_cast<uint4*>(g)[i] = a.q;
   }
+  for (int64_t i = 8 * n8 + first; i < n; i += stride)
+    g[i] = relu_bwd_one(g[i], y[i], add != nullptr, add ? add[i] : __float2bfloat16(0.0f));
 }
 
 // Soft-target cross entropy over the first nol of C logit channels.
@@ -510,6 +725,69 @@ __global__ void __launch_bounds__(256) xent_kernel(const float* __restrict__ log
   }
   for (int o = 16; o; o >>= 1) local += __shfl_xor_sync(0xffffffffu, local, o);
   if ((threadIdx.x & 31) == 0) atomicAdd(loss, local);
+}
+
+// The same for 16 channels at 16-byte alignment: a voxel's logits stay in
+// registers between the passes over them (one by one they were read four times:
+// 238 us at the 8 x 64^3 training batch; 59 us so), and the loss is summed with
+// compensation per thread and pairwise per CTA before its one atomic addition.
+__global__ void __launch_bounds__(256) xent16_kernel(const float* __restrict__ logits,
+                                                     const float* __restrict__ target,
+                                                     const float* __restrict__ weight, int64_t V, int nol, float scale,
+                                                     __nv_bfloat16* __restrict__ dlogits, float* __restrict__ loss) {
+  __shared__ double s_sum[8];
+  float sum = 0.0f, lost = 0.0f;
+  for (int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; v < V; v += (int64_t)gridDim.x * blockDim.x) {
+    float z[16], p[16];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const float4 q = reinterpret_cast<const float4*>(logits + v * 16)[k];
+      z[4 * k] = q.x; z[4 * k + 1] = q.y; z[4 * k + 2] = q.z; z[4 * k + 3] = q.w;
+    }
+#pragma unroll
+    for (int l = 0; l < 16; ++l) p[l] = l < nol ? target[v * nol + l] : 0.0f;
+    const float wv = weight ? weight[v] : 1.0f;
+    float m = -INFINITY;
+#pragma unroll
+    for (int l = 0; l < 16; ++l)
+      if (l < nol) m = fmaxf(m, z[l]);
+    float s = 0.0f;
+#pragma unroll
+    for (int l = 0; l < 16; ++l)
+      if (l < nol) s += __expf(z[l] - m);
+    const float lse = m + __logf(s);
+    float local = 0.0f;
+    uint32_t d[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      float g[2];
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int l = 2 * k + h;
+        g[h] = 0.0f;
+        if (l < nol) {
+          const float q = __expf(z[l] - lse);
+          local += -wv * p[l] * (z[l] - lse);
+          g[h] = wv * (q - p[l]) * scale;
+        }
+      }
+      d[k] = pack2(__float2bfloat16(g[0]), __float2bfloat16(g[1]));
+    }
+    uint4* o = reinterpret_cast<uint4*>(dlogits + v * 16);
+    o[0] = make_uint4(d[0], d[1], d[2], d[3]);
+    o[1] = make_uint4(d[4], d[5], d[6], d[7]);
+    const float add = __fsub_rn(local, lost), t = __fadd_rn(sum, add);
+    lost = __fsub_rn(__fsub_rn(t, sum), add);
+    sum = t;
+  }
+  double w = sum;
+  for (int o = 16; o; o >>= 1) w += __shfl_xor_sync(0xffffffffu, w, o);
+  if ((threadIdx.x & 31) == 0) s_sum[threadIdx.x >> 5] = w;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int k = 1; k < 8; ++k) w += s_sum[k];
+    atomicAdd(loss, (float)w);
+  }
 }
 
 // AdamW on fp32 master weights; writes the bf16 working copy.
@@ -713,9 +991,25 @@ extern "C" int si_nn_conv3d_wgrad(const void* x, const void* dy, float* dw, floa
   if (fast) {
     const int xchunks = (W + 63) / 64;
     const int64_t rows = (int64_t)N * D * H * xchunks;
+    const bool short_rows = dil <= kWgMaxDil;
     const int64_t want = (int64_t)sm_count() * 8;
     const int64_t per = (rows + want - 1) / want;
     const int64_t blocks = (rows + per - 1) / per;
+    if (short_rows) {
+      static std::atomic<bool> set[64];
+      int dev = 0;
+      if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) dev = 0;
+      if (!set[dev].load(std::memory_order_acquire)) {
+        if (cudaFuncSetAttribute(wgrad16_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kWgSmem) !=
+            cudaSuccess)
+          return check_launch("si_nn_conv3d_wgrad (shared memory)");
+        set[dev].store(true, std::memory_order_release);
+      }
+      wgrad16_rows_kernel<<<(unsigned)blocks, kWgWarps * 32, kWgSmem, st>>>(xb, db16, dw, db, partials, g, dil, xchunks,
+                                                                           per);
+      if (partials) reduce_wgrad_kernel<<<(kWgOut + 31) / 32, 1024, 0, st>>>(partials, (int)blocks, dw, db);
+      return check_launch("si_nn_conv3d_wgrad");
+    }
     wgrad16_kernel<<<(unsigned)blocks, 128, 0, st>>>(xb, db16, dw, partials, g, dil, xchunks, per);
     if (partials)
       reduce_partials_kernel<<<27 * 256 / 8, 256, 0, st>>>(partials, (int)blocks, 27 * 256, dw);
@@ -745,9 +1039,10 @@ extern "C" int si_nn_flip_weights(const void* w, void* w_flipped, int cout, int 
 extern "C" int si_nn_relu_bwd(void* g, const void* y, const void* add, int64_t n, void* stream) {
   clear_error();
   if (!g || !y || n < 0) return set_error(SI_ERR_ARG, "si_nn_relu_bwd: bad arguments");
-  relu_bwd_kernel<<<egrid(n), 256, 0, as_stream(stream)>>>(static_cast<__nv_bfloat16*>(g),
-                                                            static_cast<const __nv_bfloat16*>(y),
-                                                            static_cast<const __nv_bfloat16*>(add), n);
+  const int64_t n8 = ((uintptr_t)g | (uintptr_t)y | (uintptr_t)add) % 16 == 0 ? n / 8 : 0;
+  relu_bwd_kernel<<<egrid(n8 ? n8 : n), 256, 0, as_stream(stream)>>>(static_cast<__nv_bfloat16*>(g),
+                                                                      static_cast<const __nv_bfloat16*>(y),
+                                                                      static_cast<const __nv_bfloat16*>(add), n, n8);
   return check_launch("si_nn_relu_bwd");
 }
 
@@ -756,6 +1051,12 @@ extern "C" int si_nn_xent(const float* logits, const float* target, const float*
   clear_error();
   if (!logits || !target || !dlogits || !loss || nol < 1 || nol > C)
     return set_error(SI_ERR_ARG, "si_nn_xent: bad arguments");
+  if (C == 16 && ((uintptr_t)logits | (uintptr_t)dlogits) % 16 == 0) {
+    const int64_t want = (V + 255) / 256, most = (int64_t)sm_count() * 4;
+    xent16_kernel<<<(int)std::max<int64_t>(1, std::min(want, most)), 256, 0, as_stream(stream)>>>(
+        logits, target, weight, V, nol, scale, static_cast<__nv_bfloat16*>(dlogits), loss);
+    return check_launch("si_nn_xent");
+  }
   xent_kernel<<<egrid(V), 256, 0, as_stream(stream)>>>(logits, target, weight, V, C, nol, scale,
                                                         static_cast<__nv_bfloat16*>(dlogits), loss);
   return check_launch("si_nn_xent");
