@@ -15,39 +15,55 @@
 // by the tensor core 9 times instead of 27.
 //
 // Accumulator ring. The CTA's input rows form one sequence k = 0, 1, ...
-// over all its columns (column c starts at k = P_c, P_{c+1} = P_c + nt + 2);
+// over all its columns (column c starts at k = P_c, P_{c+1} = P_c + rows + 2);
 // input k adds into ring positions k, k + 1, k + 2 and completes position k
 // (output j = k - P_c - 2 of its column; positions P_c and P_c + 1 are
-// padding). Positions live in the 32 slots of 16 columns (k mod 32) of the
-// 512 tensor-memory columns; a region starting at slot 30 or 31 is issued as
-// two MMAs (N = 32 + 16 or 16 + 32) that continue at slot 0, so every
+// padding). Positions live in the 16 slots of 16 columns (k mod 16) of the
+// CTA's 256 tensor-memory columns; a region starting at slot 14 or 15 is issued
+// as two MMAs (N = 32 + 16 or 16 + 32) that continue at slot 0, so every
 // position sums its 27 products in one slot, in the same order wherever it
 // falls in the ring (results do not depend on the grid). Every MMA
 // accumulates; the epilogue zeroes a position's slot (tcgen05.st) after
 // reading it and before releasing it, and all slots start zeroed.
 //
-// Shared-memory operands, K-major without swizzle (core matrices of 8 rows x
-// 16 bytes): an input z-row is one TMA box of {8 channels, 128 + 2*dil
-// voxels, 2 channel halves} over a 5-D tensor map {8, W, 2, H, D*N} whose
-// half dimension has a 16-byte stride, which lands as [half][voxel][8
-// channels]; the A operand of shift dx is that block at a start address
-// 16*dil*(dx + 1) bytes further. Voxels outside the row arrive as zeros
-// (TMA fill); input rows outside the volume in y or z are neither loaded
+// Shared-memory operands. An input z-row is one TMA box of {16 channels,
+// voxels, 1, lines, 1} over the 5-D tensor map {16, W, H, D, N}: rows of 32
+// bytes with the 32-byte swizzle (K-major); the A operand of shift dx is that
+// block at a start address 32*dil*dx bytes further (the swizzle is a function of
+// the address, so any row may start an operand). Rows of 16-byte channel halves,
+// which need no swizzle, read every 32-byte sector of L2 twice.
+//   W > 64: a tile is 128 voxels of one line, its box has dil more on both
+//   sides, and voxels outside the row arrive as zeros (TMA fill).
+//   W <= 64: a tile is 128 / W whole lines of consecutive z (two lines of 64 voxels
+//   make one MMA instead of two half empty ones). The box has no halo; the shifted
+//   operand's rows that belong to the next line are kept out of the sums by the
+//   MMA's lane mask.
+// Input rows outside the volume in y or, with all lines, in z are neither loaded
 // nor multiplied (their contribution is zero). The weights sit once per CTA
-// as 9 blocks [dz][dx] of [half][48][8 ci].
+// as 9 blocks [dz][dx] of [half][48][8 ci], without swizzle.
 //
-// Roles (one persistent CTA per SM, 11 warps): warp 0 loads each input row's
-// z-rows into a ring of 10 row slots; warp 10 loads, for a residual layer,
-// each output row's residual tile into a ring of 12 slots (so the epilogue
-// never waits on a global load); warp 1 issues the 9 MMAs and two commits
-// per input row (row slot free; ring position complete); two groups of four
-// warps (2-5, 6-9) run the epilogue of alternate positions (thread m =
-// tensor-memory lane m = voxel x0 + m): bias, residual, ReLU, bf16 or fp32
-// store, zeroing, release. Warps 0, 1 and 10 run their loops as whole warps
-// with warp-uniform operands and issue from one elected lane (from a single
-// lane every MMA cost about 80 cycles of issue, measured). Optionally the
-// CTA's columns are dealt to 2 or 4 interleaved streams with rings of their
-// own (si_nn_conv16_tc_set_streams; measured slower than one). Every wait is
+// Split. Two CTAs per SM: the issuing warp's own instructions are a column's
+// critical path (one row costs it about 1300 cycles, 9 MMAs, however many voxels
+// it has), so a second CTA with its own issuer nearly doubles the rate. A CTA
+// walks whole columns b, b + G, ... while every CTA has one; the rows of the
+// columns that are left are split evenly. What bounds it then: the shared-memory
+// pipe, 60 % operand reads (43 wavefronts per MMA: 4 KB of A, 1.5 KB of B) and 20 %
+// copies at 200 x 192 x 216. Measured, one convolution without / with residual,
+// before (one CTA per SM, channel halves, a line per tile) and now: 8 x 64^3
+// 186 / 192 -> 45 / 50 us, 200 x 192 x 216 400 / 416 -> 171 / 199 us, 128 x 256 x
+// 1024 1223 / 1275 -> 572 / 679 us. A second epilogue group (the issue slots it
+// takes) costs 5 %, the columns split only in equal segments 5 to 10 %.
+//
+// Roles (a persistent CTA of 7 warps): warp 0 loads each input row's
+// z-rows into a ring of 5 row slots; warp 6 loads, for a residual layer,
+// each output row's residual tile into a ring of 7 slots (so the epilogue
+// never waits on a global load); warp 1 issues the 9 MMAs and one commit
+// per input row (row slot free and ring position complete); warps 2-5 run the
+// epilogue (thread m = tensor-memory lane m = voxel m of the tile): release of
+// the position, bias, residual, ReLU, bf16 or fp32 store. Warps 0, 1 and 6 run
+// their loops as whole warps with warp-uniform operands and issue from one elected
+// lane. A launch may begin while the stream's kernel before it drains (programmatic
+// dependent launch; it reads nothing until that one has ended). Every wait is
 // bounded: a role that gives up flags the CTA, the others stop at their next
 // wait, the copies and MMAs in flight are waited for (bounded), the tensor
 // memory is freed and the status records the error.
@@ -55,8 +71,8 @@
 #include <cuda_bf16.h>
 
 #include <algorithm>
-#include <atomic>
 #include <cstring>
+#include <type_traits>
 
 #include "si_common.cuh"
 #include "si_internal.h"
@@ -67,29 +83,34 @@ namespace {
 
 constexpr int kTileM = 128;
 constexpr int kMaxDil = 8;
-constexpr int kRowBytes = (kTileM + 2 * kMaxDil) * 32;  // one staged z-row, both halves: 4608 bytes
+constexpr int kRowBytes = (kTileM + 2 * kMaxDil) * 32;  // one staged z-row: 4608 bytes
 constexpr int kSlotBytes = 3 * kRowBytes;               // an input row: its three z-rows
-constexpr int kRowSlots = 10;                           // ring of staged input rows
-constexpr int kResBytes = kTileM * 32;                  // one residual row tile [half][128][8]: 4096 bytes
-constexpr int kResSlots = 12;                           // ring of staged residual rows
+constexpr int kRowSlots = 5;                            // ring of staged input rows
+constexpr int kResBytes = kTileM * 32;                  // one residual row tile [128][16]: 4096 bytes
+constexpr int kResSlots = 7;                            // ring of staged residual rows
 constexpr int kWBlockBytes = 2 * 48 * 16;               // one (dz, dx) weight block [half][48][8]
 constexpr int kWBytes = 9 * kWBlockBytes;
-constexpr int kSmemBytes = kWBytes + kRowSlots * kSlotBytes + kResSlots * kResBytes + 128;  // + alignment slack
-constexpr int kTmemCols = 512;                          // 32 physical slots
-constexpr int kEpiGroups = 2;                           // epilogue groups of 4 warps, alternate items
-constexpr int kResWarp = 2 + 4 * kEpiGroups;           // the warp loading residual rows
+constexpr int kSmemBytes = kWBytes + kRowSlots * kSlotBytes + kResSlots * kResBytes + 1024;  // + alignment slack
+constexpr int kCtasPerSm = 2;
+constexpr int kTmemCols = 512 / kCtasPerSm;
+constexpr int kR = kTmemCols / 16;                      // accumulator ring positions
+constexpr int kResWarp = 6;                             // the warp loading residual rows
 constexpr int kThreads = 32 * (kResWarp + 1);
+static_assert(kWBytes % 256 == 0 && kRowBytes % 256 == 0 && kResBytes % 256 == 0, "swizzle atoms of 256 bytes");
+static_assert(kR >= kRowSlots + 3, "a row slot's done barrier is passed before its next phase");
 
 __device__ uint32_t g_umma_status;  // bit 0: a wait gave up (read by si_nn_umma_status)
-std::atomic<int> g_umma_streams{1};  // interleaved column streams per CTA (si_nn_conv16_tc_set_streams)
 
-// Shared-memory matrix descriptor, no swizzle, K-major core matrices.
+// Shared-memory matrix descriptor, K-major core matrices; kLayout 0: no swizzle,
+// 6: rows of 32 bytes, 32-byte swizzle.
+template <int kLayout>
 __device__ __forceinline__ uint64_t smem_desc(uint32_t saddr, uint32_t lbo, uint32_t sbo) {
   uint64_t d = (uint64_t)((saddr >> 4) & 0x3FFFu);
   d |= (uint64_t)((lbo >> 4) & 0x3FFFu) << 16;
   d |= (uint64_t)((sbo >> 4) & 0x3FFFu) << 32;
   d |= (uint64_t)1 << 46;  // fixed descriptor version bits 46..48 = 0b001
-  return d;                // base offset 0, absolute offsets, no swizzle
+  d |= (uint64_t)kLayout << 61;
+  return d;                // base offset 0, absolute offsets
 }
 
 // kind::f16 instruction descriptor: fp32 D, bf16 A and B, both K-major, M = 128, N = kN.
@@ -98,14 +119,34 @@ __host__ __device__ constexpr uint32_t idesc_f16() {
   return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(kN >> 3) << 17) | ((uint32_t)(kTileM >> 4) << 24);
 }
 
-// Executed by a whole warp with warp-uniform operands (which then stay in
-// uniform registers); one elected lane issues the MMA / the commit.
+// The three x-taps of one (input z-row, accumulator region): descriptors a + dx *
+// da and b + dx * 96. Executed by a whole warp with warp-uniform operands (which
+// then stay in uniform registers); one elected lane issues the MMAs.
 template <int kN>
-__device__ __forceinline__ void umma_f16(uint32_t d_tmem, uint64_t a, uint64_t b) {
+__device__ __forceinline__ void umma3(uint32_t d_tmem, uint64_t a, uint64_t da, uint64_t b) {
   asm volatile(
-      "{\n\t.reg .pred p, e;\n\tsetp.ne.b32 p, 1, 0;\n\telect.sync _|e, 0xffffffff;\n\t"
-      "@e tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
-      "l"(a), "l"(b), "r"(idesc_f16<kN>())
+      "{\n\t.reg .pred p, e;\n\t.reg .b64 a1, a2, b1, b2;\n\tsetp.ne.b32 p, 1, 0;\n\t"
+      "add.s64 a1, %1, %2;\n\tadd.s64 a2, a1, %2;\n\tadd.s64 b1, %3, 96;\n\tadd.s64 b2, b1, 96;\n\t"
+      "elect.sync _|e, 0xffffffff;\n\t"
+      "@e tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %3, %4, p;\n\t"
+      "@e tcgen05.mma.cta_group::1.kind::f16 [%0], a1, b1, %4, p;\n\t"
+      "@e tcgen05.mma.cta_group::1.kind::f16 [%0], a2, b2, %4, p;\n\t}" ::"r"(d_tmem),
+      "l"(a), "l"(da), "l"(b), "r"(idesc_f16<kN>())
+      : "memory");
+}
+// The same; the first MMA leaves the lanes of l alone, the last those of r.
+template <int kN>
+__device__ __forceinline__ void umma3(uint32_t d_tmem, uint64_t a, uint64_t da, uint64_t b, const uint32_t (&l)[4],
+                                      const uint32_t (&r)[4]) {
+  asm volatile(
+      "{\n\t.reg .pred p, e;\n\t.reg .b64 a1, a2, b1, b2;\n\tsetp.ne.b32 p, 1, 0;\n\t"
+      "add.s64 a1, %1, %2;\n\tadd.s64 a2, a1, %2;\n\tadd.s64 b1, %3, 96;\n\tadd.s64 b2, b1, 96;\n\t"
+      "elect.sync _|e, 0xffffffff;\n\t"
+      "@e tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %3, %4, {%5, %6, %7, %8}, p;\n\t"
+      "@e tcgen05.mma.cta_group::1.kind::f16 [%0], a1, b1, %4, p;\n\t"
+      "@e tcgen05.mma.cta_group::1.kind::f16 [%0], a2, b2, %4, {%9, %10, %11, %12}, p;\n\t}" ::"r"(d_tmem),
+      "l"(a), "l"(da), "l"(b), "r"(idesc_f16<kN>()), "r"(l[0]), "r"(l[1]), "r"(l[2]), "r"(l[3]), "r"(r[0]), "r"(r[1]),
+      "r"(r[2]), "r"(r[3])
       : "memory");
 }
 __device__ __forceinline__ void umma_commit(uint64_t* bar) {
@@ -122,13 +163,13 @@ __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
 
 // The copy, the expect_tx and the plain arrival below are executed by a
 // whole warp with warp-uniform operands; one elected lane issues them.
-__device__ __forceinline__ void tma_load_5d(void* dst, const CUtensorMap* map, int c, int x, int h, int y, int zn,
+__device__ __forceinline__ void tma_load_5d(void* dst, const CUtensorMap* map, int x, int y, int z, int n,
                                             uint64_t* bar) {
   asm volatile(
       "{\n\t.reg .pred e;\n\telect.sync _|e, 0xffffffff;\n\t"
       "@e cp.async.bulk.tensor.5d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, "
       "%5, %6}], [%7];\n\t}" ::"r"(smem_u32(dst)),
-      "l"(map), "r"(c), "r"(x), "r"(h), "r"(y), "r"(zn), "r"(smem_u32(bar))
+      "l"(map), "r"(0), "r"(x), "r"(y), "r"(z), "r"(n), "r"(smem_u32(bar))
       : "memory");
 }
 __device__ __forceinline__ void expect_tx_elect(uint64_t* bar, uint32_t bytes) {
@@ -137,6 +178,17 @@ __device__ __forceinline__ void expect_tx_elect(uint64_t* bar, uint32_t bytes) {
       "@e mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n\t}" ::"r"(smem_u32(bar)),
       "r"(bytes)
       : "memory");
+}
+// 32 bytes to a 32-byte aligned address in one store, else two of 16.
+__device__ __forceinline__ void store32(void* p, const uint32_t (&v)[8], int wide) {
+  if (wide)
+    asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "r"(v[0]), "r"(v[1]), "r"(v[2]),
+                 "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7])
+                 : "memory");
+  else {
+    static_cast<uint4*>(p)[0] = make_uint4(v[0], v[1], v[2], v[3]);
+    static_cast<uint4*>(p)[1] = make_uint4(v[4], v[5], v[6], v[7]);
+  }
 }
 __device__ __forceinline__ void arrive_elect(uint64_t* bar) {
   asm volatile(
@@ -160,36 +212,124 @@ __device__ __forceinline__ void tmem_zero16(uint32_t taddr) {
       : "memory");
 }
 
+// A column: digits (y phase, x chunk, z group, n), the first fastest.
+constexpr int kDigits = 4;
 struct UmmaGeom {
-  int N, D, H, W, dil, xchunks;
-  long long columns;  // (n, z, x chunk, y phase) tuples; each is walked along y in steps of dil
+  int N, D, H, W, dil;
+  int lines;              // z-lines of a tile (1: tiles of 128 voxels with a halo along x)
+  int nt;                 // output rows of a column (phase 0; others may have one less)
+  int rounds;             // whole columns a CTA walks: b, b + G, ...
+  int radix[kDigits];     // extents of the digits
+  int step[kDigits];      // the digits of the grid size G
+  long long tail_col;     // first of the columns after the rounds, whose rows
+  long long tail_rows;    // (this many) are split evenly over the CTAs
 };
 
-// Column c -> (n, z, x0, y phase, tiles); its output rows are y = phase + j*dil, j < nt.
-struct Column {
-  int n, z, x0, yph, nt;
+// Where a CTA starts its rounds and its share of the tail (decoded once).
+struct Starts {
+  int dg[kDigits], tail_dg[kDigits], tail_j, tail;
+  __device__ static void decode(const UmmaGeom& g, unsigned long long c, int (&d)[kDigits]) {
+    for (int k = 0; k < kDigits; ++k) {
+      d[k] = (int)(c % (unsigned)g.radix[k]);
+      c /= (unsigned)g.radix[k];
+    }
+  }
+  __device__ void set(const UmmaGeom& g) {
+    const long long r0 = g.tail_rows * blockIdx.x / gridDim.x;
+    tail = (int)(g.tail_rows * (blockIdx.x + 1) / gridDim.x - r0);
+    tail_j = (int)(r0 % g.nt);
+    decode(g, blockIdx.x, dg);
+    decode(g, (unsigned long long)(g.tail_col + r0 / g.nt), tail_dg);
+  }
 };
-__device__ __forceinline__ Column column_of(const UmmaGeom& g, long long c) {
-  Column o;
-  o.yph = (int)(c % g.dil);
-  c /= g.dil;
-  o.x0 = (int)(c % g.xchunks) * kTileM;
-  c /= g.xchunks;
-  o.z = (int)(c % g.D);
-  o.n = (int)(c / g.D);
-  o.nt = (g.H - o.yph + g.dil - 1) / g.dil;
-  return o;
-}
 
-// A stream: one of the CTA's interleaved column sequences and its position
-// in it (column, input row i of the column, the stream's ring position p =
-// k mod R of its input k with the phase (k / R) & 1).
-struct Stream {
-  long long col;
-  Column c;
-  int i;
-  int p;
+// A CTA's position: a column (its digits) and the input row i in it, i < cnt + 2,
+// at y = y0 + i * dil; p = the ring position of its count, k mod kR, with the
+// phase (k / kR) & 1.
+struct Walk {
+  int dg[kDigits];
+  int rounds;      // columns left of the rounds, this one included
+  int tail;        // rows left of the CTA's share of the tail, this column's not included
+  bool live;
+  int n, z, x0, y0, cnt;
+  int i, p;
   uint32_t ph;
+  __device__ __forceinline__ void enter(const UmmaGeom& g, int j0, int rows) {
+    n = dg[3];
+    z = dg[2] * g.lines;
+    x0 = dg[1] * kTileM;
+    const int nt = (g.H - dg[0] + g.dil - 1) / g.dil;  // nt < 1: H below the dilation
+    y0 = dg[0] + (j0 - 1) * g.dil;
+    cnt = max(0, min(j0 + rows, nt) - j0);
+    i = 0;
+  }
+  __device__ __forceinline__ void enter_tail(const UmmaGeom& g, int j0) {
+    const int rows = min(g.nt - j0, tail);
+    tail -= rows;
+    enter(g, j0, rows);
+  }
+  __device__ __forceinline__ void start_tail(const UmmaGeom& g, const Starts& s) {
+    tail = s.tail;
+    live = tail > 0;
+#pragma unroll
+    for (int k = 0; k < kDigits; ++k) dg[k] = s.tail_dg[k];
+    enter_tail(g, s.tail_j);
+  }
+  __device__ __forceinline__ void start(const UmmaGeom& g, const Starts& s) {
+    p = 0;
+    ph = 0;
+    rounds = g.rounds;
+    live = true;
+    tail = 0;
+#pragma unroll
+    for (int k = 0; k < kDigits; ++k) dg[k] = s.dg[k];
+    if (rounds > 0)
+      enter(g, 0, g.nt);
+    else
+      start_tail(g, s);
+  }
+  // true when it entered another column
+  __device__ __forceinline__ bool next(const UmmaGeom& g, const Starts& s) {
+    if (++p == kR) {
+      p = 0;
+      ph ^= 1u;
+    }
+    if (++i < cnt + 2) return false;
+    if (rounds == 1) {
+      rounds = 0;
+      start_tail(g, s);
+      return true;
+    }
+    if (rounds == 0 && tail == 0) {
+      live = false;
+      return true;
+    }
+    int carry = rounds ? 0 : 1;
+#pragma unroll
+    for (int k = 0; k < kDigits; ++k) {
+      dg[k] += (rounds ? g.step[k] : 0) + carry;
+      carry = dg[k] >= g.radix[k] ? 1 : 0;
+      dg[k] -= carry ? g.radix[k] : 0;
+    }
+    if (rounds) {
+      --rounds;
+      enter(g, 0, g.nt);
+    } else {
+      enter_tail(g, 0);
+    }
+    return true;
+  }
+  // input z-rows with a line inside the volume, bit dz
+  __device__ __forceinline__ uint32_t z_mask(const UmmaGeom& g) const {
+    uint32_t m = 0;
+#pragma unroll
+    for (int dz = 0; dz < 3; ++dz) {
+      const int zz = z + (dz - 1) * g.dil;
+      m |= (zz + g.lines > 0 && zz < g.D) ? (1u << dz) : 0u;
+    }
+    return m;
+  }
+  __device__ __forceinline__ int y(const UmmaGeom& g) const { return y0 + i * g.dil; }
 };
 
 // Index and phase of a ring of kN barriers (mbarrier parity of the use).
@@ -207,34 +347,33 @@ struct Ring {
   }
 };
 
-template <bool kOutF32, int kNS>
-__global__ void __launch_bounds__(kThreads, 1) conv16_umma_kernel(const __grid_constant__ CUtensorMap xmap,
-                                                                 const __grid_constant__ CUtensorMap rmap,
-                                                                 const __nv_bfloat16* __restrict__ w,
-                                                                 const float* __restrict__ bias, int has_res,
-                                                                 void* __restrict__ y_out, UmmaGeom g, int relu,
-                                                                 uint32_t wait_lim) {
-  constexpr int kR = 32 / kNS;  // ring positions (16-column slots) of a stream
-  static_assert(kR >= 8, "accumulator ring too short");
+template <bool kOutF32, bool kPacked>
+__global__ void __launch_bounds__(kThreads, kCtasPerSm)
+    conv16_umma_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUtensorMap rmap,
+                       const __nv_bfloat16* __restrict__ w, const float* __restrict__ bias, int has_res,
+                       void* __restrict__ y_out, const __grid_constant__ UmmaGeom g, int relu, int wide,
+                       uint32_t wait_lim) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 127) & ~(uintptr_t)127);
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   uint8_t* sw = smem;                             // weight blocks [dz][dx][half][48][8]
-  uint8_t* rows = smem + kWBytes;                 // [row slot][dz][half][voxel][8]
-  uint8_t* rres = rows + kRowSlots * kSlotBytes;  // [residual slot][half][128][8]
+  uint8_t* rows = smem + kWBytes;                 // [row slot][dz][voxel][16], 32-byte swizzle
+  uint8_t* rres = rows + kRowSlots * kSlotBytes;  // [residual slot][128][16], 32-byte swizzle
   __shared__ __align__(8) uint64_t full_bar[kRowSlots];   // an item's input z-rows landed
-  __shared__ __align__(8) uint64_t empty_bar[kRowSlots];  // its MMAs completed (row slot free)
-  __shared__ __align__(8) uint64_t done_bar[kNS * kR];    // ring position of a stream complete
-  __shared__ __align__(8) uint64_t free_bar[kNS * kR];    // ... read, zeroed, released
+  __shared__ __align__(8) uint64_t done_bar[kR];          // its MMAs completed: position complete, row slot free
+  __shared__ __align__(8) uint64_t free_bar[kR];          // position read, zeroed, released
   __shared__ __align__(8) uint64_t rfull_bar[kResSlots];  // an item's residual row landed
   __shared__ __align__(8) uint64_t rfree_bar[kResSlots];  // ... and was read
   __shared__ uint32_t tmem_base;
   __shared__ float s_bias[16];
+  __shared__ Starts s_start;
   __shared__ volatile int s_fail;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int dil = g.dil;
-  const int rv = kTileM + 2 * dil;  // staged voxels per z-row
-  const uint32_t box_bytes = 32u * (uint32_t)rv;
 
+  // the next convolution's CTAs may take the place of this one's that have ended
+  // (2.4 us a launch); they too wait here for the whole grid before them
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
   for (int i = tid; i < 9 * 48 * 2; i += kThreads) {
     const int blk = i / 96, nrow = (i / 2) % 48, h = i % 2;
     const int q = nrow / 16, co = nrow % 16;
@@ -245,11 +384,8 @@ __global__ void __launch_bounds__(kThreads, 1) conv16_umma_kernel(const __grid_c
   if (tid < 16) s_bias[tid] = bias ? bias[tid] : 0.0f;
   if (tid == 0) {
     s_fail = 0;
-    for (int b = 0; b < kRowSlots; ++b) {
-      mbar_init(&full_bar[b], 1);
-      mbar_init(&empty_bar[b], 1);
-    }
-    for (int b = 0; b < kNS * kR; ++b) {
+    for (int b = 0; b < kRowSlots; ++b) mbar_init(&full_bar[b], 1);
+    for (int b = 0; b < kR; ++b) {
       mbar_init(&done_bar[b], 1);
       mbar_init(&free_bar[b], 4);  // one arrival per epilogue warp
     }
@@ -259,6 +395,7 @@ __global__ void __launch_bounds__(kThreads, 1) conv16_umma_kernel(const __grid_c
     }
     fence_barrier_init();
   }
+  if (tid == 32 * kResWarp) s_start.set(g);
   if (warp == 1) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base)),
                  "r"(kTmemCols)
@@ -271,42 +408,20 @@ __global__ void __launch_bounds__(kThreads, 1) conv16_umma_kernel(const __grid_c
   tmem_fence_after();
   const uint32_t tmem = tmem_base;
   const uint32_t lane_base = (uint32_t)(32 * (warp & 3)) << 16;  // this warp's tensor-memory lane quadrant
-  if (warp >= 2 && warp < 6) {  // all 32 slots start at zero
-    for (int b = 0; b < 32; ++b) tmem_zero16(tmem + lane_base + (uint32_t)(16 * b));
+  if (warp >= 2 && warp < 6) {  // all slots start at zero
+    for (int b = 0; b < kR; ++b) tmem_zero16(tmem + lane_base + (uint32_t)(16 * b));
     asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
   }
   tmem_fence_before();
   __syncthreads();
   tmem_fence_after();
 
-  // The CTA's columns b, b + G, b + 2G, ... (G = gridDim.x) are dealt to the
-  // kNS streams in turn; items (one input row of one stream) are visited by
-  // every role in the same order: groups of one input per live stream,
-  // streams in order.
-  const long long cstep = (long long)kNS * gridDim.x;
-  Stream st[kNS];
-#pragma unroll
-  for (int s = 0; s < kNS; ++s) {
-    st[s].col = blockIdx.x + (long long)s * gridDim.x;
-    st[s].i = 0;
-    st[s].p = 0;
-    st[s].ph = 0;
-    if (st[s].col < g.columns) st[s].c = column_of(g, st[s].col);
-  }
-  auto advance = [&](Stream& t) {
-    if (++t.p == kR) {
-      t.p = 0;
-      t.ph ^= 1u;
-    }
-    if (++t.i == t.c.nt + 2) {
-      t.i = 0;
-      t.col += cstep;
-      if (t.col < g.columns) t.c = column_of(g, t.col);
-    }
-  };
-  auto row_y = [&](const Stream& t) { return t.c.yph + (t.i - 1) * dil; };
+  // Every role visits the CTA's columns and their input rows (items) in the same
+  // order.
+  Walk t;
+  t.start(g, s_start);
 
-  // progress (lane 0 of warps 0 / 1): items whose rows / residual rows were
+  // progress (warps 0 / 1 / kResWarp): items whose rows / residual rows were
   // loaded; the done barrier and parity of the last commit
   long long q_loaded = 0, q_res = 0;
   int last_done = -1;
@@ -314,279 +429,214 @@ __global__ void __launch_bounds__(kThreads, 1) conv16_umma_kernel(const __grid_c
   if (warp == 0) {
     // ---- producer, the whole warp in step, one elected lane issuing: each
     // item's z-rows into the row ring
+    const uint32_t box_bytes = 32u * (uint32_t)(kPacked ? g.W * g.lines : kTileM + 2 * dil);
+    const int xo = kPacked ? 0 : dil;
     Ring<kRowSlots> rr;
-    bool stop = false, any = true;
-    while (any && !stop) {
-      any = false;
-#pragma unroll
-      for (int s = 0; s < kNS; ++s) {
-        Stream& t = st[s];
-        if (stop || t.col >= g.columns) continue;
-        any = true;
-        const bool okE = !rr.wrapped || mbar_wait_fast(&empty_bar[rr.idx], rr.ph ^ 1u, wait_lim);
-        if (!__all_sync(0xffffffffu, okE && !s_fail)) {
-          s_fail = 1;
-          stop = true;
-          continue;
-        }
-        const int yy = row_y(t);
-        uint32_t nvalid = 0;
-        if (yy >= 0 && yy < g.H)
-          for (int dz = 0; dz < 3; ++dz) {
-            const int zz = t.c.z + (dz - 1) * dil;
-            nvalid += (zz >= 0 && zz < g.D) ? 1u : 0u;
-          }
-        if (nvalid == 0) {
-          arrive_elect(&full_bar[rr.idx]);
-        } else {
-          expect_tx_elect(&full_bar[rr.idx], nvalid * box_bytes);
-          uint8_t* dst = rows + (size_t)rr.idx * kSlotBytes;
-          for (int dz = 0; dz < 3; ++dz) {
-            const int zz = t.c.z + (dz - 1) * dil;
-            if (zz >= 0 && zz < g.D)
-              tma_load_5d(dst + dz * kRowBytes, &xmap, 0, t.c.x0 - dil, 0, yy, t.c.n * g.D + zz, &full_bar[rr.idx]);
-          }
-        }
-        rr.next();
-        ++q_loaded;
-        advance(t);
+    Ring<kR> old;  // the done barrier of the item kRowSlots before
+    uint32_t zm = t.z_mask(g);
+    while (t.live) {
+      bool ok = !s_fail;
+      if (rr.wrapped) {
+        ok = ok && mbar_wait_fast(&done_bar[old.idx], old.ph, wait_lim);
+        old.next();
       }
+      if (!__all_sync(0xffffffffu, ok)) {
+        s_fail = 1;
+        break;
+      }
+      const int yy = t.y(g);
+      if (yy < 0 || yy >= g.H || zm == 0) {
+        arrive_elect(&full_bar[rr.idx]);
+      } else {
+        expect_tx_elect(&full_bar[rr.idx], (uint32_t)__popc(zm) * box_bytes);
+        uint8_t* dst = rows + (size_t)rr.idx * kSlotBytes;
+#pragma unroll
+        for (int dz = 0; dz < 3; ++dz)
+          if (zm & (1u << dz))
+            tma_load_5d(dst + dz * kRowBytes, &xmap, t.x0 - xo, yy, t.z + (dz - 1) * dil, t.n, &full_bar[rr.idx]);
+      }
+      rr.next();
+      ++q_loaded;
+      if (t.next(g, s_start)) zm = t.z_mask(g);
     }
   } else if (warp == kResWarp) {
     // ---- residual loader, the whole warp in step: for each item the
     // residual row of the position it completes (output j = i - 2; padding
     // positions arrive without a copy)
     Ring<kResSlots> sr;
-    bool stop = !has_res, any = true;
-    while (any && !stop) {
-      any = false;
-#pragma unroll
-      for (int s = 0; s < kNS; ++s) {
-        Stream& t = st[s];
-        if (stop || t.col >= g.columns) continue;
-        any = true;
-        const bool okR = !sr.wrapped || mbar_wait_fast(&rfree_bar[sr.idx], sr.ph ^ 1u, wait_lim);
-        if (!__all_sync(0xffffffffu, okR && !s_fail)) {
-          s_fail = 1;
-          stop = true;
-          continue;
-        }
-        if (t.i >= 2) {
-          expect_tx_elect(&rfull_bar[sr.idx], (uint32_t)kResBytes);
-          tma_load_5d(rres + (size_t)sr.idx * kResBytes, &rmap, 0, t.c.x0, 0, t.c.yph + (t.i - 2) * dil,
-                      t.c.n * g.D + t.c.z, &rfull_bar[sr.idx]);
-        } else {
-          arrive_elect(&rfull_bar[sr.idx]);
-        }
-        sr.next();
-        ++q_res;
-        advance(t);
+    const uint32_t res_bytes = kPacked ? 32u * (uint32_t)(g.W * g.lines) : (uint32_t)kResBytes;
+    while (has_res && t.live) {
+      bool ok = !s_fail;
+      if (sr.wrapped) ok = ok && mbar_wait_fast(&rfree_bar[sr.idx], sr.ph ^ 1u, wait_lim);
+      if (!__all_sync(0xffffffffu, ok)) {
+        s_fail = 1;
+        break;
       }
+      if (t.i >= 2) {
+        expect_tx_elect(&rfull_bar[sr.idx], res_bytes);
+        tma_load_5d(rres + (size_t)sr.idx * kResBytes, &rmap, t.x0, t.y(g) - dil, t.z, t.n, &rfull_bar[sr.idx]);
+      } else {
+        arrive_elect(&rfull_bar[sr.idx]);
+      }
+      sr.next();
+      ++q_res;
+      t.next(g, s_start);
     }
   } else if (warp == 1) {
     // ---- MMA issuer, the whole warp in step (operands warp-uniform), one
-    // elected lane issuing: descriptors precomputed; per item only the row
-    // slot's base and the accumulator column change; a group's MMAs
-    // alternate between its streams
+    // elected lane issuing. Its own instructions bound a column's walk, so an
+    // item costs it one barrier test (even lanes the row, odd lanes the
+    // position), three issue blocks and one commit.
     const uint32_t tm = __shfl_sync(0xffffffffu, tmem, 0);
     // weight block b = dz*3 + dx: descriptor bdesc0 + b * kWBlockBytes / 16
-    const uint64_t bdesc0 = smem_desc(smem_u32(sw), 768, 128);
-    const uint64_t adesc0 = smem_desc(smem_u32(rows), 16u * (uint32_t)rv, 128);
-    const uint64_t ddx = (uint64_t)dil;  // one dx step in descriptor start-address units (16 bytes)
-    Ring<kRowSlots> rr;
-    // position k + 2 of each stream (first touched by input k): index, phase, wrapped
-    int p2[kNS];
-    uint32_t ph2[kNS], w2[kNS];
+    const uint64_t bdesc0 = smem_desc<0>(smem_u32(sw), 768, 128);
+    const uint64_t ddx = (uint64_t)(2 * dil);  // one dx step in descriptor start-address units (16 bytes)
+    const uint64_t adesc0 = smem_desc<6>(smem_u32(rows) - (kPacked ? 32u * (uint32_t)dil : 0u), 16, 256);
+    uint32_t ml[4], mr[4];  // packed: lanes whose left / right neighbour is outside the row
+    if (kPacked) {
 #pragma unroll
-    for (int s = 0; s < kNS; ++s) {
-      p2[s] = 2;
-      ph2[s] = 0;
-      w2[s] = 0;
+      for (int q = 0; q < 4; ++q) {
+        const int m = 32 * q + lane, x = m % g.W;
+        ml[q] = __ballot_sync(0xffffffffu, x < dil);
+        mr[q] = __ballot_sync(0xffffffffu, x + dil >= g.W);
+      }
     }
-    bool run = true;
-    while (run) {
-      bool live[kNS];
-      int ns = 0;
-#pragma unroll
-      for (int s = 0; s < kNS; ++s) {
-        live[s] = st[s].col < g.columns;
-        ns += live[s] ? 1 : 0;
+    Ring<kRowSlots> rr;
+    Ring<kR> p2;  // position k + 2, first touched by input k
+    p2.idx = 2;
+    uint32_t zm = t.z_mask(g);
+    auto issue = [&](uint32_t d, uint64_t a, uint64_t b, auto width) {
+      constexpr int kN = decltype(width)::value;
+      if (kPacked)
+        umma3<kN>(d, a, ddx, b, ml, mr);
+      else
+        umma3<kN>(d, a, ddx, b);
+    };
+    while (t.live) {
+      const bool odd = (lane & 1) && p2.wrapped;
+      const int failed = s_fail;
+      const bool ok = mbar_wait_fast(odd ? &free_bar[p2.idx] : &full_bar[rr.idx], odd ? p2.ph ^ 1u : rr.ph, wait_lim);
+      if (!__all_sync(0xffffffffu, ok && !failed)) {  // one decision for the whole warp
+        s_fail = 1;
+        break;
       }
-      if (ns == 0) break;
-      bool ok = true;
-      uint64_t ad[kNS];
-      uint32_t dd[kNS], d0[kNS], zm[kNS];
-      int wrap[kNS];  // 0: the region fits; 1: 2 + 1 slots split at the ring end; 2: 1 + 2
-      int slot[kNS];
-      Ring<kRowSlots> r2 = rr;
+      __syncwarp();  // what the odd lanes saw released holds for the issuing lane
+      tmem_fence_after();
+      const int yy = t.y(g);
+      if (yy >= 0 && yy < g.H) {
+        const uint64_t ad = adesc0 + (uint64_t)((rr.idx * kSlotBytes) >> 4);
+        const uint32_t dd = tm + (uint32_t)(16 * t.p);
+        if (t.p <= kR - 3) {
 #pragma unroll
-      for (int s = 0; s < kNS; ++s) {
-        zm[s] = 0;
-        slot[s] = r2.idx;
-        if (!live[s]) continue;
-        const Stream& t = st[s];
-        ok = ok && mbar_wait_fast(&full_bar[r2.idx], r2.ph, wait_lim);
-        if (w2[s]) ok = ok && mbar_wait_fast(&free_bar[s * kR + p2[s]], ph2[s] ^ 1u, wait_lim);
-        ad[s] = adesc0 + (uint64_t)((r2.idx * kSlotBytes) >> 4);
-        dd[s] = tm + (uint32_t)(s * kR * 16 + 16 * t.p);
-        d0[s] = tm + (uint32_t)(s * kR * 16);
-        wrap[s] = t.p <= kR - 3 ? 0 : (t.p == kR - 2 ? 1 : 2);
-        const int yy = row_y(t);
-        if (yy >= 0 && yy < g.H)
-#pragma unroll
+          for (int dz = 0; dz < 3; ++dz)
+            if (zm & (1u << dz))
+              issue(dd, ad + (uint64_t)((dz * kRowBytes) >> 4), bdesc0 + (uint64_t)(dz * 3 * (kWBlockBytes >> 4)),
+                    std::integral_constant<int, 48>{});
+        } else {
+          // a region running past the ring end continues at slot 0; the
+          // second piece starts 32 or 16 weight rows (16 bytes each) in
+#pragma unroll 1
           for (int dz = 0; dz < 3; ++dz) {
-            const int zz = t.c.z + (dz - 1) * dil;
-            zm[s] |= (zz >= 0 && zz < g.D) ? (1u << dz) : 0u;
+            if (!(zm & (1u << dz))) continue;
+            const uint64_t a = ad + (uint64_t)((dz * kRowBytes) >> 4);
+            const uint64_t b = bdesc0 + (uint64_t)(dz * 3 * (kWBlockBytes >> 4));
+            if (t.p == kR - 2) {
+              issue(dd, a, b, std::integral_constant<int, 32>{});
+              issue(tm, a, b + 32, std::integral_constant<int, 16>{});
+            } else {
+              issue(dd, a, b, std::integral_constant<int, 16>{});
+              issue(tm, a, b + 16, std::integral_constant<int, 32>{});
+            }
           }
-        r2.next();
+        }
       }
-      if (!__all_sync(0xffffffffu, ok && !s_fail)) {  // one decision for the whole warp
+      last_done = t.p;
+      last_par = t.ph;
+      umma_commit(&done_bar[last_done]);
+      rr.next();
+      p2.next();
+      if (t.next(g, s_start)) zm = t.z_mask(g);
+    }
+  } else {
+    // ---- epilogue (warps 2 .. kResWarp - 1): every item's completed position, in item order
+    const int m = 32 * (warp & 3) + lane;  // tensor-memory lane = voxel offset in the tile
+    const int line = kPacked ? m / g.W : 0, mx = kPacked ? m - line * g.W : m;
+    Ring<kResSlots> sr;
+    while (t.live) {
+      const int p = t.p;
+      bool ok = !s_fail && mbar_wait_fast(&done_bar[p], t.ph, wait_lim);
+      if (has_res) ok = ok && mbar_wait_fast(&rfull_bar[sr.idx], sr.ph, wait_lim);
+      if (!__all_sync(0xffffffffu, ok)) {
         s_fail = 1;
         break;
       }
       tmem_fence_after();
-      bool any_wrap = false;
-#pragma unroll
-      for (int s = 0; s < kNS; ++s) any_wrap |= wrap[s] != 0;
-      if (!any_wrap) {  // every region fits: 9 MMAs of N = 48 per item
-#pragma unroll
-        for (int dz = 0; dz < 3; ++dz)
-#pragma unroll
-          for (int dx = 0; dx < 3; ++dx)
-#pragma unroll
-            for (int s = 0; s < kNS; ++s)
-              if (zm[s] & (1u << dz))
-                umma_f16<48>(dd[s], ad[s] + (uint64_t)((dz * kRowBytes) >> 4) + (uint64_t)dx * ddx,
-                             bdesc0 + (uint64_t)((dz * 3 + dx) * (kWBlockBytes >> 4)));
-      } else {
-#pragma unroll 1
-        for (int dz = 0; dz < 3; ++dz)
-#pragma unroll 1
-          for (int dx = 0; dx < 3; ++dx)
-#pragma unroll
-            for (int s = 0; s < kNS; ++s) {
-              if (!(zm[s] & (1u << dz))) continue;
-              const uint64_t a = ad[s] + (uint64_t)((dz * kRowBytes) >> 4) + (uint64_t)dx * ddx;
-              const uint64_t b = bdesc0 + (uint64_t)((dz * 3 + dx) * (kWBlockBytes >> 4));
-              // a region running past the ring end continues at slot 0; the
-              // second piece starts 32 or 16 weight rows (16 bytes each) in
-              if (wrap[s] == 0) {
-                umma_f16<48>(dd[s], a, b);
-              } else if (wrap[s] == 1) {
-                umma_f16<32>(dd[s], a, b);
-                umma_f16<16>(d0[s], a, b + 32);
-              } else {
-                umma_f16<16>(dd[s], a, b);
-                umma_f16<32>(d0[s], a, b + 16);
-              }
-            }
+      const uint32_t ta = tmem + lane_base + (uint32_t)(16 * p);
+      uint32_t v[16];
+      if (t.i >= 2) {  // output row j = i - 2
+        tmem_ld16(ta, v);
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
       }
-#pragma unroll
-      for (int s = 0; s < kNS; ++s) {
-        if (!live[s]) continue;
-        Stream& t = st[s];
-        umma_commit(&empty_bar[slot[s]]);
-        last_done = s * kR + t.p;
-        last_par = t.ph;
-        umma_commit(&done_bar[last_done]);
-        if (++p2[s] == kR) {
-          p2[s] = 0;
-          ph2[s] ^= 1u;
-          w2[s] = 1u;
-        }
-        advance(t);
+      uint4 rq[2];
+      if (has_res) {
+        const uint8_t* rp = rres + (size_t)sr.idx * kResBytes + m * 32;
+        const int sz = (m >> 2) & 1;  // the swizzle swaps the halves of every other four rows
+        rq[0] = *reinterpret_cast<const uint4*>(rp + 16 * sz);
+        rq[1] = *reinterpret_cast<const uint4*>(rp + 16 * (sz ^ 1));
       }
-      rr = r2;
-    }
-  } else {
-    // ---- epilogue (warps 2 .. kResWarp - 1): every item's completed position, in item order, the
-    // groups taking turns
-    const int m = 32 * (warp & 3) + lane;  // tensor-memory lane = voxel offset in the tile
-    const int group = (warp - 2) >> 2;
-    int turn = 0;
-    Ring<kResSlots> sr;
-    bool stop = false, any = true;
-    while (any && !stop) {
-      any = false;
+      // position and residual slot are free before the row is finished and stored
+      tmem_zero16(ta);
+      asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+      tmem_fence_before();
+      __syncwarp();
+      if (lane == 0) {
+        mbar_arrive(&free_bar[p]);
+        if (has_res) mbar_arrive(&rfree_bar[sr.idx]);
+      }
+      if (t.i >= 2) {
+        float u[16];
 #pragma unroll
-      for (int s = 0; s < kNS; ++s) {
-        Stream& t = st[s];
-        if (stop || t.col >= g.columns) continue;
-        any = true;
-        const bool mine = turn == group;
-        if (++turn == kEpiGroups) turn = 0;
-        if (!mine) {
-          if (has_res) sr.next();
-          advance(t);
-          continue;
-        }
-        const int p = t.p;
-        bool ok = !s_fail && mbar_wait_fast(&done_bar[s * kR + p], t.ph, wait_lim);
-        if (has_res) ok = ok && mbar_wait_fast(&rfull_bar[sr.idx], sr.ph, wait_lim);
-        if (!__all_sync(0xffffffffu, ok)) {
-          s_fail = 1;
-          stop = true;
-          continue;
-        }
-        tmem_fence_after();
-        const uint32_t ta = tmem + lane_base + (uint32_t)(s * kR * 16 + 16 * p);
-        if (t.i >= 2) {  // output row j = i - 2 of the column
-          uint32_t v[16];
-          tmem_ld16(ta, v);
-          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-          float u[16];
+        for (int e = 0; e < 16; ++e) u[e] = __uint_as_float(v[e]);
+        const int x = t.x0 + mx, z = t.z + line;
+        if (x < g.W && line < g.lines && z < g.D) {
+          const long long r = (((long long)t.n * g.D + z) * g.H + (t.y(g) - dil)) * g.W + x;
 #pragma unroll
-          for (int e = 0; e < 16; ++e) u[e] = __uint_as_float(v[e]);
-          const int x = t.c.x0 + m, yo = t.c.yph + (t.i - 2) * dil;
-          if (x < g.W) {
-            const long long r = (((long long)t.c.n * g.D + t.c.z) * g.H + yo) * g.W + x;
+          for (int e = 0; e < 16; ++e) u[e] += s_bias[e];
+          if (has_res) {
 #pragma unroll
-            for (int e = 0; e < 16; ++e) u[e] += s_bias[e];
-            if (has_res) {
-              const uint8_t* rp = rres + (size_t)sr.idx * kResBytes + m * 16;
+            for (int h = 0; h < 2; ++h) {
+              const uint32_t words[4] = {rq[h].x, rq[h].y, rq[h].z, rq[h].w};
 #pragma unroll
-              for (int h = 0; h < 2; ++h) {
-                const uint4 rq = *reinterpret_cast<const uint4*>(rp + h * (kResBytes / 2));
-                const uint32_t words[4] = {rq.x, rq.y, rq.z, rq.w};
-#pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                  u[h * 8 + 2 * e] += __bfloat162float(__ushort_as_bfloat16((unsigned short)(words[e] & 0xFFFFu)));
-                  u[h * 8 + 2 * e + 1] += __bfloat162float(__ushort_as_bfloat16((unsigned short)(words[e] >> 16)));
-                }
+              for (int e = 0; e < 4; ++e) {
+                u[h * 8 + 2 * e] += __bfloat162float(__ushort_as_bfloat16((unsigned short)(words[e] & 0xFFFFu)));
+                u[h * 8 + 2 * e + 1] += __bfloat162float(__ushort_as_bfloat16((unsigned short)(words[e] >> 16)));
               }
-            }
-            if (relu) {
-#pragma unroll
-              for (int e = 0; e < 16; ++e) u[e] = fmaxf(u[e], 0.0f);
-            }
-            if (kOutF32) {
-              float4* op = reinterpret_cast<float4*>(static_cast<float*>(y_out) + r * 16);
-#pragma unroll
-              for (int e = 0; e < 4; ++e) op[e] = make_float4(u[4 * e], u[4 * e + 1], u[4 * e + 2], u[4 * e + 3]);
-            } else {
-              uint32_t pk[8];
-#pragma unroll
-              for (int e = 0; e < 8; ++e) {
-                const __nv_bfloat162 b2 = __floats2bfloat162_rn(u[2 * e], u[2 * e + 1]);
-                pk[e] = *reinterpret_cast<const uint32_t*>(&b2);
-              }
-              uint4* op = reinterpret_cast<uint4*>(static_cast<__nv_bfloat16*>(y_out) + r * 16);
-              op[0] = make_uint4(pk[0], pk[1], pk[2], pk[3]);
-              op[1] = make_uint4(pk[4], pk[5], pk[6], pk[7]);
             }
           }
+          if (relu) {
+#pragma unroll
+            for (int e = 0; e < 16; ++e) u[e] = fmaxf(u[e], 0.0f);
+          }
+          uint32_t pk[8];
+          if (kOutF32) {
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+#pragma unroll
+              for (int e = 0; e < 8; ++e) pk[e] = __float_as_uint(u[8 * h + e]);
+              store32(static_cast<float*>(y_out) + r * 16 + 8 * h, pk, wide);
+            }
+          } else {
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+              const __nv_bfloat162 b2 = __floats2bfloat162_rn(u[2 * e], u[2 * e + 1]);
+              pk[e] = *reinterpret_cast<const uint32_t*>(&b2);
+            }
+            store32(static_cast<__nv_bfloat16*>(y_out) + r * 16, pk, wide);
+          }
         }
-        tmem_zero16(ta);
-        asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-        tmem_fence_before();
-        __syncwarp();
-        if (lane == 0) {
-          mbar_arrive(&free_bar[s * kR + p]);
-          if (has_res) mbar_arrive(&rfree_bar[sr.idx]);
-        }
-        if (has_res) sr.next();
-        advance(t);
       }
+      sr.next();
+      t.next(g, s_start);
     }
   }
   __syncwarp();
@@ -611,14 +661,23 @@ __global__ void __launch_bounds__(kThreads, 1) conv16_umma_kernel(const __grid_c
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTmemCols) : "memory");
 }
 
-template <bool kOutF32, int kNS>
+template <bool kOutF32, bool kPacked>
 cudaError_t launch_conv16(const CUtensorMap& map, const CUtensorMap& rmap, const __nv_bfloat16* w, const float* bias,
-                          int has_res, void* y, const UmmaGeom& g, int relu, uint32_t wl, int grid, cudaStream_t st) {
-  const cudaError_t ae =
-      cudaFuncSetAttribute(conv16_umma_kernel<kOutF32, kNS>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
+                          int has_res, void* y, const UmmaGeom& g, int relu, int wide, int grid, cudaStream_t st) {
+  const auto kernel = conv16_umma_kernel<kOutF32, kPacked>;
+  const cudaError_t ae = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
   if (ae != cudaSuccess) return ae;
-  conv16_umma_kernel<kOutF32, kNS><<<grid, kThreads, kSmemBytes, st>>>(map, rmap, w, bias, has_res, y, g, relu, wl);
-  return cudaSuccess;
+  cudaLaunchConfig_t c{};
+  c.gridDim = dim3((unsigned)grid);
+  c.blockDim = dim3(kThreads);
+  c.dynamicSmemBytes = kSmemBytes;
+  c.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  c.attrs = at;
+  c.numAttrs = 1;
+  return cudaLaunchKernelEx(&c, kernel, map, rmap, w, bias, has_res, y, g, relu, wide, wait_limit());
 }
 
 }  // namespace
@@ -631,45 +690,55 @@ int conv16_umma(const void* x, const void* w, const float* bias, const void* res
   if ((long long)N * D > 0x7FFFFFFFll) return set_error(SI_ERR_ARG, "conv16_umma: too many z-planes");
   const EncodeTiledFn enc = encode_fn();
   if (!enc) return set_error(SI_ERR_CUDA, "conv16_umma: cuTensorMapEncodeTiled unavailable");
-  CUtensorMap map;
-  std::memset(&map, 0, sizeof(map));
-  // {8 channels, x, channel half, y, z*N}: the half dimension (16-byte stride)
-  // outside x makes one box land as [half][voxel][8 channels]
-  const cuuint64_t dims[5] = {8, (cuuint64_t)W, 2, (cuuint64_t)H, (cuuint64_t)D * (cuuint64_t)N};
-  const cuuint64_t strides[4] = {32ull, 16ull, 32ull * W, 32ull * W * H};  // bytes, dims 1..4
-  const cuuint32_t box[5] = {8, (cuuint32_t)(kTileM + 2 * dil), 2, 1, 1};
-  const cuuint32_t estr[5] = {1, 1, 1, 1, 1};
-  const CUresult cr = enc(&map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, const_cast<void*>(x), dims, strides, box, estr,
-                          CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
-                          CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  if (cr != CUDA_SUCCESS) return set_error(SI_ERR_CUDA, "conv16_umma: tensor map encoding failed (%d)", (int)cr);
-  // the residual, same layout, in boxes of one 128-voxel output tile
-  CUtensorMap rmap;
-  std::memset(&rmap, 0, sizeof(rmap));
-  if (residual) {
-    const cuuint32_t rbox[5] = {8, (cuuint32_t)kTileM, 2, 1, 1};
-    const CUresult rr = enc(&rmap, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, const_cast<void*>(residual), dims, strides,
-                            rbox, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
-                            CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (rr != CUDA_SUCCESS)
-      return set_error(SI_ERR_CUDA, "conv16_umma: residual tensor map encoding failed (%d)", (int)rr);
+  UmmaGeom g{};
+  g.N = N;
+  g.D = D;
+  g.H = H;
+  g.W = W;
+  g.dil = dil;
+  g.lines = std::max(1, std::min(kTileM / W, D));
+  const bool packed = g.lines > 1;
+  const int xchunks = (W + kTileM - 1) / kTileM, zgroups = (D + g.lines - 1) / g.lines;
+  const long long columns = (long long)N * zgroups * xchunks * dil;
+  g.nt = (H + dil - 1) / dil;
+  // one CTA per row at most; whole columns while every CTA has one, then rows
+  const long long grid = std::min(columns * g.nt, (long long)kCtasPerSm * sm_count());
+  g.rounds = (int)std::min<long long>(columns / grid, 0x7FFFFFFF);
+  g.tail_col = g.rounds * grid;
+  g.tail_rows = (columns - g.tail_col) * g.nt;
+  const int radix[kDigits] = {dil, xchunks, zgroups, N};
+  long long rest = grid;
+  for (int k = 0; k < kDigits; ++k) {
+    g.radix[k] = radix[k];
+    g.step[k] = (int)(rest % radix[k]);
+    rest /= radix[k];
   }
-  UmmaGeom g{N, D, H, W, dil, (W + kTileM - 1) / kTileM, 0};
-  g.columns = (long long)N * D * g.xchunks * dil;
-  if (g.columns == 0) return SI_OK;
-  const int has_res = residual ? 1 : 0;
-  const uint32_t wl = wait_limit();
-  const long long want = std::min<long long>(g.columns, (long long)sm_count());
+  // {16 channels, x, y, z, n}: a box lands as [line][voxel][16 channels], the halves
+  // of rows 4..7 of every eight swapped (32-byte swizzle)
+  const cuuint64_t dims[5] = {16, (cuuint64_t)W, (cuuint64_t)H, (cuuint64_t)D, (cuuint64_t)N};
+  const cuuint64_t strides[4] = {32ull, 32ull * W, 32ull * W * H, 32ull * W * H * D};  // bytes, dims 1..4
+  const cuuint32_t estr[5] = {1, 1, 1, 1, 1};
+  const cuuint32_t box[5] = {16, (cuuint32_t)(packed ? W : kTileM + 2 * dil), 1, (cuuint32_t)g.lines, 1};
+  const cuuint32_t rbox[5] = {16, (cuuint32_t)(packed ? W : kTileM), 1, (cuuint32_t)g.lines, 1};
+  CUtensorMap map, rmap;
+  std::memset(&map, 0, sizeof(map));
+  std::memset(&rmap, 0, sizeof(rmap));
+  const auto encode = [&](CUtensorMap* m, const void* ptr, const cuuint32_t* b) {
+    return enc(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, const_cast<void*>(ptr), dims, strides, b, estr,
+               CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_32B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  };
+  const CUresult cr = encode(&map, x, box);
+  if (cr != CUDA_SUCCESS) return set_error(SI_ERR_CUDA, "conv16_umma: tensor map encoding failed (%d)", (int)cr);
+  const CUresult rr = residual ? encode(&rmap, residual, rbox) : CUDA_SUCCESS;
+  if (rr != CUDA_SUCCESS)
+    return set_error(SI_ERR_CUDA, "conv16_umma: residual tensor map encoding failed (%d)", (int)rr);
+  const int has_res = residual ? 1 : 0, wide = (uintptr_t)y % 32 == 0;
   const auto* wb = static_cast<const __nv_bfloat16*>(w);
-  const int ns = g_umma_streams.load(std::memory_order_relaxed);
-  const cudaError_t ae =
-      out_f32 ? (ns == 4 ? launch_conv16<true, 4>(map, rmap, wb, bias, has_res, y, g, relu, wl, (int)want, st)
-                 : ns == 2 ? launch_conv16<true, 2>(map, rmap, wb, bias, has_res, y, g, relu, wl, (int)want, st)
-                           : launch_conv16<true, 1>(map, rmap, wb, bias, has_res, y, g, relu, wl, (int)want, st))
-              : (ns == 4 ? launch_conv16<false, 4>(map, rmap, wb, bias, has_res, y, g, relu, wl, (int)want, st)
-                 : ns == 2 ? launch_conv16<false, 2>(map, rmap, wb, bias, has_res, y, g, relu, wl, (int)want, st)
-                           : launch_conv16<false, 1>(map, rmap, wb, bias, has_res, y, g, relu, wl, (int)want, st));
-  if (ae != cudaSuccess) return set_error(SI_ERR_CUDA, "conv16_umma: shared memory opt-in: %s", cudaGetErrorString(ae));
+  const auto launch = out_f32 ? (packed ? launch_conv16<true, true> : launch_conv16<true, false>)
+                              : (packed ? launch_conv16<false, true> : launch_conv16<false, false>);
+  const cudaError_t ae = launch(map, rmap, wb, bias, has_res, y, g, relu, wide, (int)grid, st);
+  if (ae != cudaSuccess) return set_error(SI_ERR_CUDA, "conv16_umma: launch: %s", cudaGetErrorString(ae));
   return check_launch("conv16_umma");
 }
 
@@ -695,6 +764,5 @@ extern "C" int si_nn_conv16_tc_set_streams(int streams) {
   si::clear_error();
   if (streams != 1 && streams != 2 && streams != 4)
     return si::set_error(SI_ERR_ARG, "si_nn_conv16_tc_set_streams: 1, 2 or 4");
-  si::g_umma_streams.store(streams, std::memory_order_relaxed);
   return SI_OK;
 }

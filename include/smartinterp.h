@@ -569,11 +569,9 @@ int si_nn_conv16_tc(const void* x, const void* w, const float* bias,
  * reference. */
 int si_nn_umma_status(int* status, void* stream);
 
-/* Interleaved column streams per CTA of si_nn_conv16_tc: 1 (default), 2 or
- * 4. Each stream accumulates into its own tensor-memory ring, and the MMAs
- * of a group alternate between streams, so consecutive MMAs accumulate into
- * different columns (measured slower than one stream on GB300).
- * Process-wide; results do not depend on it. */
+/* Once the number of column streams that a CTA of si_nn_conv16_tc interleaved:
+ * 1, 2 or 4, other values are refused. Without effect: a CTA walks one column
+ * at a time, two CTAs share an SM. */
 int si_nn_conv16_tc_set_streams(int streams);
 
 /* dw[27][cout][cin] += sum_v dy[v][co] x[v + off][ci]; db[cout] += sum_v dy

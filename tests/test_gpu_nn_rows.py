@@ -89,3 +89,57 @@ def test_relu_backward(n, shift, with_add, cuda):
         exp = exp + t[2].float()
     S.relu_bwd(t[0], t[1], t[2] if with_add else None)
     assert torch.equal(t[0], exp.to(torch.bfloat16))
+
+
+def _conv64(x, w, b, d):
+    xd = torch.nn.functional.pad(x.double(), (0, 0, d, d, d, d, d, d))
+    _, D, H, W, _ = x.shape
+    out, mag = 0, 0
+    for k in range(27):
+        z, y, v = d * (k // 9), d * (k // 3 % 3), d * (k % 3)
+        s = xd[:, z:z + D, y:y + H, v:v + W]
+        out = out + s @ w[k].double().T
+        mag = mag + s.abs() @ w[k].double().abs().T
+    return out + b.double(), mag + b.double().abs()
+
+
+@pytest.mark.parametrize("shape,dil", [
+    ((1, 5, 4, 64), 1), ((2, 3, 9, 64), 8),    # two lines a tile, an odd last group
+    ((1, 7, 3, 40), 2), ((1, 4, 3, 43), 4),    # three and two lines, not a multiple of eight voxels
+    ((1, 130, 2, 1), 1), ((1, 40, 2, 3), 8),   # many lines; neighbours always outside the row
+    ((2, 1, 5, 64), 1),                        # one line: the tile with a halo
+    ((1, 2, 3, 65), 1), ((1, 3, 2, 128), 8), ((1, 2, 4, 129), 3),
+    ((1, 3, 5, 70), 8),                        # fewer rows than the dilation
+    ((1, 40, 90, 300), 1), ((3, 33, 70, 64), 2),  # whole columns and a split rest, rings that wrap
+], ids=str)
+def test_convolution_tiles(shape, dil, cuda):
+    g = torch.Generator(device="cuda").manual_seed(sum(shape) + dil)
+    x, res = _bf((*shape, 16), g), _bf((*shape, 16), g)
+    w, b = _bf((27, 16, 16), g, 0.1), torch.randn(16, generator=g, device="cuda")
+    x[:, -1, -1, -1] = 1e4  # a stray neighbour would be seen
+    st = torch.cuda.current_stream().cuda_stream
+    exp, mag = _conv64(x, w, b, dil)
+    tol = 16 * 2.0 ** -24 * np.sqrt(432)
+    for shift in (0, 4):  # outputs at 32-byte boundaries and 16 bytes past them
+        y = torch.empty(x.numel() + 8, device="cuda")[shift:shift + x.numel()].view(x.shape)
+        nat.call("si_nn_conv16_tc", x.data_ptr(), w.data_ptr(), b.data_ptr(), None, y.data_ptr(), *shape, dil, 0, 1, st)
+        assert float(((y.double() - exp).abs() / mag).max()) < tol
+        r = torch.empty(x.numel() + 16, dtype=torch.bfloat16, device="cuda")[2 * shift:2 * shift + x.numel()].view(x.shape)
+        nat.call("si_nn_conv16_tc", x.data_ptr(), w.data_ptr(), b.data_ptr(), res.data_ptr(), r.data_ptr(), *shape, dil,
+                 1, 0, st)
+        assert torch.equal(r, torch.relu(y + res.float()).to(torch.bfloat16))
+    S.umma_check()
+
+
+def test_convolution_infinite_neighbours(cuda):
+    """An infinity at the end of a line reaches its own line only."""
+    shape = (1, 4, 3, 64)
+    x = torch.zeros((*shape, 16), dtype=torch.bfloat16, device="cuda")
+    x[0, 1, 1, -1] = float("inf")
+    w = torch.ones((27, 16, 16), dtype=torch.bfloat16, device="cuda")
+    y = torch.empty((*shape, 16), device="cuda")
+    nat.call("si_nn_conv16_tc", x.data_ptr(), w.data_ptr(), None, None, y.data_ptr(), *shape, 1, 0, 1,
+             torch.cuda.current_stream().cuda_stream)
+    exp = torch.zeros_like(y)
+    exp[0, :3, :, -2:] = float("inf")
+    assert torch.equal(y, exp)
