@@ -981,8 +981,8 @@ extern "C" int si_nn_conv3d_wgrad(const void* x, const void* dy, float* dw, floa
   const auto* db16 = static_cast<const __nv_bfloat16*>(dy);
   const bool aligned = ((uintptr_t)x % 16 == 0) && ((uintptr_t)dy % 16 == 0);
   const bool fast = cout == 16 && cin == 16 && aligned;
+  uint64_t need = 0;
   if (partials) {
-    uint64_t need = 0;
     si_nn_wgrad_partial_bytes(N, D, H, W, cin, cout, &need);
     if (!fast) return set_error(SI_ERR_ARG, "si_nn_conv3d_wgrad: deterministic partials need cin = cout = 16");
     if (partial_bytes < need || (uintptr_t)partials % 16)
@@ -992,7 +992,10 @@ extern "C" int si_nn_conv3d_wgrad(const void* x, const void* dy, float* dw, floa
     const int xchunks = (W + 63) / 64;
     const int64_t rows = (int64_t)N * D * H * xchunks;
     const bool short_rows = dil <= kWgMaxDil;
-    const int64_t want = (int64_t)sm_count() * 8;
+    // wgrad16_rows_kernel's blocks write the bias sums behind their weight sums:
+    // as many blocks as the buffer holds
+    int64_t want = (int64_t)sm_count() * 8;
+    if (partials && short_rows) want = std::min(want, (int64_t)(need / (kWgOut * sizeof(float))));
     const int64_t per = (rows + want - 1) / want;
     const int64_t blocks = (rows + per - 1) / per;
     if (short_rows) {

@@ -143,3 +143,20 @@ def test_convolution_infinite_neighbours(cuda):
     exp = torch.zeros_like(y)
     exp[0, :3, :, -2:] = float("inf")
     assert torch.equal(y, exp)
+
+
+@pytest.mark.parametrize("shape", [(1, 19, 64, 64), (1, 8, 152, 1), (1, 1, 1, 1), (2, 30, 50, 70)], ids=str)
+def test_weight_gradient_stays_in_its_buffer(shape, cuda):
+    import ctypes
+    g = torch.Generator(device="cuda").manual_seed(1)
+    x, dy = _bf((*shape, 16), g), _bf((*shape, 16), g)
+    need = ctypes.c_uint64(0)
+    nat.call("si_nn_wgrad_partial_bytes", *shape, 16, 16, ctypes.byref(need))
+    guard = 1 << 18
+    buf = torch.full(((need.value + guard) // 4,), 7.0, device="cuda")
+    dw, db = torch.zeros(27 * 256, device="cuda"), torch.zeros(16, device="cuda")
+    nat.call("si_nn_conv3d_wgrad", x.data_ptr(), dy.data_ptr(), dw.data_ptr(), db.data_ptr(), *shape, 16, 16, 1,
+             buf.data_ptr(), need.value, torch.cuda.current_stream().cuda_stream)
+    assert bool((buf[need.value // 4:] == 7.0).all())
+    w, wm, b, bm = _wgrad64(x, dy, 1)
+    assert float(((dw.double().view(27, 16, 16) - w).abs() / (wm + 1)).max()) < 1e-5
