@@ -12,6 +12,7 @@
 
 #include <algorithm>
 #include <atomic>
+#include <type_traits>
 
 #include "si_common.cuh"
 #include "si_internal.h"
@@ -302,7 +303,7 @@ __global__ void __launch_bounds__(128) conv3d_wgrad_kernel(const __nv_bfloat16* 
 }
 
 // ---------------------------------------------------------------------------
-// 16 x 16 weight gradient for dilations that wgrad16_rows_kernel's rows do not
+// 16 x 16 weight gradient for dilations that wgrad16_columns_kernel's rows do not
 // hold. A block of 4 warps walks a run of 64-voxel x-rows;
 // per row the dY row is staged once in shared memory, and each warp handles
 // the taps w, w + 4, ... : it stages the shifted X row (zeros outside the
@@ -415,172 +416,252 @@ __global__ void __launch_bounds__(128) wgrad16_kernel(const __nv_bfloat16* __res
 }
 
 // ---------------------------------------------------------------------------
-// 16 x 16 weight and bias gradient, dilation up to kWgMaxDil. A CTA of nine
-// warps walks a run of 64-voxel x-rows of dY; warp j takes the input row at
-// (dz, dy) = (j / 3, j % 3) - 1 and its three taps along x, which read the same
-// staged row (64 voxels and the dilation on both sides) at shifted addresses. Rows
-// are staged two steps ahead by asynchronous copies in a ring of three slots, with
-// one CTA barrier per row. What bounds it: with a copy of every tap's row through
-// registers and no copy in flight across rows (wgrad16_kernel) the global loads'
-// latency did, 306 us on 8 x 64^3 voxels (94 TFLOP/s); this one takes 123 us (236
-// TFLOP/s), its shared-memory operand loads and mma.sync issue. The bias
-// gradient's sums are taken from the staged dY rows (37 us as a pass of its own).
+// 16 x 16 weight and bias gradient, dilation up to kWgMaxDil, by columns: (n, z,
+// x chunk of 64 voxels, y phase), rows y = phase + j * dil. Three warps walk a
+// column together; warp dz takes the input rows of plane z + (dz - 1) * dil and
+// meets every one with the dY rows above, at and below it: nine taps per warp. The
+// operands of the three dY rows stay in registers and move on with the walk, so a
+// row costs 4 + 12 ldmatrix for 72 MMAs, and is staged once (one dY row and three
+// input rows per step) by asynchronous copies in a ring of three slots.
+// The rows are split evenly into units, each with sums of its own. What bounds it:
+// mma.sync issue. Per layer of 8 x 64^3 voxels: 306 us with every tap's row copied
+// through registers (wgrad16_kernel), 121 us with nine staged input rows per dY row
+// and a tap row per warp (shared-memory loads, 36 ldmatrix for 54 MMAs), 88 us so.
+// The bias gradient's sums are taken from the same registers (37 us as a pass of its own).
 // ---------------------------------------------------------------------------
-constexpr int kWgMaxDil = 8, kWgWarps = 9, kWgStages = 3;
-constexpr int kWgRow = (64 + 2 * kWgMaxDil) * 32;          // bytes of a staged input row
-constexpr int kWgStage = 64 * 32 + kWgWarps * kWgRow;      // dY row, input rows
-constexpr int kWgSmem = kWgStages * kWgStage;
-constexpr int kWgOut = 27 * 256 + 16;                      // sums of a block: weights, bias
+constexpr int kWgMaxDil = 8, kWgGroups = 4, kWgStages = 3;
+constexpr int kWgRow = (64 + 2 * kWgMaxDil) * 32;   // bytes of a staged input row
+constexpr int kWgStage = 64 * 32 + 3 * kWgRow;      // dY row, input rows
+constexpr int kWgSmem = kWgGroups * kWgStages * kWgStage;
+constexpr int kXPieces = (64 + 2 * kWgMaxDil) * 2 / 32;  // 16-byte pieces of an input row per lane
+constexpr int kWgOut = 27 * 256 + 16;               // sums of a unit: weights, bias
+
+struct WgGeom {
+  int N, D, H, W, dil, xchunks;
+  int nt;          // rows of a column (of phase 0; others may have one less)
+  unsigned rows;   // rows of all columns, nt each
+  unsigned units;  // unit u takes rows [u * rows / units, (u + 1) * rows / units)
+};
 
 // 16 bytes to shared memory; zeros where !ok (src is not read then).
 __device__ __forceinline__ void copy_async16(uint32_t dst, const void* src, bool ok) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(ok ? 16 : 0) : "memory");
 }
 
-__global__ void __launch_bounds__(kWgWarps * 32, 3)
-    wgrad16_rows_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ dy,
-                        float* __restrict__ dw, float* __restrict__ db, float* __restrict__ partials, Vol5 g, int dil,
-                        int xchunks, int64_t rows_per_block) {
+__global__ void __launch_bounds__(kWgGroups * 96, 1)
+    wgrad16_columns_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ dy,
+                           float* __restrict__ dw, float* __restrict__ db, float* __restrict__ partials,
+                           const __grid_constant__ WgGeom g, int units_per_group) {
   extern __shared__ __align__(128) uint8_t smem[];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int64_t rows = (int64_t)g.N * g.D * g.H * xchunks;
-  const int64_t r0 = (int64_t)blockIdx.x * rows_per_block;
-  const int64_t r1 = r0 + rows_per_block < rows ? r0 + rows_per_block : rows;
-  const uint32_t base = (uint32_t)__cvta_generic_to_shared(smem);
-  const int dz = (warp / 3 - 1) * dil, dyo = (warp % 3 - 1) * dil;
-  const int chunks = (64 + 2 * dil) * 2;  // 16-byte pieces of an input row
-  // position of the next row to stage; whether this warp's input row exists
-  int xc, yy, zz, n;
-  {
-    int64_t t = r0;
-    xc = (int)(t % xchunks);
-    t /= xchunks;
-    yy = (int)(t % g.H);
-    t /= g.H;
-    zz = (int)(t % g.D);
-    n = (int)(t / g.D);
-  }
-  unsigned exists = 0u;  // bit s: slot s holds an input row
-  auto stage = [&](int64_t row, int slot) {
-    if (row < r1) {
-      const uint32_t at = base + slot * kWgStage;
-      const int xb = xc * 64;
-      const int64_t vox = (((int64_t)n * g.D + zz) * g.H + yy) * g.W;
-      if (warp < 4) {  // 128 threads x 16 bytes of dY
-        const int v = threadIdx.x >> 1, h = threadIdx.x & 1;
-        const bool ok = xb + v < g.W;
-        copy_async16(at + swz(v, h), dy + (vox + (ok ? xb + v : 0)) * 16 + h * 8, ok);
-      }
-      const int zi = zz + dz, yi = yy + dyo;
-      const bool zy = (unsigned)zi < (unsigned)g.D && (unsigned)yi < (unsigned)g.H;
-      exists = (exists & ~(1u << slot)) | ((unsigned)zy << slot);
-      if (zy) {
-        const __nv_bfloat16* xrow = x + (((int64_t)n * g.D + zi) * g.H + yi) * g.W * 16;
-        const uint32_t to = at + 64 * 32 + warp * kWgRow;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, group = warp / 3, dzi = warp % 3;
+  const int gt = dzi * 32 + lane;  // thread of the group
+  const uint32_t base = (uint32_t)__cvta_generic_to_shared(smem) + group * (kWgStages * kWgStage);
+  const unsigned u0 = (blockIdx.x * kWgGroups + group) * (unsigned)units_per_group;
+  const unsigned u1 = min(u0 + (unsigned)units_per_group, g.units);
+  const int dz = (dzi - 1) * g.dil;
+  const int chunks = (64 + 2 * g.dil) * 2;  // 16-byte pieces of an input row
+
+  // The next step to stage: input row i of the segment (a column's part in the
+  // unit), with the dY row i + 1 below it.
+  unsigned u = u0, r = 0, r1 = 0;  // unit; first row behind the segment; end of the unit
+  int i = 0, jn = 0, yi = 0;  // yi: the input row's y
+  bool empty = false, zin = false;
+  unsigned okx = 0, okd = 0;  // this lane's pieces that lie inside the row
+  const char *xp = nullptr, *dp = nullptr;  // its first piece of the input row, of the dY row
+  const int64_t step = (int64_t)g.dil * g.W * 32;
+  auto enter = [&]() {  // the segment at row r
+    unsigned c = r / (unsigned)g.nt;
+    const int j0 = (int)(r - c * (unsigned)g.nt);
+    const int yph = (int)(c % (unsigned)g.dil);
+    c /= (unsigned)g.dil;
+    const int xb = (int)(c % (unsigned)g.xchunks) * 64;
+    c /= (unsigned)g.xchunks;
+    const int z = (int)(c % (unsigned)g.D), n = (int)(c / (unsigned)g.D);
+    const int most = (int)min((unsigned)(g.nt - j0), r1 - r);
+    r += (unsigned)most;
+    jn = min(j0 + most, (g.H - yph + g.dil - 1) / g.dil);
+    empty = jn <= j0;  // a row that this phase does not have: a step without rows
+    i = j0 - 1;
+    if (empty) jn = i;
+    yi = yph + i * g.dil;
+    zin = (unsigned)(z + dz) < (unsigned)g.D;
+    okx = okd = 0;
 #pragma unroll
-        for (int k = 0; k < (64 + 2 * kWgMaxDil) * 2 / 32; ++k) {
-          const int q = lane + 32 * k, v = q >> 1, h = q & 1;
-          const int xi = xb - dil + v;
-          const bool ok = (unsigned)xi < (unsigned)g.W;
-          if (q < chunks) copy_async16(to + swz(v, h), xrow + (int64_t)(ok ? xi : 0) * 16 + h * 8, ok);
-        }
+    for (int k = 0; k < kXPieces; ++k) {
+      const int q = lane + 32 * k;
+      if (q < chunks && (unsigned)(xb - g.dil + (q >> 1)) < (unsigned)g.W) okx |= 1u << k;
+    }
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      const int q = gt + 96 * k;
+      if (q < 128 && xb + (q >> 1) < g.W) okd |= 1u << k;
+    }
+    const int64_t plane = ((int64_t)n * g.D + z) * g.H;
+    xp = reinterpret_cast<const char*>(x) + ((plane + (int64_t)dz * g.H + yi) * g.W + xb - g.dil) * 32 + lane * 16;
+    dp = reinterpret_cast<const char*>(dy) + ((plane + yi + g.dil) * g.W + xb) * 32 + gt * 16;
+  };
+  auto bounds = [&]() {
+    r = (unsigned)((unsigned long long)g.rows * u / g.units);
+    r1 = (unsigned)((unsigned long long)g.rows * (u + 1) / g.units);
+    enter();
+  };
+  if (u < u1) bounds();
+  // per slot: 1 a step, 2 input row, 4 dY row, 8 first of a segment, 16 last of a unit
+  unsigned flags = 0;
+  bool first = true;
+  auto stage = [&](int slot) {
+    unsigned f = 0;
+    if (u < u1) {
+      const uint32_t at = base + slot * kWgStage;
+      f = 1u | (first ? 8u : 0u);
+      first = false;
+      // pieces of 16 bytes, 32 or 96 of them apart: 16 or 48 voxels, whole turns of the swizzle
+      if (i + 1 < jn && !empty) {
+        f |= 4u;
+#pragma unroll
+        for (int k = 0; k < 2; ++k)
+          if (gt + 96 * k < 128)
+            copy_async16(at + swz(gt >> 1, gt & 1) + k * 1536, (okd >> k) & 1u ? dp + k * 1536 : (const char*)dy,
+                         (okd >> k) & 1u);
       }
-      if (++xc == xchunks) {
-        xc = 0;
-        if (++yy == g.H) {
-          yy = 0;
-          if (++zz == g.D) {
-            zz = 0;
-            ++n;
-          }
+      if (!empty && zin && (unsigned)yi < (unsigned)g.H) {
+        f |= 2u;
+        const uint32_t to = at + 64 * 32 + dzi * kWgRow + swz(lane >> 1, lane & 1);
+#pragma unroll
+        for (int k = 0; k < kXPieces; ++k)
+          if (lane + 32 * k < chunks)
+            copy_async16(to + k * 512, (okx >> k) & 1u ? xp + k * 512 : (const char*)x, (okx >> k) & 1u);
+      }
+      yi += g.dil;
+      xp += step;
+      dp += step;
+      if (i++ == jn) {  // the segment's last step
+        first = true;
+        if (r < r1) {
+          enter();
+        } else {
+          f |= 16u;
+          if (++u < u1) bounds();
         }
       }
     }
+    flags = (flags & ~(31u << (5 * slot))) | (f << (5 * slot));
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
-  float acc[3][2][4];
+
+  float acc[9][2][4];
 #pragma unroll
-  for (int i = 0; i < 3; ++i)
+  for (int t = 0; t < 9; ++t)
 #pragma unroll
-    for (int j = 0; j < 2; ++j) acc[i][j][0] = acc[i][j][1] = acc[i][j][2] = acc[i][j][3] = 0.0f;
-  float bias = 0.0f, lost = 0.0f;  // thread t < 256: channel t % 16, voxels 4 (t / 16) .. + 3 of every row
-  const int bc = threadIdx.x & 15, bv = (threadIdx.x >> 4) * 4;
-  // ldmatrix row addresses as in wgrad16_kernel
-  const int q = lane >> 3, i8 = lane & 7;
-  const int va = i8 + ((q >> 1) << 3), ha = q & 1;
+    for (int j = 0; j < 2; ++j) acc[t][j][0] = acc[t][j][1] = acc[t][j][2] = acc[t][j][3] = 0.0f;
+  float bias[2] = {0.0f, 0.0f}, lost[2] = {0.0f, 0.0f};  // channels grp and grp + 8, this lane's voxels
+  uint32_t a[3][4][4];                                   // dY rows i - 1, i, i + 1 by k step
+  unsigned have = 0;                                     // bit: row in a[.]
+  const int q = lane >> 3, i8 = lane & 7, grp = lane >> 2, tig = lane & 3;
+  const int va = i8 + ((q >> 1) << 3), ha = q & 1;  // ldmatrix row addresses as in wgrad16_kernel
   const int vb = i8 + ((q & 1) << 3), hb = q >> 1;
-  stage(r0, 0);
-  stage(r0 + 1, 1);
+  unsigned unit = u0;
+  stage(0);
+  stage(1);
   int slot = 0;
-  for (int64_t row = r0; row < r1; ++row) {
+  while (true) {
+    const unsigned f = (flags >> (5 * slot)) & 31u;
+    if (!(f & 1u)) break;
     asm volatile("cp.async.wait_group 1;" ::: "memory");
-    __syncthreads();  // the row has landed; the slot staged below was last read one row ago
-    stage(row + 2, slot == 0 ? 2 : slot - 1);
-    const uint32_t sdy = base + slot * kWgStage, sx = sdy + 64 * 32 + warp * kWgRow;
-    if ((exists >> slot) & 1u) {
+    // the step's rows have landed; the slot staged below was last read a step ago
+    asm volatile("bar.sync %0, 96;" ::"r"(group + 1) : "memory");
+    stage(slot == 0 ? 2 : slot - 1);
+    const uint32_t sdy = base + slot * kWgStage, sx = sdy + 64 * 32 + dzi * kWgRow;
+    have = (f & 8u) ? 0u : have >> 1;
 #pragma unroll
-      for (int ks = 0; ks < 4; ++ks) {
-        uint32_t a[4];
-        ldsm_x4_trans(a, sdy + swz(ks * 16 + va, ha));
+    for (int ks = 0; ks < 4; ++ks)
 #pragma unroll
-        for (int i = 0; i < 3; ++i) {
-          uint32_t b[4];
-          ldsm_x4_trans(b, sx + swz(ks * 16 + vb + i * dil, hb));
-          mma_bf16(acc[i][0], a, b[0], b[1]);
-          mma_bf16(acc[i][1], a, b[2], b[3]);
+      for (int e = 0; e < 4; ++e) {
+        a[0][ks][e] = a[1][ks][e];
+        a[1][ks][e] = a[2][ks][e];
+      }
+    if (f & 4u) {
+      have |= 4u;
+#pragma unroll
+      for (int ks = 0; ks < 4; ++ks) ldsm_x4_trans(a[2][ks], sdy + swz(ks * 16 + va, ha));
+      if (db && dzi == 1) {
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+          float t = 0.0f;
+#pragma unroll
+          for (int ks = 0; ks < 4; ++ks) {
+            const uint32_t w0 = a[2][ks][c], w1 = a[2][ks][c + 2];
+            t += (__uint_as_float(w0 << 16) + __uint_as_float(w0 & 0xFFFF0000u)) +
+                 (__uint_as_float(w1 << 16) + __uint_as_float(w1 & 0xFFFF0000u));
+          }
+          // compensated (Kahan): the sum of a unit's rows is as good as one rounding
+          const float add = __fsub_rn(t, lost[c]), sum = __fadd_rn(bias[c], add);
+          lost[c] = __fsub_rn(__fsub_rn(sum, bias[c]), add);
+          bias[c] = sum;
         }
       }
     }
-    if (db && threadIdx.x < 256) {
-      float t[4];
+    // dY row i - 1 + k meets the input row at 1 - k along y
+    auto multiply = [&](auto all) {
 #pragma unroll
-      for (int k = 0; k < 4; ++k)
-        t[k] = __bfloat162float(*reinterpret_cast<const __nv_bfloat16*>(smem + slot * kWgStage +
-                                                                       swz(bv + k, bc >> 3) + (bc & 7) * 2));
-      // compensated (Kahan): the sum of a block's rows is as good as one rounding
-      const float add = __fsub_rn((t[0] + t[1]) + (t[2] + t[3]), lost), sum = __fadd_rn(bias, add);
-      lost = __fsub_rn(__fsub_rn(sum, bias), add);
-      bias = sum;
+      for (int ks = 0; ks < 4; ++ks) {
+        uint32_t b[3][4];
+#pragma unroll
+        for (int dx = 0; dx < 3; ++dx) ldsm_x4_trans(b[dx], sx + swz(ks * 16 + vb + dx * g.dil, hb));
+#pragma unroll
+        for (int k = 0; k < 3; ++k)
+          if (decltype(all)::value || (have & (1u << k)))
+#pragma unroll
+            for (int dx = 0; dx < 3; ++dx) {
+              mma_bf16(acc[(2 - k) * 3 + dx][0], a[k][ks], b[dx][0], b[dx][1]);
+              mma_bf16(acc[(2 - k) * 3 + dx][1], a[k][ks], b[dx][2], b[dx][3]);
+            }
+      }
+    };
+    if (f & 2u) {
+      if (have == 7u)
+        multiply(std::true_type{});
+      else
+        multiply(std::false_type{});
+    }
+    if (f & 16u) {  // the unit's sums
+      float* out = partials ? partials + (int64_t)unit * kWgOut : dw;
+#pragma unroll
+      for (int t = 0; t < 9; ++t)
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          float* d = out + (dzi * 9 + t) * 256 + grp * 16 + j * 8 + tig * 2;
+          if (partials) {  // deterministic: reduced in unit order afterwards
+            *reinterpret_cast<float2*>(d) = make_float2(acc[t][j][0], acc[t][j][1]);
+            *reinterpret_cast<float2*>(d + 128) = make_float2(acc[t][j][2], acc[t][j][3]);
+          } else {
+            atomicAdd(d, acc[t][j][0]);
+            atomicAdd(d + 1, acc[t][j][1]);
+            atomicAdd(d + 128, acc[t][j][2]);
+            atomicAdd(d + 129, acc[t][j][3]);
+          }
+          acc[t][j][0] = acc[t][j][1] = acc[t][j][2] = acc[t][j][3] = 0.0f;
+        }
+      if (dzi == 1) {
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+          float t = bias[c];
+          t += __shfl_xor_sync(0xffffffffu, t, 1);
+          t += __shfl_xor_sync(0xffffffffu, t, 2);
+          if (tig == 0) {
+            if (partials)
+              out[27 * 256 + grp + 8 * c] = t;
+            else if (db)
+              atomicAdd(&db[grp + 8 * c], t);
+          }
+          bias[c] = lost[c] = 0.0f;
+        }
+      }
+      ++unit;
     }
     slot = slot == 2 ? 0 : slot + 1;
   }
   asm volatile("cp.async.wait_all;" ::: "memory");
-  const int grp = lane >> 2, tig = lane & 3;
-  float* out = partials ? partials + (int64_t)blockIdx.x * kWgOut : dw;
-#pragma unroll
-  for (int i = 0; i < 3; ++i) {
-    const int tap = warp * 3 + i;
-#pragma unroll
-    for (int j = 0; j < 2; ++j) {
-      float* d = out + tap * 256 + grp * 16 + j * 8 + tig * 2;
-      if (partials) {  // deterministic: this block's sums, reduced in block order afterwards
-        *reinterpret_cast<float2*>(d) = make_float2(acc[i][j][0], acc[i][j][1]);
-        *reinterpret_cast<float2*>(d + 128) = make_float2(acc[i][j][2], acc[i][j][3]);
-      } else {
-        atomicAdd(d, acc[i][j][0]);
-        atomicAdd(d + 1, acc[i][j][1]);
-        atomicAdd(d + 128, acc[i][j][2]);
-        atomicAdd(d + 129, acc[i][j][3]);
-      }
-    }
-  }
-  if (db) {  // the 16 threads of a channel, pairwise
-    __syncthreads();
-    float* s = reinterpret_cast<float*>(smem);
-    if (threadIdx.x < 256) s[threadIdx.x] = bias;
-    __syncthreads();
-    if (threadIdx.x < 16) {
-      float u[16];
-      for (int k = 0; k < 16; ++k) u[k] = s[16 * k + threadIdx.x];
-      for (int o = 8; o; o >>= 1)
-        for (int k = 0; k < o; ++k) u[k] += u[k + o];
-      const float t = u[0];
-      if (partials)
-        out[27 * 256 + threadIdx.x] = t;
-      else
-        atomicAdd(&db[threadIdx.x], t);
-    }
-  }
 }
 
 // dw[i] += sum_b partials[b][i], db likewise, in the order of
@@ -990,29 +1071,34 @@ extern "C" int si_nn_conv3d_wgrad(const void* x, const void* dy, float* dw, floa
   }
   if (fast) {
     const int xchunks = (W + 63) / 64;
-    const int64_t rows = (int64_t)N * D * H * xchunks;
-    const bool short_rows = dil <= kWgMaxDil;
-    // wgrad16_rows_kernel's blocks write the bias sums behind their weight sums:
-    // as many blocks as the buffer holds
-    int64_t want = (int64_t)sm_count() * 8;
-    if (partials && short_rows) want = std::min(want, (int64_t)(need / (kWgOut * sizeof(float))));
-    const int64_t per = (rows + want - 1) / want;
-    const int64_t blocks = (rows + per - 1) / per;
-    if (short_rows) {
+    const int64_t columns = (int64_t)N * D * xchunks * dil, nt = (H + dil - 1) / dil;
+    const int64_t want = (int64_t)sm_count() * 8;
+    // staged rows hold a dilation up to kWgMaxDil, and rows are counted in 32 bits
+    if (dil <= kWgMaxDil && columns * nt < (int64_t)1 << 31) {
       static std::atomic<bool> set[64];
       int dev = 0;
       if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) dev = 0;
       if (!set[dev].load(std::memory_order_acquire)) {
-        if (cudaFuncSetAttribute(wgrad16_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kWgSmem) !=
+        if (cudaFuncSetAttribute(wgrad16_columns_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kWgSmem) !=
             cudaSuccess)
           return check_launch("si_nn_conv3d_wgrad (shared memory)");
         set[dev].store(true, std::memory_order_release);
       }
-      wgrad16_rows_kernel<<<(unsigned)blocks, kWgWarps * 32, kWgSmem, st>>>(xb, db16, dw, db, partials, g, dil, xchunks,
-                                                                           per);
-      if (partials) reduce_wgrad_kernel<<<(kWgOut + 31) / 32, 1024, 0, st>>>(partials, (int)blocks, dw, db);
+      // units: as many sums per weight as 8 blocks per SM had (fewer, longer sums are
+      // less accurate), and no more than the buffer holds
+      int64_t units = std::min(want, columns * nt);
+      if (partials) units = std::min(units, (int64_t)(need / (kWgOut * sizeof(float))));
+      const int64_t groups = (int64_t)sm_count() * kWgGroups;
+      const int per_group = (int)((units + groups - 1) / groups);
+      const int64_t ctas = (units + (int64_t)per_group * kWgGroups - 1) / ((int64_t)per_group * kWgGroups);
+      const WgGeom wg{N, D, H, W, dil, xchunks, (int)nt, (unsigned)(columns * nt), (unsigned)units};
+      wgrad16_columns_kernel<<<(unsigned)ctas, kWgGroups * 96, kWgSmem, st>>>(xb, db16, dw, db, partials, wg, per_group);
+      if (partials) reduce_wgrad_kernel<<<(kWgOut + 31) / 32, 1024, 0, st>>>(partials, (int)units, dw, db);
       return check_launch("si_nn_conv3d_wgrad");
     }
+    const int64_t rows = (int64_t)N * D * H * xchunks;
+    const int64_t per = (rows + want - 1) / want;
+    const int64_t blocks = (rows + per - 1) / per;
     wgrad16_kernel<<<(unsigned)blocks, 128, 0, st>>>(xb, db16, dw, partials, g, dil, xchunks, per);
     if (partials)
       reduce_partials_kernel<<<27 * 256 / 8, 256, 0, st>>>(partials, (int)blocks, 27 * 256, dw);
