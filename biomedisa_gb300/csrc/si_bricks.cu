@@ -1078,7 +1078,8 @@ extern "C" int si_walk_sorted(const void* packed, int work_is_float, int Zc, int
   if ((uint64_t)Zc * Yc * Xc > 0xFFFFFFFFull) return set_error(SI_ERR_LIMIT, "si_walk_sorted: volume above 2^32");
   if (nbrw < 0 || sorw < 0 || (uint64_t)nbrw * (uint64_t)sorw >= (1ull << 24))
     return set_error(SI_ERR_LIMIT, "si_walk_sorted: nbrw*sorw must be below 2^24");
-  if (sweep_steps <= 0) sweep_steps = default_sweep_steps(sorw);
+  const bool default_steps = sweep_steps <= 0;
+  if (default_steps) sweep_steps = default_sweep_steps(sorw);
   if (sort_edge <= 0) sort_edge = kSortEdge;
   if (sort_edge > 1024) return set_error(SI_ERR_ARG, "si_walk_sorted: sort_edge above 1024");
   cudaStream_t st = as_stream(stream);
@@ -1113,6 +1114,10 @@ extern "C" int si_walk_sorted(const void* packed, int work_is_float, int Zc, int
   const uint64_t nbatch = std::max<uint64_t>(1, (walks + per_range / 2) / per_range);
   // walkers per thread: mode 0 -> 1, 1 -> 2, 2 -> 3, 3 -> 4
   const int mode = g_sweep_pairs.load(std::memory_order_relaxed);
+  // walks of which the SMs hold one per thread. A sweep of so few is bound by its
+  // launches and tail as well: twice the steps, 3.39 and 3.21 ms on 40x36x33.
+  const uint64_t resident = (uint64_t)sms * 768;
+  if (default_steps && sorw >= kLongWalk && walks <= resident) sweep_steps *= 2;
   const uint32_t limit = round_limit();
   const bool device_loop = g_device_loop.load(std::memory_order_relaxed) != 0;
   const ScanArgs a{w.counts, nbt, w.offsets, w.ctrs, limit, 0, {}};
@@ -1132,11 +1137,14 @@ extern "C" int si_walk_sorted(const void* packed, int work_is_float, int Zc, int
     // those running at any moment share a compact part of the volume. (A grid of
     // 8 CTAs per SM that strides over the walkers: 419x492x462 915 ms, this one
     // 857 ms; 176x224x208 with labels on all axes 370 and 332 ms.) Walks that
-    // do not fill the SMs once go out in small CTAs, spread more evenly:
-    // 40x36x33, 95 thousand walks, 4.5 and 4.2 ms.
-    const uint64_t per = (uint64_t)mode + 1;
-    const bool few = mode == 1 && n0 <= (uint64_t)sms * 2 * 768;
-    const int tpb = few ? 64 : mode == 3 ? 128 : mode == 1 && work_is_float ? kFloatThreads : 256;
+    // do not fill the SMs once go out in small CTAs, spread more evenly; where a
+    // thread for each is resident at once, each gets one, as two in a thread wait
+    // for the slower of their loads: 40x36x33, 95 thousand walks, pairs in CTAs of
+    // 256 4.5 ms, of 64 4.2 ms (3.78 with the later sweeps), single 3.39 ms.
+    const bool single = mode == 1 && n0 <= resident;
+    const bool few = mode == 1 && !single && n0 <= 2 * resident;
+    const uint64_t per = single ? 1u : (uint64_t)mode + 1;
+    const int tpb = few ? 64 : mode == 3 || single ? 128 : mode == 1 && work_is_float ? kFloatThreads : 256;
     const uint32_t blocks = (uint32_t)(((n0 + per - 1) / per + tpb - 1) / tpb);
     const uint32_t sort_blocks = (uint32_t)std::min<uint64_t>(gb, (n0 + 255) / 256);
     auto sweep = [&](cudaStream_t s, uint4* states) {
@@ -1147,6 +1155,8 @@ extern "C" int si_walk_sorted(const void* packed, int work_is_float, int Zc, int
       SI_SWEEP((sweep_multi_kernel<F, 4, 128, 3>));    \
     else if (mode == 2)                                \
       SI_SWEEP((sweep_multi_kernel<F, 3, 256, 2>));    \
+    else if (single)                                   \
+      SI_SWEEP((sweep_multi_kernel<F, 1, 128, 6>));    \
     else if (few)                                      \
       SI_SWEEP((sweep_multi_kernel<F, 2, 64, F ? 9 : 12>)); \
     else if (mode == 1)                                \

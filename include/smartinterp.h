@@ -218,7 +218,8 @@ int si_walk_sorted_scratch(int Zc, int Yc, int Xc, uint64_t max_walks, int nol,
 /* Sorted-sweep walker: the same walk and the same uint32 hit maps as si_walk
  * over packed records (si_pack_neighbours), run as sweeps in which every live
  * walker advances min(sweep_steps, steps left) steps (default when <= 0: 128
- * for walks of at least 1000 steps, else 32);
+ * for walks of at least 1000 steps, 256 for those where the device holds a
+ * thread for each, else 32);
  * between sweeps the walkers are counting-sorted by (label slot, brick of
  * sort_edge^3 voxels; default 6 when <= 0),
  * so concurrently running walkers share a compact, cache-resident part of

@@ -120,3 +120,15 @@ def test_batch_of_many_volumes(cuda):
     for img, lab, g in zip(imgs, labs, got):
         one = smart_interpolation(img, lab, walker="packed", **kw)
         assert np.array_equal(g["hits"], one["hits"])
+
+
+@pytest.mark.parametrize("nbrw", [3, 5, 7], ids=["105k", "174k", "244k"])
+@pytest.mark.parametrize("dtype", [np.uint8, np.float32], ids=["u8", "f32"])
+def test_one_walk_or_two_per_thread(nbrw, dtype, cuda):
+    """Walks on both sides of one and two per resident thread (117 and 233
+    thousand on 152 SMs), with more steps than the longest default sweep."""
+    img, lab = _volume((21, 60, 58), 11, 2)  # 11 slices, 35 thousand seeds
+    kw = dict(nbrw=nbrw, sorw=1003 if nbrw == 3 else 70, return_hits=True)
+    exp = O.smart_interpolation(img.astype(dtype), lab, key=3, **kw)
+    got = smart_interpolation(img.astype(dtype), lab, rng_seed=3, **kw)
+    assert np.array_equal(got["hits"], exp["hits"])
