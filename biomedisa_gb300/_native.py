@@ -21,6 +21,7 @@ _c_float = ctypes.c_float
 # name -> argtypes (all return int status unless noted)
 _SIGNATURES = {
     "si_label_histogram": [_c_void_p, _c_int, _c_u64, _c_void_p, _c_void_p],
+    "si_label_agreement": [_c_void_p, _c_int, _c_void_p, _c_u64, _c_void_p, _c_void_p],
     "si_slice_flags": [_c_void_p, _c_int, _c_int, _c_int, _c_int, _c_void_p, _c_int, _c_void_p, _c_void_p, _c_void_p,
                        _c_void_p, _c_void_p],
     "si_image_minmax": [_c_void_p, _c_int, _c_u64, _c_void_p, _c_void_p],
@@ -169,3 +170,13 @@ def call(name: str, *args) -> None:
     if rc != 0:
         msg = L.si_last_error().decode(errors="replace")
         raise NativeError(f"{name} failed ({rc}): {msg}")
+
+
+def stream() -> int:
+    """Handle of the current CUDA stream of the current device. (Through
+    torch.cuda.current_stream() the lookup takes longer than a launch.)"""
+    import torch
+
+    if not torch.cuda.is_initialized():
+        return torch.cuda.current_stream().cuda_stream
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())

@@ -47,6 +47,48 @@ __global__ void __launch_bounds__(256) label_hist_kernel(const T* __restrict__ l
 }
 
 // ---------------------------------------------------------------------------
+// Agreement of a result with the labels it came from: counts[0] += labels > 0,
+// counts[1] += those with a result > 0, counts[2] += those with the result equal
+// to the label. One pass over both volumes, 16 voxels a thread and step where both
+// start at a 16-byte boundary, and one read of the counts by the host. (It was a
+// dozen tensor operations over copies of both volumes with three reads; with the
+// other host work of a call cut as well, 40x36x33 4.59 and 3.6 ms.)
+// ---------------------------------------------------------------------------
+template <typename T>
+__global__ void __launch_bounds__(256) label_agreement_kernel(const T* __restrict__ lab,
+                                                              const uint8_t* __restrict__ res, uint64_t n, uint64_t wide,
+                                                              unsigned long long* __restrict__ counts) {
+  uint32_t c[3] = {0u, 0u, 0u};
+  auto count = [&](int v, int r) {
+    c[0] += v > 0;
+    c[1] += v > 0 && r > 0;
+    c[2] += v > 0 && r == v;
+  };
+  const uint64_t at = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x, stride = (uint64_t)gridDim.x * blockDim.x;
+  for (uint64_t i = at; i < wide; i += stride) {
+    union {
+      uint4 q[sizeof(T)];
+      T v[16];
+    } l;
+    union {
+      uint4 q;
+      uint8_t v[16];
+    } r;
+    r.q = reinterpret_cast<const uint4*>(res)[i];
+#pragma unroll
+    for (int k = 0; k < (int)sizeof(T); ++k) l.q[k] = reinterpret_cast<const uint4*>(lab)[i * sizeof(T) + k];
+#pragma unroll
+    for (int k = 0; k < 16; ++k) count((int)l.v[k], (int)r.v[k]);
+  }
+  for (uint64_t i = wide * 16 + at; i < n; i += stride) count((int)lab[i], (int)res[i]);
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    const uint32_t s = __reduce_add_sync(0xffffffffu, c[k]);
+    if ((threadIdx.x & 31) == 0 && s) atomicAdd(&counts[k], (unsigned long long)s);
+  }
+}
+
+// ---------------------------------------------------------------------------
 // Labelled-slice flags and bounding box (padded coordinates).
 // nz(v): value nonzero after pre-processing (negative -> nonzero, > 255 -> 0).
 // All-axis test for a slice with in-slice rows r and columns c
@@ -302,6 +344,30 @@ extern "C" int si_label_histogram(const void* labels, int dtype, uint64_t n, uns
       return set_error(SI_ERR_ARG, "si_label_histogram: unsupported label dtype %d", dtype);
   }
   return check_launch("si_label_histogram");
+}
+
+extern "C" int si_label_agreement(const void* labels, int dtype, const uint8_t* result, uint64_t n,
+                                  unsigned long long* counts, void* stream) {
+  clear_error();
+  if (!labels || !result || !counts) return set_error(SI_ERR_ARG, "si_label_agreement: null pointer");
+  if (n == 0) return SI_OK;
+  const uint64_t wide = ((uintptr_t)labels | (uintptr_t)result) % 16 ? 0 : n / 16;
+  const int block = 256, grid = grid_for(wide ? wide : n, block);
+  cudaStream_t st = as_stream(stream);
+  switch (dtype) {
+    case SI_U8:
+      label_agreement_kernel<<<grid, block, 0, st>>>(static_cast<const uint8_t*>(labels), result, n, wide, counts);
+      break;
+    case SI_I16:
+      label_agreement_kernel<<<grid, block, 0, st>>>(static_cast<const int16_t*>(labels), result, n, wide, counts);
+      break;
+    case SI_I32:
+      label_agreement_kernel<<<grid, block, 0, st>>>(static_cast<const int32_t*>(labels), result, n, wide, counts);
+      break;
+    default:
+      return set_error(SI_ERR_ARG, "si_label_agreement: unsupported label dtype %d", dtype);
+  }
+  return check_launch("si_label_agreement");
 }
 
 extern "C" int si_slice_flags(const void* labels, int dtype, int Z0, int Y0, int X0, const uint8_t* nz_lut,

@@ -84,7 +84,7 @@ def smooth_check():
 
 
 def _stream() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    return nat.stream()
 
 
 def _ptr(t: torch.Tensor | None) -> int | None:
@@ -176,15 +176,12 @@ def plan_labels(hist: np.ndarray, only: str = "all", ignore: str = "none") -> La
             if k in all_labels:
                 all_labels.remove(k)
     all_labels = np.asarray(all_labels, np.int64)
-    slot_of = {int(v): i for i, v in enumerate(all_labels)}
-    nz_lut = np.zeros(256, np.uint8)
-    slot_lut = np.full(256, -1, np.int16)
-    for v in range(256):
-        eff = 0 if (v in removed and v != 0) else v
-        if v in removed and v == 0:
-            eff = 0
-        nz_lut[v] = 1 if (eff != 0 and v not in removed) else 0
-        slot_lut[v] = slot_of.get(eff, -1)
+    eff = np.arange(256)  # removed labels count as background
+    eff[list(removed)] = 0
+    nz_lut = (eff != 0).astype(np.uint8)
+    slot_of = np.full(256, -1, np.int16)
+    slot_of[all_labels] = np.arange(len(all_labels))
+    slot_lut = slot_of[eff]
     return LabelPlan(all_labels, nz_lut, slot_lut, bool(hist[256] > 0), bool(hist[257] > 0))
 
 
@@ -302,17 +299,20 @@ class DeviceJob:
         if self.lplan.nol < 2:
             return "No labeled slices found."
         Z0, Y0, X0 = self.shape0
-        fz = torch.zeros(Z0 + 2, dtype=torch.uint8, device=self.dev)
-        fy = torch.zeros(Y0 + 2, dtype=torch.uint8, device=self.dev)
-        fx = torch.zeros(X0 + 2, dtype=torch.uint8, device=self.dev)
+        # one buffer up and down: bounding box, label table, flags of the three axes
+        ends = np.cumsum([24, 256, Z0 + 2, Y0 + 2, X0 + 2])
+        host = np.zeros(ends[-1], np.uint8)
         imax = np.iinfo(np.int32).max
-        bbox = torch.tensor([imax, -1, imax, -1, imax, -1], dtype=torch.int32, device=self.dev)
-        nz = torch.from_numpy(self.lplan.nz_lut).to(self.dev)
-        nat.call("si_slice_flags", _ptr(self.lab), self.lab_code, Z0, Y0, X0, _ptr(nz), int(self.allaxis), _ptr(fz),
-                 _ptr(fy), _ptr(fx), _ptr(bbox), _stream())
+        host[:24].view(np.int32)[:] = [imax, -1, imax, -1, imax, -1]
+        host[24:280] = self.lplan.nz_lut
+        buf = torch.from_numpy(host).to(self.dev)
+        at = [_ptr(buf)] + [_ptr(buf) + int(e) for e in ends[:4]]
+        nat.call("si_slice_flags", _ptr(self.lab), self.lab_code, Z0, Y0, X0, at[1], int(self.allaxis), *at[2:],
+                 at[0], _stream())
         self.launches += 1
-        flags = [fz.cpu().numpy(), fy.cpu().numpy(), fx.cpu().numpy()]
-        bb = bbox.cpu().numpy()
+        host = buf.cpu().numpy()
+        flags = [host[a:b] for a, b in zip(ends[1:4], ends[2:])]
+        bb = host[:24].view(np.int32)
         if bb[1] < 0:
             return "No labeled slices found."
         if self.allaxis:
@@ -349,15 +349,18 @@ class DeviceJob:
         cap = max(cp.seed_capacity(slice_list), 1)
         self.seed_capacity = cap
         self.seeds = torch.empty(cap * SEED_RECORD_BYTES, dtype=torch.uint8, device=self.dev)
-        self.n_seeds = torch.zeros(1, dtype=torch.int32, device=self.dev)
         n_sl = len(slice_list)
-        self.row_counts = torch.zeros(max(n_sl * cp.max_rows + 1, 1), dtype=torch.int32, device=self.dev)
-        sl = torch.from_numpy(np.ascontiguousarray(slice_list.reshape(-1))).to(self.dev) if n_sl else \
-            torch.zeros(2, dtype=torch.int32, device=self.dev)
-        slot_lut = torch.from_numpy(self.lplan.slot_lut).to(self.dev)
-        slot_label = np.zeros(256, np.uint8)
-        slot_label[: self.lplan.nol] = self.lplan.all_labels.astype(np.uint8)
-        self.slot_label = torch.from_numpy(slot_label).to(self.dev)
+        rows = max(n_sl * cp.max_rows + 1, 1)
+        counts = torch.zeros((rows + 3) // 4 * 4 + 1, dtype=torch.int32, device=self.dev)
+        self.row_counts, self.n_seeds = counts[:rows], counts[-1:]
+        # one upload: slots of the labels, labels of the slots, slice list
+        tables = np.zeros(768 + 8 * max(n_sl, 1), np.uint8)
+        tables[:512].view(np.int16)[:] = self.lplan.slot_lut
+        tables[512:512 + self.lplan.nol] = self.lplan.all_labels.astype(np.uint8)
+        tables[768:].view(np.int32)[:2 * n_sl] = slice_list.reshape(-1)
+        dtab = torch.from_numpy(tables).to(self.dev)
+        slot_lut, self.slot_label = dtab[:512].view(torch.int16), dtab[512:768]
+        sl = dtab[768:].view(torch.int32)
         if self.seeding == "large":
             self._large_seeds(slice_list, sl, slot_lut)
         else:
@@ -748,11 +751,10 @@ def smart_interpolation(data, labelData, nbrw=10, sorw=4000, acwe=False, acwe_al
                       (cp.Zc, cp.Yc, cp.Xc))
         res["acwe"], res["refined"] = acwe_results(frame, res["regular"], acwe_alpha, acwe_smooth, acwe_steps)
     # sanity check of rw_small.py:203-211 (Dice of the input slices vs result)
-    mask = lab > 0
-    gt = lab.to(torch.int32)
-    rr = res["regular"].to(torch.int32) * mask
-    den = float((gt > 0).sum() + (rr > 0).sum())
-    dice = 2.0 * float(torch.logical_and(gt == rr, (gt + rr) > 0).sum()) / den if den else 1.0
+    counts = torch.zeros(3, dtype=torch.int64, device=lab.device)
+    nat.call("si_label_agreement", _ptr(lab), job.lab_code, _ptr(res["regular"]), lab.numel(), _ptr(counts), _stream())
+    labelled, kept, equal = counts.tolist()
+    dice = 2.0 * equal / (labelled + kept) if labelled + kept else 1.0
     if dice < 0.3:
         print('Warning: Bad result! Use "--allaxis" if you labeled axes other than the xy-plane.')
     if return_device:

@@ -12,7 +12,7 @@ from . import _native as nat
 
 
 def _stream() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    return nat.stream()
 
 
 def _scratch(shape, device):

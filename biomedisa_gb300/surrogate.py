@@ -35,7 +35,7 @@ MAX_SLOTS = 13  # one-hot slot channels of the input
 
 
 def _stream() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    return nat.stream()
 
 
 def _p(t):
@@ -296,17 +296,14 @@ def slice_table(Zc: int, zs) -> np.ndarray:
     zs = np.asarray(sorted(set(int(v) for v in zs)), np.int64)
     out = np.zeros((Zc, 4), np.float32)
     out[:, 0] = slice_distance(Zc, zs)
-    for z in range(Zc):
-        k = np.searchsorted(zs, z, side="right")
-        lo = int(zs[k - 1]) if k > 0 else -1
-        hi = int(zs[k]) if k < zs.size else -1
-        if lo == z:
-            hi = -1
-        if lo >= 0 and hi >= 0:
-            w = (hi - z) / (hi - lo)
-        else:
-            w = 1.0 if lo >= 0 else 0.0
-        out[z] = (out[z, 0], lo, hi, w)
+    z = np.arange(Zc)
+    k = np.searchsorted(zs, z, side="right")
+    ends = np.concatenate([[-1], zs, [-1]])  # below the first, above the last: none
+    lo, hi = ends[k], ends[k + 1]
+    hi = np.where(lo == z, -1, hi)
+    both = (lo >= 0) & (hi >= 0)
+    out[:, 1], out[:, 2] = lo, hi
+    out[:, 3] = np.where(both, (hi - z) / np.where(both, hi - lo, 1), lo >= 0)
     return out
 
 

@@ -81,6 +81,13 @@ const char* si_last_error(void);
 int si_label_histogram(const void* labels, int dtype, uint64_t n,
                        unsigned long long* hist, void* stream);
 
+/* counts[0] += voxels with a label above 0, counts[1] += those of them with a
+ * result above 0, counts[2] += those with the result equal to the label (the
+ * Dice check of a result on its input slices, rw_small.py:203-211). dtype:
+ * SI_U8, SI_I16 or SI_I32; the caller zeroes counts[3]. */
+int si_label_agreement(const void* labels, int dtype, const uint8_t* result,
+                       uint64_t n, unsigned long long* counts, void* stream);
+
 /* Labelled-slice flags and bounding box of nonzero labels on the zero-padded
  * frame (dims Z0+2, Y0+2, X0+2) without materialising the pad.
  * nz_lut[v] (v = 0..255) is 1 iff value v is nonzero after pre-processing;
