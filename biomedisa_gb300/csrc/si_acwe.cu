@@ -19,6 +19,7 @@
 #include <cmath>
 #include <cstdint>
 
+#include "si_common.cuh"
 #include "si_internal.h"
 
 namespace si {
@@ -255,11 +256,20 @@ __global__ void __launch_bounds__(256) acwe_pack_kernel(const uint8_t* __restric
     for (int w0 = 0; w0 < W; w0 += 32) {
       uint32_t mine = 0;  // lane i keeps word w0 + i
       const int nw = min(32, W - w0);
-      for (int i = 0; i < nw; ++i) {
-        const int x = 32 * (w0 + i) + lane;
-        const bool hit = x < X && row[x] == label;
-        const uint32_t word = __ballot_sync(0xffffffffu, hit);
-        if (lane == i) mine = word;
+      // eight loads in flight (one by one a row waited for each of its loads: 13 us a
+      // pass over 192x256x250 voxels)
+      for (int i = 0; i < nw; i += 8) {
+        int v[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+          const int x = 32 * (w0 + i + k) + lane;
+          v[k] = x < X ? (int)row[x] : -1;
+        }
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+          const uint32_t word = __ballot_sync(0xffffffffu, v[k] == label);
+          if (lane == i + k) mine = word;
+        }
       }
       if (lane < nw) mrow[w0 + lane] = mine;
     }
@@ -274,9 +284,8 @@ __global__ void __launch_bounds__(256) acwe_morph_bits_kernel(uint8_t* __restric
   const int64_t n = (int64_t)Z * Y * W;
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
-    const int w = (int)(i % W);
-    const int64_t zy = i / W;
-    const int y = (int)(zy % Y), z = (int)(zy / Y);
+    int z, y, w;
+    voxel_of((uint64_t)i, Y, W, z, y, w);
     const uint32_t m = Min[i];
     if (z < 1 || z > Z - 2 || y < 1 || y > Y - 2) {
       Mout[i] = m;
@@ -424,9 +433,8 @@ __global__ void __launch_bounds__(256) acwe_gather_kernel(const T* __restrict__ 
   const uint64_t n = (uint64_t)cb.cZ * cb.cY * cb.cX;
   const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
   for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
-    const int xc = (int)(i % cb.cX);
-    const uint64_t zy = i / cb.cX;
-    const int yc = (int)(zy % cb.cY), zc = (int)(zy / cb.cY);
+    int zc, yc, xc;
+    voxel_of(i, cb.cY, cb.cX, zc, yc, xc);
     const int pz = cb.cz0 + zc, py = cb.cy0 + yc, px = cb.cx0 + xc;
     uint8_t d = 0, l = 0;
     if (pz >= 1 && pz <= f.Z && py >= 1 && py <= f.Y && px >= 1 && px <= f.X) {
@@ -495,9 +503,8 @@ __global__ void __launch_bounds__(256) acwe_scatter_kernel(const uint8_t* __rest
   const uint64_t n = (uint64_t)Z * Y * X;
   const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
   for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
-    const int x = (int)(i % X);
-    const uint64_t zy = i / X;
-    const int y = (int)(zy % Y), z = (int)(zy / Y);
+    int z, y, x;
+    voxel_of(i, Y, X, z, y, x);
     const int a = z + 1 - cb.cz0, b = y + 1 - cb.cy0, c = x + 1 - cb.cx0;
     uint8_t v = 0;
     if ((unsigned)a < (unsigned)cb.cZ && (unsigned)b < (unsigned)cb.cY && (unsigned)c < (unsigned)cb.cX)
@@ -690,9 +697,8 @@ __global__ void __launch_bounds__(256) acwe_refine_apply_kernel(const float* __r
   const uint64_t n = (uint64_t)Z * Y * X;
   const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
   for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
-    const int x = (int)(i % X);
-    const uint64_t zy = i / X;
-    const int y = (int)(zy % Y), z = (int)(zy / Y);
+    int z, y, x;
+    voxel_of(i, Y, X, z, y, x);
     const int a = z + 1 - cb.cz0, b = y + 1 - cb.cy0, c = x + 1 - cb.cx0;
     uint8_t v = 0;
     if ((unsigned)a < (unsigned)cb.cZ && (unsigned)b < (unsigned)cb.cY && (unsigned)c < (unsigned)cb.cX) {

@@ -488,4 +488,20 @@ __device__ __forceinline__ void walk_steps_multi(const void* __restrict__ packed
   }
 }
 
+// z, y and x of voxel i of rows of X and planes of Y rows. Indices below 2^32
+// take 32-bit divisions (a 64-bit one is some five times as many instructions).
+__device__ __forceinline__ void voxel_of(uint64_t i, int Y, int X, int& z, int& y, int& x) {
+  if ((i >> 32) == 0u) {
+    const uint32_t v = (uint32_t)i, zy = v / (uint32_t)X;
+    x = (int)(v - zy * (uint32_t)X);
+    z = (int)(zy / (uint32_t)Y);
+    y = (int)(zy - (uint32_t)z * (uint32_t)Y);
+  } else {
+    const uint64_t zy = i / (uint32_t)X;
+    x = (int)(i - zy * (uint32_t)X);
+    z = (int)(zy / (uint32_t)Y);
+    y = (int)(zy - (uint64_t)z * (uint32_t)Y);
+  }
+}
+
 }  // namespace si

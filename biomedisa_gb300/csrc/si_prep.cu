@@ -106,7 +106,9 @@ struct LabelView {
   // nonzero test at ORIGINAL coordinates, zero outside.
   __device__ __forceinline__ bool nz(int z, int y, int x) const {
     if ((unsigned)z >= (unsigned)Z0 || (unsigned)y >= (unsigned)Y0 || (unsigned)x >= (unsigned)X0) return false;
-    const int v = load_label(lab, ((uint64_t)z * Y0 + y) * X0 + x);
+    return set(load_label(lab, ((uint64_t)z * Y0 + y) * X0 + x));
+  }
+  __device__ __forceinline__ bool set(int v) const {
     if (v < 0) return neg_nz;
     if (v > 255) return false;
     return nz_lut[v] != 0;
@@ -138,29 +140,37 @@ __global__ void __launch_bounds__(256) slice_flags_kernel(const T* __restrict__ 
   LabelView<T> lv{lab, lut, Z0, Y0, X0, allaxis != 2};
   int bmin[3] = {INT_MAX, INT_MAX, INT_MAX};
   int bmax[3] = {-1, -1, -1};
-  const uint64_t n = (uint64_t)Z0 * Y0 * X0;
-  const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-  for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
-    const int x = (int)(i % X0);
-    const uint64_t zy = i / X0;
-    const int y = (int)(zy % Y0);
-    const int z = (int)(zy / Y0);
-    if (!lv.nz(z, y, x)) continue;
-    // padded coordinates
-    const int pz = z + 1, py = y + 1, px = x + 1;
-    bmin[0] = min(bmin[0], pz); bmax[0] = max(bmax[0], pz);
-    bmin[1] = min(bmin[1], py); bmax[1] = max(bmax[1], py);
-    bmin[2] = min(bmin[2], px); bmax[2] = max(bmax[2], px);
-    if (!allaxis) {
-      fz[pz] = 1;
-    } else {
-      // axis 0: slice at fixed z, rows along y, columns along x
-      if (!fz[pz] && survives(lv, z, y, x, 0, 1, 0, 0, 0, 1)) fz[pz] = 1;
-      // axis 1: slice at fixed y, rows along z, columns along x
-      if (!fy[py] && survives(lv, z, y, x, 1, 0, 0, 0, 0, 1)) fy[py] = 1;
-      // axis 2: slice at fixed x, rows along z, columns along y
-      if (!fx[px] && survives(lv, z, y, x, 1, 0, 0, 0, 1, 0)) fx[px] = 1;
+  // a warp per x-row, four loads in flight a lane (a thread per voxel spent its
+  // time on the divisions of a 64-bit index: 88 us on 192x256x250 uint8)
+  const uint64_t rows = (uint64_t)Z0 * Y0;
+  const uint64_t stride = (uint64_t)gridDim.x * (blockDim.x >> 5);
+  const int lane = threadIdx.x & 31;
+  for (uint64_t row = (uint64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); row < rows; row += stride) {
+    const int z = (int)(row / (unsigned)Y0), y = (int)(row - (uint64_t)z * Y0);
+    const int pz = z + 1, py = y + 1;  // padded coordinates
+    const T* at = lab + row * X0;
+    for (int x0 = lane; x0 < X0; x0 += 128) {
+      int v[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) v[k] = x0 + 32 * k < X0 ? load_label(at, (uint64_t)(x0 + 32 * k)) : 256;
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const int x = x0 + 32 * k, px = x + 1;
+        if (!lv.set(v[k])) continue;
+        bmin[0] = min(bmin[0], pz); bmax[0] = max(bmax[0], pz);
+        bmin[1] = min(bmin[1], py); bmax[1] = max(bmax[1], py);
+        bmin[2] = min(bmin[2], px); bmax[2] = max(bmax[2], px);
+        if (allaxis) {
+          // axis 0: slice at fixed z, rows along y, columns along x
+          if (!fz[pz] && survives(lv, z, y, x, 0, 1, 0, 0, 0, 1)) fz[pz] = 1;
+          // axis 1: slice at fixed y, rows along z, columns along x
+          if (!fy[py] && survives(lv, z, y, x, 1, 0, 0, 0, 0, 1)) fy[py] = 1;
+          // axis 2: slice at fixed x, rows along z, columns along y
+          if (!fx[px] && survives(lv, z, y, x, 1, 0, 0, 0, 1, 0)) fx[px] = 1;
+        }
+      }
     }
+    if (!allaxis && bmax[0] == pz) fz[pz] = 1;
   }
 #pragma unroll
   for (int a = 0; a < 3; ++a) {
@@ -378,8 +388,7 @@ extern "C" int si_slice_flags(const void* labels, int dtype, int Z0, int Y0, int
   if (allaxis < 0 || allaxis > 2) return set_error(SI_ERR_ARG, "si_slice_flags: allaxis must be 0, 1 or 2");
   if (allaxis && (!flags_y || !flags_x)) return set_error(SI_ERR_ARG, "si_slice_flags: allaxis needs flags_y/flags_x");
   if (Z0 <= 0 || Y0 <= 0 || X0 <= 0) return set_error(SI_ERR_ARG, "si_slice_flags: bad dims");
-  const uint64_t n = (uint64_t)Z0 * Y0 * X0;
-  const int block = 256, grid = grid_for(n, block);
+  const int block = 256, grid = grid_for((uint64_t)Z0 * Y0, block / 32);
   cudaStream_t st = as_stream(stream);
   switch (dtype) {
     case SI_U8:
