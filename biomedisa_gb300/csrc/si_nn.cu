@@ -1034,7 +1034,17 @@ extern "C" int si_nn_conv16_tc(const void* x, const void* w, const float* bias, 
   if (N < 1 || D < 1 || H < 1 || W < 1) return set_error(SI_ERR_ARG, "si_nn_conv16_tc: bad shape");
   if (((uintptr_t)x | (uintptr_t)w | (uintptr_t)y | (uintptr_t)residual) % 16)
     return set_error(SI_ERR_ARG, "si_nn_conv16_tc: tensors must be 16-byte aligned");
-  return conv16_umma(x, w, bias, residual, y, N, D, H, W, dil, relu, out_f32, as_stream(stream));
+  return conv16_umma(x, w, bias, residual, nullptr, y, N, D, H, W, dil, relu, out_f32, as_stream(stream));
+}
+
+extern "C" int si_nn_conv16_tc_masked(const void* x, const void* w, const void* residual, const void* mask, void* y,
+                                      int N, int D, int H, int W, int dil, void* stream) {
+  clear_error();
+  if (!x || !w || !mask || !y) return set_error(SI_ERR_ARG, "si_nn_conv16_tc_masked: null pointer");
+  if (N < 1 || D < 1 || H < 1 || W < 1) return set_error(SI_ERR_ARG, "si_nn_conv16_tc_masked: bad shape");
+  if (((uintptr_t)x | (uintptr_t)w | (uintptr_t)y | (uintptr_t)residual | (uintptr_t)mask) % 16)
+    return set_error(SI_ERR_ARG, "si_nn_conv16_tc_masked: tensors must be 16-byte aligned");
+  return conv16_umma(x, w, nullptr, residual, mask, y, N, D, H, W, dil, 0, 0, as_stream(stream));
 }
 
 extern "C" int si_nn_wgrad_partial_bytes(int N, int D, int H, int W, int cin, int cout, uint64_t* bytes) {

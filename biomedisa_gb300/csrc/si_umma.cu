@@ -351,7 +351,7 @@ template <bool kOutF32, bool kPacked>
 __global__ void __launch_bounds__(kThreads, kCtasPerSm)
     conv16_umma_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUtensorMap rmap,
                        const __nv_bfloat16* __restrict__ w, const float* __restrict__ bias, int has_res,
-                       void* __restrict__ y_out, const __grid_constant__ UmmaGeom g, int relu, int wide,
+                       const __nv_bfloat16* __restrict__ mask, void* __restrict__ y_out, const __grid_constant__ UmmaGeom g, int relu, int wide,
                        uint32_t wait_lim) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
@@ -564,6 +564,14 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm)
     Ring<kResSlots> sr;
     while (t.live) {
       const int p = t.p;
+      const int x = t.x0 + mx, z = t.z + line;
+      const bool out = t.i >= 2 && x < g.W && line < g.lines && z < g.D;  // output row j = i - 2
+      const long long r = (((long long)t.n * g.D + z) * g.H + (t.y(g) - dil)) * g.W + x;
+      uint4 mq[2];
+      if (mask && out) {  // arrives while the MMAs are waited for
+        mq[0] = __ldg(reinterpret_cast<const uint4*>(mask + r * 16));
+        mq[1] = __ldg(reinterpret_cast<const uint4*>(mask + r * 16) + 1);
+      }
       bool ok = !s_fail && mbar_wait_fast(&done_bar[p], t.ph, wait_lim);
       if (has_res) ok = ok && mbar_wait_fast(&rfull_bar[sr.idx], sr.ph, wait_lim);
       if (!__all_sync(0xffffffffu, ok)) {
@@ -573,7 +581,7 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm)
       tmem_fence_after();
       const uint32_t ta = tmem + lane_base + (uint32_t)(16 * p);
       uint32_t v[16];
-      if (t.i >= 2) {  // output row j = i - 2
+      if (t.i >= 2) {
         tmem_ld16(ta, v);
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
       }
@@ -593,46 +601,51 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm)
         mbar_arrive(&free_bar[p]);
         if (has_res) mbar_arrive(&rfree_bar[sr.idx]);
       }
-      if (t.i >= 2) {
+      if (out) {
         float u[16];
 #pragma unroll
-        for (int e = 0; e < 16; ++e) u[e] = __uint_as_float(v[e]);
-        const int x = t.x0 + mx, z = t.z + line;
-        if (x < g.W && line < g.lines && z < g.D) {
-          const long long r = (((long long)t.n * g.D + z) * g.H + (t.y(g) - dil)) * g.W + x;
+        for (int e = 0; e < 16; ++e) u[e] = __uint_as_float(v[e]) + s_bias[e];
+        if (has_res) {
 #pragma unroll
-          for (int e = 0; e < 16; ++e) u[e] += s_bias[e];
-          if (has_res) {
+          for (int h = 0; h < 2; ++h) {
+            const uint32_t words[4] = {rq[h].x, rq[h].y, rq[h].z, rq[h].w};
 #pragma unroll
-            for (int h = 0; h < 2; ++h) {
-              const uint32_t words[4] = {rq[h].x, rq[h].y, rq[h].z, rq[h].w};
-#pragma unroll
-              for (int e = 0; e < 4; ++e) {
-                u[h * 8 + 2 * e] += __bfloat162float(__ushort_as_bfloat16((unsigned short)(words[e] & 0xFFFFu)));
-                u[h * 8 + 2 * e + 1] += __bfloat162float(__ushort_as_bfloat16((unsigned short)(words[e] >> 16)));
-              }
+            for (int e = 0; e < 4; ++e) {
+              u[h * 8 + 2 * e] += __uint_as_float(words[e] << 16);
+              u[h * 8 + 2 * e + 1] += __uint_as_float(words[e] & 0xFFFF0000u);
             }
           }
-          if (relu) {
+        }
+        if (relu) {
 #pragma unroll
-            for (int e = 0; e < 16; ++e) u[e] = fmaxf(u[e], 0.0f);
-          }
-          uint32_t pk[8];
-          if (kOutF32) {
+          for (int e = 0; e < 16; ++e) u[e] = fmaxf(u[e], 0.0f);
+        }
+        if (mask) {
 #pragma unroll
-            for (int h = 0; h < 2; ++h) {
+          for (int h = 0; h < 2; ++h) {
+            const uint32_t words[4] = {mq[h].x, mq[h].y, mq[h].z, mq[h].w};
 #pragma unroll
-              for (int e = 0; e < 8; ++e) pk[e] = __float_as_uint(u[8 * h + e]);
-              store32(static_cast<float*>(y_out) + r * 16 + 8 * h, pk, wide);
+            for (int e = 0; e < 4; ++e) {
+              if (!(__uint_as_float(words[e] << 16) > 0.0f)) u[h * 8 + 2 * e] = 0.0f;
+              if (!(__uint_as_float(words[e] & 0xFFFF0000u) > 0.0f)) u[h * 8 + 2 * e + 1] = 0.0f;
             }
-          } else {
-#pragma unroll
-            for (int e = 0; e < 8; ++e) {
-              const __nv_bfloat162 b2 = __floats2bfloat162_rn(u[2 * e], u[2 * e + 1]);
-              pk[e] = *reinterpret_cast<const uint32_t*>(&b2);
-            }
-            store32(static_cast<__nv_bfloat16*>(y_out) + r * 16, pk, wide);
           }
+        }
+        uint32_t pk[8];
+        if (kOutF32) {
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+#pragma unroll
+            for (int e = 0; e < 8; ++e) pk[e] = __float_as_uint(u[8 * h + e]);
+            store32(static_cast<float*>(y_out) + r * 16 + 8 * h, pk, wide);
+          }
+        } else {
+#pragma unroll
+          for (int e = 0; e < 8; ++e) {
+            const __nv_bfloat162 b2 = __floats2bfloat162_rn(u[2 * e], u[2 * e + 1]);
+            pk[e] = *reinterpret_cast<const uint32_t*>(&b2);
+          }
+          store32(static_cast<__nv_bfloat16*>(y_out) + r * 16, pk, wide);
         }
       }
       sr.next();
@@ -663,7 +676,8 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm)
 
 template <bool kOutF32, bool kPacked>
 cudaError_t launch_conv16(const CUtensorMap& map, const CUtensorMap& rmap, const __nv_bfloat16* w, const float* bias,
-                          int has_res, void* y, const UmmaGeom& g, int relu, int wide, int grid, cudaStream_t st) {
+                          int has_res, const __nv_bfloat16* mask, void* y, const UmmaGeom& g, int relu, int wide,
+                          int grid, cudaStream_t st) {
   const auto kernel = conv16_umma_kernel<kOutF32, kPacked>;
   const cudaError_t ae = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
   if (ae != cudaSuccess) return ae;
@@ -677,15 +691,16 @@ cudaError_t launch_conv16(const CUtensorMap& map, const CUtensorMap& rmap, const
   at[0].val.programmaticStreamSerializationAllowed = 1;
   c.attrs = at;
   c.numAttrs = 1;
-  return cudaLaunchKernelEx(&c, kernel, map, rmap, w, bias, has_res, y, g, relu, wide, wait_limit());
+  return cudaLaunchKernelEx(&c, kernel, map, rmap, w, bias, has_res, mask, y, g, relu, wide, wait_limit());
 }
 
 }  // namespace
 
 // 16 -> 16 convolution on the tensor cores (see the file comment). x, w,
-// residual, y 16-byte aligned; dil <= 8. Returns SI_OK or an error code.
-int conv16_umma(const void* x, const void* w, const float* bias, const void* residual, void* y, int N, int D, int H,
-                int W, int dil, int relu, int out_f32, cudaStream_t st) {
+// residual, mask, y 16-byte aligned; dil <= 8. With a mask (bf16, shaped like y)
+// values where it is not above 0 are stored as 0. Returns SI_OK or an error code.
+int conv16_umma(const void* x, const void* w, const float* bias, const void* residual, const void* mask, void* y,
+                int N, int D, int H, int W, int dil, int relu, int out_f32, cudaStream_t st) {
   if (dil < 1 || dil > kMaxDil) return set_error(SI_ERR_ARG, "conv16_umma: dilation must be 1..%d", kMaxDil);
   if ((long long)N * D > 0x7FFFFFFFll) return set_error(SI_ERR_ARG, "conv16_umma: too many z-planes");
   const EncodeTiledFn enc = encode_fn();
@@ -737,7 +752,8 @@ int conv16_umma(const void* x, const void* w, const float* bias, const void* res
   const auto* wb = static_cast<const __nv_bfloat16*>(w);
   const auto launch = out_f32 ? (packed ? launch_conv16<true, true> : launch_conv16<true, false>)
                               : (packed ? launch_conv16<false, true> : launch_conv16<false, false>);
-  const cudaError_t ae = launch(map, rmap, wb, bias, has_res, y, g, relu, wide, (int)grid, st);
+  const cudaError_t ae =
+      launch(map, rmap, wb, bias, has_res, static_cast<const __nv_bfloat16*>(mask), y, g, relu, wide, (int)grid, st);
   if (ae != cudaSuccess) return set_error(SI_ERR_CUDA, "conv16_umma: launch: %s", cudaGetErrorString(ae));
   return check_launch("conv16_umma");
 }

@@ -86,19 +86,26 @@ def conv_fwd(x, conv: Conv, shape, relu, residual=None, out_f32=False, tensor_co
     return y
 
 
-def conv_dgrad(dy, conv: Conv, shape, residual=None, tensor_core=False):
-    """dX = conv(dY, W flipped) (+ residual added in the epilogue)."""
+def conv_dgrad(dy, conv: Conv, shape, residual=None, tensor_core=False, mask=None):
+    """dX = conv(dY, W flipped) (+ residual added in the epilogue), 0 where
+    mask, the output of the ReLU that made X, is not above 0."""
     N, D, H, W = shape
     if conv.wf is None:
         conv.wf = torch.empty_like(conv.wb)
     nat.call("si_nn_flip_weights", _p(conv.wb), _p(conv.wf), conv.cout, conv.cin, _stream())
     dx = torch.empty((N, D, H, W, conv.cin), dtype=BF16, device=dy.device)
     if _tensor_core_ok(conv, tensor_core):
+        if mask is not None:
+            nat.call("si_nn_conv16_tc_masked", _p(dy), _p(conv.wf), _p(residual), _p(mask), _p(dx), N, D, H, W,
+                     conv.dil, _stream())
+            return dx
         nat.call("si_nn_conv16_tc", _p(dy), _p(conv.wf), None, _p(residual), _p(dx), N, D, H, W, conv.dil, 0, 0,
                  _stream())
     else:
         nat.call("si_nn_conv3d_fwd", _p(dy), _p(conv.wf), None, _p(residual), _p(dx), N, D, H, W, conv.cout,
                  conv.cin, conv.dil, 0, 0, _stream())
+    if mask is not None:
+        relu_bwd(dx, mask)
     return dx
 
 
@@ -199,17 +206,16 @@ class SurrogateNet:
         head = self.convs[-1]
         conv_wgrad(acts[-1], dlogits, head, shape)
         tc = self.tensor_core
-        da = conv_dgrad(dlogits, head, shape, tensor_core=tc)
+        # da, dt: gradients of pre-activations (masked where the ReLU gave 0)
+        da = conv_dgrad(dlogits, head, shape, tensor_core=tc, mask=acts[-1])
         for i in reversed(range(len(self.dilations))):
             c1, c2 = self.convs[1 + 2 * i], self.convs[2 + 2 * i]
-            a_in, t, a_out = acts[1 + 2 * i], acts[2 + 2 * i], acts[3 + 2 * i]
-            relu_bwd(da, a_out)                 # g = dL/d(pre-activation of the block output)
+            a_in, t = acts[1 + 2 * i], acts[2 + 2 * i]
             conv_wgrad(t, da, c2, shape)
-            dt = conv_dgrad(da, c2, shape, tensor_core=tc)
-            relu_bwd(dt, t)
+            dt = conv_dgrad(da, c2, shape, tensor_core=tc, mask=t)
             conv_wgrad(a_in, dt, c1, shape)
-            da = conv_dgrad(dt, c1, shape, residual=da, tensor_core=tc)  # conv1^T(dt) + g through the skip
-        relu_bwd(da, acts[1])
+            # conv1^T(dt) + the block's gradient through the skip
+            da = conv_dgrad(dt, c1, shape, residual=da, tensor_core=tc, mask=a_in)
         conv_wgrad(acts[0], da, self.convs[0], shape)
         self._acts = None
 

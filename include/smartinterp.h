@@ -563,11 +563,19 @@ int si_nn_conv3d_fwd(const void* x, const void* w, const float* bias,
  * meets, 16 channels each), K = 16, into a ring of fp32 accumulators in
  * tensor memory; rows staged by TMA. Same results as si_nn_conv3d_fwd up to
  * fp32 accumulation order, and independent of the grid. The default of
- * SurrogateNet for its 16 -> 16 layers (2.4x the mma.sync kernel on large
- * volumes, measured). No counterpart in the reference. */
+ * SurrogateNet for its 16 -> 16 layers (4 to 5 times the mma.sync kernel's rate,
+ * measured). No counterpart in the reference. */
 int si_nn_conv16_tc(const void* x, const void* w, const float* bias,
                     const void* residual, void* y, int N, int D, int H, int W,
                     int dil, int relu, int out_f32, void* stream);
+
+/* The data gradient through a ReLU in one pass: y = conv(x, w) + residual where
+ * mask (bf16, shaped like y; the ReLU's output) is above 0, else 0. residual
+ * nullable; otherwise as si_nn_conv16_tc followed by si_nn_relu_bwd, bit for bit.
+ * No counterpart in the reference. */
+int si_nn_conv16_tc_masked(const void* x, const void* w, const void* residual,
+                           const void* mask, void* y, int N, int D, int H,
+                           int W, int dil, void* stream);
 
 /* Status of the tensor-core convolution kernel (si_nn_conv16_tc) on the
  * current device since the last call:

@@ -160,3 +160,24 @@ def test_weight_gradient_stays_in_its_buffer(shape, cuda):
     assert bool((buf[need.value // 4:] == 7.0).all())
     w, wm, b, bm = _wgrad64(x, dy, 1)
     assert float(((dw.double().view(27, 16, 16) - w).abs() / (wm + 1)).max()) < 1e-5
+
+
+@pytest.mark.parametrize("shape,dil", [((2, 5, 4, 64), 1), ((1, 3, 9, 130), 2), ((1, 4, 5, 40), 8)], ids=str)
+@pytest.mark.parametrize("with_residual", [False, True])
+def test_masked_data_gradient(shape, dil, with_residual, cuda):
+    """Equal to the convolution and the ReLU mask after it, bit for bit."""
+    g = torch.Generator(device="cuda").manual_seed(sum(shape))
+    dy, res, act = (_bf((*shape, 16), g) for _ in range(3))
+    act = torch.relu(act)
+    act[..., 3] = float("nan")
+    act[..., 4] = -0.0
+    net = S.SurrogateNet(dilations=(1,))
+    conv = net.convs[1]
+    conv.dil = dil
+    kw = dict(residual=res if with_residual else None)
+    for tc in (True, False):
+        got = S.conv_dgrad(dy, conv, shape, tensor_core=tc, mask=act, **kw)
+        exp = S.conv_dgrad(dy, conv, shape, tensor_core=tc, **kw)
+        S.relu_bwd(exp, act)
+        assert torch.equal(got, exp) and bool((got[..., 3:5] == 0).all()) and bool((got != 0).any())
+    S.umma_check()
