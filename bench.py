@@ -557,14 +557,15 @@ def run_batch_bench(args, wl):
 
 def launches_since(before, sweeps=0):
     """Kernel launches of libsmartinterp calls made since the `before`
-    snapshot of _native.CALLS (si_walk_sorted: 6 per sweep + 4)."""
+    snapshot of _native.CALLS (si_walk_sorted: a scatter, a sweep and at least
+    one scan kernel per sweep, two before the first)."""
     from biomedisa_gb300 import _native as nat
 
     n = 0
     for k, v in nat.CALLS.items():
         d = v - before.get(k, 0)
         if k == "si_walk_sorted":
-            n += 6 * sweeps + 4 * d
+            n += 3 * sweeps + 2 * d
         else:
             n += MULTI_LAUNCH.get(k, 1) * d
     return n
