@@ -171,17 +171,26 @@ __global__ void __launch_bounds__(256) remap_kernel(uint8_t* __restrict__ out, P
 // outside it do nothing (or write zeros, when their destination may hold
 // older values).
 // ---------------------------------------------------------------------------
-// kP packed pairs per thread: the CTA's column is 64 * kP voxels wide
-// (voxels x0 + tx + 32 j, j < 2 kP; pair p = columns 2p and 2p + 1).
-constexpr int kSY = 8;
-template <int kP>
+// A CTA's column is kW x kRows voxels, kP packed pairs per thread. From 64 wide on
+// a warp takes a row, voxels x0 + tx + 32 j, j < 2 kP, pair p = columns 2p and 2p + 1;
+// the narrow columns (kP = 1) pair rows ty and ty + kRows / 2.
+template <int kW>
 struct SmoothTile {
-  static constexpr int kSX = 64 * kP;
-  static constexpr int kBoxX = kSX + 8, kBoxY = kSY + 2;
-  static constexpr int kPlaneFloats = kBoxX * kBoxY;                  // floats per plane box
+  static constexpr int kP = kW > 64 ? kW / 64 : 1;
+  static constexpr int kRows = kW < 64 ? 512 / kW : 8;
+  static constexpr int kBoxX = kW + 8, kBoxY = kRows + 2;
+  static constexpr int kPlaneFloats = kBoxX * kBoxY;                 // floats per plane box
   static constexpr int kSlotFloats = (kPlaneFloats + 31) / 32 * 32;  // slots 128-byte aligned
 };
+constexpr int kNarrow[2] = {32, 8};  // widths of the narrow columns
+constexpr int kNarrowSlot = SmoothTile<kNarrow[1]>::kSlotFloats;
+static_assert(kNarrowSlot >= SmoothTile<kNarrow[0]>::kSlotFloats, "");
 constexpr int kSlots = 4;
+// The columns of a step: nx x ny wide ones, then nn narrow ones of width kNarrow[kind]
+// side by side in y, at the end of the rows.
+struct SmoothColumns {
+  int nx, ny, nn, kind;
+};
 constexpr int kHeadFloats = 64;              // before the pitched volume in tmp1: the support box
 
 // Sticky status of the smoothing kernels (bit 0: a TMA wait gave up); read
@@ -245,39 +254,38 @@ __global__ void __launch_bounds__(256) smooth_convert_kernel(const void* __restr
   }
 }
 
-template <bool kF64, int kP>
-__global__ void __launch_bounds__(256, kP == 1 ? 3 : 2) smooth_tma_kernel(const __grid_constant__ CUtensorMap src,
-                                                                         float* __restrict__ dst, int dst_pitch,
-                                                                         int Zc, int Yc, int Xc,
-                                                                         const int* __restrict__ box, int grow,
-                                                                         int write_outside, int planes,
-                                                                         uint32_t wait_lim) {
-  using T = SmoothTile<kP>;
-  constexpr int kBoxX = T::kBoxX;
-  __shared__ __align__(128) float pl[kSlots][T::kSlotFloats];
-  __shared__ __align__(8) uint64_t bar[kSlots];
-  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-  const int x0 = blockIdx.x * T::kSX, y0 = blockIdx.y * kSY, zb = blockIdx.z * planes;
-  const int ze = min(zb + planes, Zc);
-  const int y = y0 + ty;
+template <bool kF64, int kW>
+__device__ __forceinline__ void smooth_column(const CUtensorMap* src, float (*pl)[SmoothTile<kW>::kSlotFloats],
+                                              uint64_t* bar, float* __restrict__ dst, int dst_pitch, int Zc, int Yc,
+                                              int Xc, const int* __restrict__ box, int grow, int write_outside,
+                                              int planes, int x0, int y0, uint32_t wait_lim) {
+  using T = SmoothTile<kW>;
+  constexpr int kP = T::kP, kBoxX = T::kBoxX;
+  constexpr int kDx = kW < 64 ? 0 : 32, kDy = kW < 64 ? T::kRows / 2 : 0;  // second voxel of a pair
+  constexpr int kDi = kDx + kDy * kBoxX;
+  const int tx = kW < 64 ? (int)threadIdx.x % kW : (int)threadIdx.x & 31;
+  const int ty = kW < 64 ? (int)threadIdx.x / kW : (int)threadIdx.x >> 5;
+  const int zb = blockIdx.y * planes, ze = min(zb + planes, Zc);
   const size_t dF = (size_t)Yc * dst_pitch;
-  if (threadIdx.x == 0) {
-    for (int s = 0; s < kSlots; ++s) mbar_init(&bar[s], 1);
-    fence_barrier_init();
-  }
-  // the step before this one has written its maps and read this one's
-  // destination; the next step may be set up meanwhile
-  asm volatile("griddepcontrol.wait;" ::: "memory");
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  if (box_outside(box, grow, zb, ze - 1, y0, min(y0 + kSY, Yc) - 1, x0, min(x0 + T::kSX, Xc) - 1)) {
-    if (write_outside && y < Yc) {
-      for (int z = zb; z < ze; ++z) {
-        float* row = dst + (size_t)z * dF + (size_t)y * dst_pitch;
+  bool in[kP][2], inner[kP][2];  // voxel of the volume, not of its outermost layer in x or y
 #pragma unroll
-        for (int j = 0; j < 2 * kP; ++j)
-          if (x0 + tx + 32 * j < Xc) row[x0 + tx + 32 * j] = 0.0f;
-      }
+  for (int p = 0; p < kP; ++p)
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int x = x0 + tx + 64 * p + h * kDx, y = y0 + ty + h * kDy;
+      in[p][h] = x < Xc && y < Yc;
+      inner[p][h] = x > 0 && x < Xc - 1 && y > 0 && y < Yc - 1;
     }
+  float* const out = dst + (size_t)(y0 + ty) * dst_pitch + x0 + tx;  // the thread's first voxel, plane 0
+  const ptrdiff_t second = kDx + (ptrdiff_t)kDy * dst_pitch;
+  if (box_outside(box, grow, zb, ze - 1, y0, min(y0 + T::kRows, Yc) - 1, x0, min(x0 + kW, Xc) - 1)) {
+    if (write_outside)
+      for (int z = zb; z < ze; ++z)
+#pragma unroll
+        for (int p = 0; p < kP; ++p) {
+          if (in[p][0]) out[z * dF + 64 * p] = 0.0f;
+          if (in[p][1]) out[z * dF + 64 * p + second] = 0.0f;
+        }
     return;
   }
   const int nq = ze - zb + 2;  // planes zb-1 .. ze; plane zb-1+q sits in slot q & 3
@@ -287,13 +295,12 @@ __global__ void __launch_bounds__(256, kP == 1 ? 3 : 2) smooth_tma_kernel(const 
     fence_proxy_async_shared();
     for (; issued < kSlots && issued < nq; ++issued) {
       mbar_expect_tx(&bar[issued], T::kPlaneFloats * (uint32_t)sizeof(float));
-      tma_load_box(pl[issued], &src, x0 - 4, y0 - 1, zb - 1 + issued, &bar[issued]);
+      tma_load_box(pl[issued], src, x0 - 4, y0 - 1, zb - 1 + issued, &bar[issued]);
     }
   }
-  const int ly = ty + 1;
-  const int i0 = ly * kBoxX + tx + 4;  // column j of the thread sits at i0 + 32 j
+  const int i0 = (ty + 1) * kBoxX + tx + 4;  // of the first voxel; the second kDi further
   auto cross = [&](const float* P, int p, uint64_t& cc, uint64_t& xm, uint64_t& xp, uint64_t& ym, uint64_t& yp) {
-    const int ia = i0 + 64 * p, ib = ia + 32;
+    const int ia = i0 + 64 * p, ib = ia + kDi;
     cc = f2_pack(P[ia], P[ib]);
     xm = f2_pack(P[ia - 1], P[ib - 1]);
     xp = f2_pack(P[ia + 1], P[ib + 1]);
@@ -326,7 +333,6 @@ __global__ void __launch_bounds__(256, kP == 1 ? 3 : 2) smooth_tma_kernel(const 
   const uint64_t half = f2_splat(0.5f), quarter = f2_splat(0.25f);
   const uint64_t eps = f2_splat(1e-10f), hundredth = f2_splat(0.01f);
   const uint64_t nz = f2_negzero();  // products as fma(a, b, -0): never fused into a later sum
-  const bool row_in = y < Yc, row_interior = y > 0 && y < Yc - 1;
   const int n = ze - zb;
   auto step = [&](int k, Cross& M, Cross& Q, Cross& N) -> bool {  // planes z-1, z, z+1
     const int z = zb + k;
@@ -335,10 +341,10 @@ __global__ void __launch_bounds__(256, kP == 1 ? 3 : 2) smooth_tma_kernel(const 
       const float* C = pl[(k + 1) & 3];
       const float* Pn = pl[(k + 2) & 3];
       const bool z_int = z > 0 && z < Zc - 1;
-      float* row = dst + (size_t)z * dF + (size_t)y * dst_pitch;
+      float* const at = out + (size_t)z * dF;
 #pragma unroll
       for (int p = 0; p < kP; ++p) {
-        const int ia = i0 + 64 * p, ib = ia + 32;
+        const int ia = i0 + 64 * p, ib = ia + kDi;
         const uint64_t k_mm = f2_pack(C[ia - kBoxX - 1], C[ib - kBoxX - 1]);
         const uint64_t k_pp = f2_pack(C[ia + kBoxX + 1], C[ib + kBoxX + 1]);
         const uint64_t k_mp = f2_pack(C[ia - kBoxX + 1], C[ib - kBoxX + 1]);
@@ -383,9 +389,8 @@ __global__ void __launch_bounds__(256, kP == 1 ? 3 : 2) smooth_tma_kernel(const 
         } else {
           f2_unpack(f2_add(Q.c[p], f2_mul(hundredth, f2_pack(ka, kb), nz)), oa, ob);
         }
-        const int xa = x0 + tx + 64 * p, xb = xa + 32;
-        if (row_in && xa < Xc) row[xa] = (z_int && row_interior && xa > 0 && xa < Xc - 1) ? oa : ca;
-        if (row_in && xb < Xc) row[xb] = (z_int && row_interior && xb > 0 && xb < Xc - 1) ? ob : cb;
+        if (in[p][0]) at[64 * p] = z_int && inner[p][0] ? oa : ca;
+        if (in[p][1]) at[64 * p + second] = z_int && inner[p][1] ? ob : cb;
       }
     }
     if (__syncthreads_or(!ok)) {
@@ -402,13 +407,47 @@ __global__ void __launch_bounds__(256, kP == 1 ? 3 : 2) smooth_tma_kernel(const 
     if (threadIdx.x == 0 && issued < nq) {
       fence_proxy_async_shared();
       mbar_expect_tx(&bar[issued & 3], T::kPlaneFloats * (uint32_t)sizeof(float));
-      tma_load_box(pl[issued & 3], &src, x0 - 4, y0 - 1, zb - 1 + issued, &bar[issued & 3]);
+      tma_load_box(pl[issued & 3], src, x0 - 4, y0 - 1, zb - 1 + issued, &bar[issued & 3]);
       ++issued;
     }
     return k + 1 < n;
   };
   for (int k = 0;; k += 3)
     if (!step(k, S0, S1, S2) || !step(k + 1, S1, S2, S0) || !step(k + 2, S2, S0, S1)) return;
+}
+
+// One step of one map. `wide`: boxes of the columns of kW; `narrow`: of the narrow
+// ones, if there are any.
+template <bool kF64, int kW>
+__global__ void __launch_bounds__(256, kW == 64 ? 3 : 2)
+    smooth_tma_kernel(const __grid_constant__ CUtensorMap wide, const __grid_constant__ CUtensorMap narrow,
+                      float* __restrict__ dst, int dst_pitch, int Zc, int Yc, int Xc, const int* __restrict__ box,
+                      int grow, int write_outside, int planes, const __grid_constant__ SmoothColumns c,
+                      uint32_t wait_lim) {
+  constexpr int kOwn = SmoothTile<kW>::kSlotFloats, kMost = kOwn > kNarrowSlot ? kOwn : kNarrowSlot;
+  __shared__ __align__(128) float pl[kSlots * kMost];
+  __shared__ __align__(8) uint64_t bar[kSlots];
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < kSlots; ++s) mbar_init(&bar[s], 1);
+    fence_barrier_init();
+  }
+  // the step before this one has written its maps and read this one's
+  // destination; the next step may be set up meanwhile
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  const int wides = c.nx * c.ny, i = blockIdx.x;
+#define SI_COLUMN(MAP, W, X0, Y0)                                                                                      \
+  smooth_column<kF64, W>(&MAP, reinterpret_cast<float(*)[SmoothTile<W>::kSlotFloats]>(pl), bar, dst, dst_pitch, Zc, Yc, \
+                         Xc, box, grow, write_outside, planes, X0, Y0, wait_lim)
+  if (i < wides) {
+    SI_COLUMN(wide, kW, i % c.nx * kW, i / c.nx * SmoothTile<kW>::kRows);
+  } else if (kW == 64) {
+    if (c.kind == 0)
+      SI_COLUMN(narrow, kNarrow[0], c.nx * kW, (i - wides) * SmoothTile<kNarrow[0]>::kRows);
+    else
+      SI_COLUMN(narrow, kNarrow[1], c.nx * kW, (i - wides) * SmoothTile<kNarrow[1]>::kRows);
+  }
+#undef SI_COLUMN
 }
 
 __global__ void __launch_bounds__(256) u32_to_f32_kernel(const uint32_t* __restrict__ src, float* __restrict__ dst,
@@ -465,14 +504,14 @@ namespace {
 
 // Tensor map over a pitched float32 volume (Zc, Yc, Xp) with logical extents
 // (Zc, Yc, Xc): reads beyond Xc, Yc, Zc or below 0 return zero.
-int encode_volume_map(CUtensorMap* map, float* base, int Zc, int Yc, int Xc, int box_x, const char* what) {
+int encode_volume_map(CUtensorMap* map, float* base, int Zc, int Yc, int Xc, int box_x, int box_y, const char* what) {
   const EncodeTiledFn enc = encode_fn();
   if (!enc) return set_error(SI_ERR_CUDA, "%s: cuTensorMapEncodeTiled unavailable", what);
   std::memset(map, 0, sizeof(*map));
   const int Xp = pitch4(Xc);
   const cuuint64_t dims[3] = {(cuuint64_t)Xc, (cuuint64_t)Yc, (cuuint64_t)Zc};
   const cuuint64_t strides[2] = {(cuuint64_t)Xp * sizeof(float), (cuuint64_t)Xp * Yc * sizeof(float)};
-  const cuuint32_t boxd[3] = {(cuuint32_t)box_x, (cuuint32_t)(kSY + 2), 1};
+  const cuuint32_t boxd[3] = {(cuuint32_t)box_x, (cuuint32_t)box_y, 1};
   const cuuint32_t estr[3] = {1, 1, 1};
   const CUresult cr = enc(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, base, dims, strides, boxd, estr,
                           CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
@@ -528,16 +567,32 @@ int smooth_maps(void* maps, float* tmp0, float* tmp1, int nol, int Zc, int Yc, i
   // pairs per thread: 128-wide columns only when selected and the rows are long enough
   const int kp = g_smooth_pairs.load(std::memory_order_relaxed) == 1 || Xc <= 64 ? 1 : 2;
   const int sx = 64 * kp;
-  CUtensorMap map0, map1;
+  // The last column of a row is as narrow as what is left of the row lets it be, so
+  // that a volume just above a multiple of 64 (a power of two with its padding) does
+  // not pay for one of 64. A step: 130^3 16.2 and 12.7 us, 119x143x135 15.8 and 12.4,
+  // 178x226x210 37.7 and 32.2, 402x514x514 294 and 258.
+  SmoothColumns c{(Xc + sx - 1) / sx, (Yc + 7) / 8, 0, 0};
+  const int left = Xc % 64;
+  if (kp == 1 && left && left <= kNarrow[0]) {
+    c.kind = left <= kNarrow[1] ? 1 : 0;
+    c.nx = Xc / 64;
+    const int rows = 512 / kNarrow[c.kind];
+    c.nn = (Yc + rows - 1) / rows;
+  }
+  CUtensorMap map0{}, map1{}, nmap0{}, nmap1{};
   if (iters > 0) {
-    int rc = encode_volume_map(&map0, tmp0, Zc, Yc, Xc, sx + 8, what);
-    if (rc) return rc;
-    rc = encode_volume_map(&map1, tmp1v, Zc, Yc, Xc, sx + 8, what);
+    int rc = encode_volume_map(&map0, tmp0, Zc, Yc, Xc, sx + 8, 10, what);
+    if (!rc) rc = encode_volume_map(&map1, tmp1v, Zc, Yc, Xc, sx + 8, 10, what);
+    if (c.nn) {
+      const int w = kNarrow[c.kind], rows = 512 / w;
+      if (!rc) rc = encode_volume_map(&nmap0, tmp0, Zc, Yc, Xc, w + 8, rows + 2, what);
+      if (!rc) rc = encode_volume_map(&nmap1, tmp1v, Zc, Yc, Xc, w + 8, rows + 2, what);
+    }
     if (rc) return rc;
   }
-  const int columns = ((Xc + sx - 1) / sx) * ((Yc + kSY - 1) / kSY);
+  const int columns = c.nx * c.ny + c.nn;
   const int planes = smooth_planes(columns, Zc);
-  const dim3 grid((Xc + sx - 1) / sx, (Yc + kSY - 1) / kSY, (Zc + planes - 1) / planes);
+  const dim3 grid(columns, (Zc + planes - 1) / planes);
   const int cgrid = std::max(1, std::min(sm_count() * 8, (Zc * Yc + 7) / 8));
   const uint32_t wl = wait_limit();
   for (int l = 0; l < nol; ++l) {
@@ -553,26 +608,27 @@ int smooth_maps(void* maps, float* tmp0, float* tmp1, int nol, int Zc, int Yc, i
     for (int it = 1; it <= iters; ++it) {
       const bool last = it == iters;
       const CUtensorMap& sm = (it & 1) ? map0 : map1;
+      const CUtensorMap& nm = (it & 1) ? nmap0 : nmap1;
       float* dst = last ? mf : ((it & 1) ? tmp1v : tmp0);
       const int pitch = last ? Xc : Xp;
       // only iteration 1's destination (tmp1) may hold another map's values
       // outside the support; every later destination is +0 there already
       const int write_outside = (it == 1 && !last) ? 1 : 0;
-#define SI_SMOOTH(F64, P)                                                                                          \
-  if (launch_step(smooth_tma_kernel<F64, P>, grid, st, sm, dst, pitch, Zc, Yc, Xc, box, it, write_outside, planes, \
-                  wl) != cudaSuccess)                                                                              \
+#define SI_SMOOTH(F64, W)                                                                                         \
+  if (launch_step(smooth_tma_kernel<F64, W>, grid, st, sm, nm, dst, pitch, Zc, Yc, Xc, box, it, write_outside,    \
+                  planes, c, wl) != cudaSuccess)                                                                  \
   return check_launch(what)
       if (update) {
         if (kp == 2) {
-          SI_SMOOTH(true, 2);
+          SI_SMOOTH(true, 128);
         } else {
-          SI_SMOOTH(true, 1);
+          SI_SMOOTH(true, 64);
         }
       } else {
         if (kp == 2) {
-          SI_SMOOTH(false, 2);
+          SI_SMOOTH(false, 128);
         } else {
-          SI_SMOOTH(false, 1);
+          SI_SMOOTH(false, 64);
         }
       }
 #undef SI_SMOOTH
