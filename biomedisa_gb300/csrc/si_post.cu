@@ -522,15 +522,16 @@ int encode_volume_map(CUtensorMap* map, float* base, int Zc, int Yc, int Xc, int
 
 // Planes a CTA marches through: 32, or fewer where that leaves fewer than five
 // waves of CTAs (3 per SM): a step then lasts as long as one column takes,
-// about 0.7 us a plane. Two planes more than it writes are read per CTA, so
-// large volumes keep long columns. One step on a hit map, 32 / 16 / 8 / 4
-// planes, each started after the one before it: 42x38x35 23.8 / 14.7 / 9.9 /
-// 7.8 us, 130^3 34.5 / 24.7 / 20.5 / 20.0, 178x226x210 53.5 / 47.9 / 45.9 / 47.6,
-// 402x514x514 375 / 375 / 386 / 420.
+// about 0.7 us a plane; 2 where even those CTAs all run at once. Two planes more
+// than it writes are read per CTA, so large volumes keep long columns. One step,
+// 16 / 8 / 4 / 2 planes: 42x38x35 11.1 / 6.6 / 4.4 / 3.6 us, 66^3 11.8 / 7.6 / 5.7 /
+// 4.5, 130^3 17.2 / 13.4 / 12.8 / 14.8, 178x226x210 33.3 / 32.3 / 35.4 / 44.3,
+// 258^3 59.5 / 61.3 / 69.1 / 87.4.
 int smooth_planes(int columns, int Zc) {
   const int want = 5 * 3 * sm_count();
   int planes = 32;
   while (planes > 4 && (long long)columns * ((Zc + planes - 1) / planes) < want) planes /= 2;
+  if (planes == 4 && (long long)columns * ((Zc + 1) / 2) <= 3 * sm_count()) planes = 2;
   return planes;
 }
 
