@@ -19,6 +19,7 @@
 #include <cuda.h>
 
 #include <algorithm>
+#include <cmath>
 #include <atomic>
 #include <cstring>
 #include <mutex>
@@ -59,6 +60,7 @@ struct BrickGeom {
   int edge;  // brick edge used for bucketing
   int nbz, nby, nbx;
   uint32_t nb;   // bricks per label
+  uint32_t label_step, brick_step;  // bucket = label slot * label_step + brick * brick_step
   uint32_t F;    // Yc * Xc
   uint32_t Xp;   // record row pitch (even)
   FastDiv by_F, by_X, by_edge;
@@ -80,7 +82,7 @@ __device__ __forceinline__ uint32_t bucket_of(const BrickGeom& g, const uint4& s
   coords(g, s.x, z, y, x);
   const uint32_t brick = (g.by_edge((uint32_t)z) * (uint32_t)g.nby + g.by_edge((uint32_t)y)) * (uint32_t)g.nbx +
                          g.by_edge((uint32_t)x);
-  return (s.w >> 24) * g.nb + brick;
+  return (s.w >> 24) * g.label_step + brick * g.brick_step;
 }
 
 template <bool kFirst>
@@ -562,6 +564,8 @@ BrickGeom make_geom(int Zc, int Yc, int Xc, int edge = kCore) {
   g.nby = (Yc + edge - 1) / edge;
   g.nbx = (Xc + edge - 1) / edge;
   g.nb = (uint32_t)g.nbz * g.nby * g.nbx;
+  g.label_step = g.nb;
+  g.brick_step = 1u;
   g.F = (uint32_t)Yc * Xc;
   g.Xp = (uint32_t)((Xc + 1) & ~1);
   g.by_F = FastDiv(g.F);
@@ -710,7 +714,17 @@ extern "C" int si_walk_bricks(const void* work, int Zc, int Yc, int Xc, const si
 namespace si {
 namespace {
 constexpr uint64_t kBatchWalks = 1ull << 25;  // default walks per seed range of si_walk_sorted
-constexpr int kSortEdge = 6;
+// Sort bricks. Their labels follow one another in the sorted order, so walkers that
+// run at the same time share records and add to different maps (label by label the
+// same bricks came round again for every label, and all walkers of a moment added
+// to one map: 128^3 41.5 ms, now 41.0). Default edge: about kBrickWalks walks per
+// brick, 4 to 8. Smaller bricks keep a dense set of walkers closer together, of a
+// sparse one a CTA then spans too many: 176x224x208 with 2.4 walks a voxel, edge
+// 4 / 6 / 8 309 / 317 / 333 ms, 128^3 with 1.0 41.4 / 41.0 / 41.3, 419x492x462 with
+// 0.45 854 / 828 / 820.
+constexpr int kSortEdge = 6;  // of batches
+constexpr int kMinSortEdge = 4, kMaxSortEdge = 8;
+constexpr double kBrickWalks = 160.0;
 // Default sweep length: 32 steps, 128 for walks of kLongWalk steps and more.
 // Longer sweeps share the sort's cost among more steps, but let the walkers
 // spread further between sorts. Walks of 4000 steps, 48 / 64 / 96 / 128 / 256
@@ -1032,13 +1046,42 @@ int finish_walk(cudaStream_t st, const WalkBuffers& w, std::vector<cudaGraphExec
 }  // namespace
 }  // namespace si
 
+namespace si {
+namespace {
+BrickGeom sort_geom(int Zc, int Yc, int Xc, int nol, int edge) {
+  BrickGeom g = make_geom(Zc, Yc, Xc, edge);
+  g.label_step = 1u;
+  g.brick_step = (uint32_t)nol;
+  return g;
+}
+
+uint64_t sort_bytes(int Zc, int Yc, int Xc, uint64_t walks, int nol, int edge) {
+  return sort_layout((uint64_t)make_geom(Zc, Yc, Xc, edge).nb * (uint64_t)nol, walks, 0).total;
+}
+
+// The default sort edge for this many walks; kSortEdge where the preferred one has too
+// many buckets or does not fit in `bytes`. More walks prefer no larger edge, so what
+// si_walk_sorted_scratch asks for is enough for any fewer.
+int default_sort_edge(int Zc, int Yc, int Xc, uint64_t walks, int nol, unsigned long long bytes) {
+  const double per_voxel = (double)std::max<uint64_t>(walks, 1) / ((double)Zc * Yc * Xc);
+  const double want = std::cbrt(kBrickWalks / per_voxel);
+  const int edge = want >= kMaxSortEdge ? kMaxSortEdge : std::max(kMinSortEdge, (int)std::lround(want));
+  const bool counts = (uint64_t)make_geom(Zc, Yc, Xc, edge).nb * (uint64_t)nol < 0xFFFFFFFFull;
+  return counts && sort_bytes(Zc, Yc, Xc, walks, nol, edge) <= bytes ? edge : kSortEdge;
+}
+}  // namespace
+}  // namespace si
+
 extern "C" int si_walk_sorted_scratch(int Zc, int Yc, int Xc, uint64_t max_walks, int nol, int sort_edge,
                                       unsigned long long* bytes) {
   clear_error();
   if (!bytes || Zc < 3 || Yc < 3 || Xc < 3 || nol < 1 || nol > 256 || sort_edge < 0 || sort_edge > 1024)
     return set_error(SI_ERR_ARG, "si_walk_sorted_scratch: bad arguments");
-  const BrickGeom g = make_geom(Zc, Yc, Xc, sort_edge > 0 ? sort_edge : kSortEdge);
-  *bytes = sort_layout((uint64_t)g.nb * nol, max_walks, 0).total;
+  *bytes = sort_bytes(Zc, Yc, Xc, max_walks, nol, sort_edge > 0 ? sort_edge : kSortEdge);
+  if (sort_edge <= 0) {
+    const int edge = default_sort_edge(Zc, Yc, Xc, max_walks, nol, ~0ull);
+    *bytes = std::max<unsigned long long>(*bytes, sort_bytes(Zc, Yc, Xc, max_walks, nol, edge));
+  }
   return SI_OK;
 }
 
@@ -1080,7 +1123,6 @@ extern "C" int si_walk_sorted(const void* packed, int work_is_float, int Zc, int
     return set_error(SI_ERR_LIMIT, "si_walk_sorted: nbrw*sorw must be below 2^24");
   const bool default_steps = sweep_steps <= 0;
   if (default_steps) sweep_steps = default_sweep_steps(sorw);
-  if (sort_edge <= 0) sort_edge = kSortEdge;
   if (sort_edge > 1024) return set_error(SI_ERR_ARG, "si_walk_sorted: sort_edge above 1024");
   cudaStream_t st = as_stream(stream);
   if (rounds_out) *rounds_out = 0;
@@ -1092,7 +1134,11 @@ extern "C" int si_walk_sorted(const void* packed, int work_is_float, int Zc, int
   const uint64_t walks = (uint64_t)ns * (uint64_t)nbrw;
   if (walks == 0 || sorw == 0) return SI_OK;
   if (walks >= 0xFFFFFFFFull) return set_error(SI_ERR_LIMIT, "si_walk_sorted: more than 2^32 walks");
-  const BrickGeom g = make_geom(Zc, Yc, Xc, sort_edge);
+  if (sort_edge <= 0)  // less than kSortEdge takes is refused below, whatever the default
+    sort_edge = scratch_bytes < sort_bytes(Zc, Yc, Xc, walks, nol, kSortEdge)
+                    ? kSortEdge
+                    : default_sort_edge(Zc, Yc, Xc, walks, nol, scratch_bytes);
+  const BrickGeom g = sort_geom(Zc, Yc, Xc, nol, sort_edge);
   if ((uint64_t)g.nb * (uint64_t)nol >= 0xFFFFFFFFull) return set_error(SI_ERR_LIMIT, "si_walk_sorted: too many buckets");
   const uint32_t nbt = g.nb * (uint32_t)nol;
   const SortLayout L = sort_layout(nbt, walks, 0);
@@ -1208,6 +1254,7 @@ struct VolDesc {
   int Zc, Yc, Xc;
   int nby, nbx;     // bricks per row / column
   uint32_t nb;      // bricks per label
+  uint32_t nol;
   uint32_t bucket0; // first bucket of this volume
   uint64_t walk0;   // first global walk index of this volume (round 0)
   uint32_t ns;      // seeds
@@ -1225,7 +1272,7 @@ __device__ __forceinline__ uint32_t bbucket(const VolDesc& v, const FastDiv& by_
   const uint32_t y = v.by_X(r);
   const uint32_t x = r - y * (uint32_t)v.Xc;
   const uint32_t brick = (by_edge(z) * (uint32_t)v.nby + by_edge(y)) * (uint32_t)v.nbx + by_edge(x);
-  return v.bucket0 + (s.w >> 24) * v.nb + brick;
+  return v.bucket0 + (s.w >> 24) + brick * v.nol;
 }
 
 template <bool kFirst>
@@ -1416,6 +1463,7 @@ int make_batch_plan(const si_volume_t* vols, int n_vols, int nbrw, int edge, con
     d.nby = (in.Yc + edge - 1) / edge;
     d.nbx = (in.Xc + edge - 1) / edge;
     d.nb = (uint32_t)nbz * d.nby * d.nbx;
+    d.nol = (uint32_t)in.nol;
     d.bucket0 = (uint32_t)bucket;
     d.walk0 = walk;
     d.ns = ns_host ? (ns_host[v] < in.max_seeds ? ns_host[v] : in.max_seeds) : in.max_seeds;

@@ -132,3 +132,43 @@ def test_one_walk_or_two_per_thread(nbrw, dtype, cuda):
     exp = O.smart_interpolation(img.astype(dtype), lab, key=3, **kw)
     got = smart_interpolation(img.astype(dtype), lab, rng_seed=3, **kw)
     assert np.array_equal(got["hits"], exp["hits"])
+
+
+@pytest.mark.parametrize("dense", [False, True])
+def test_default_bricks_fit_the_scratch(dense, cuda):
+    """The default sort edge follows the walks per voxel; a scratch sized for
+    bricks of six voxels, or for any number of walks above the actual one, is
+    enough for it, and the hits stay the oracle's."""
+    import ctypes
+
+    import torch
+
+    from biomedisa_gb300 import interpolation as I
+
+    img, lab = _volume((26, 40, 44), 7, 2 if dense else 13)
+    nbrw = 12 if dense else 1
+    ti, tl = I.upload(*I.normalize_host_dtypes(img, lab))
+    job = I.DeviceJob(ti, nat.SI_U8, tl, nat.SI_I32, nbrw=nbrw, sorw=90, rng_seed=8)
+    assert job.analyze() is None
+    job.prepare()
+    cp, nol = job.cplan, job.lplan.nol
+    exp = O.smart_interpolation(img, lab, key=8, nbrw=nbrw, sorw=90, return_hits=True)["hits"]
+    n = int(job.n_seeds.item())
+    sizes = set()
+    for edge, walks in ((6, n * nbrw), (0, n * nbrw), (0, 40 * n * nbrw)):
+        need = ctypes.c_ulonglong(0)
+        nat.call("si_walk_sorted_scratch", cp.Zc, cp.Yc, cp.Xc, walks, nol, edge, ctypes.byref(need))
+        sizes.add(need.value)
+        scratch = torch.full((need.value + 4096,), 99, dtype=torch.uint8, device="cuda")
+        job.hits = torch.zeros((nol, cp.Zc, cp.Yc, cp.Xc), dtype=torch.int32, device="cuda")
+        nat.call("si_walk_sorted", job.packed.data_ptr(), 0, cp.Zc, cp.Yc, cp.Xc, job.seeds.data_ptr(),
+                 job.n_seeds.data_ptr(), n, nbrw, 90, 8, job.hits.data_ptr(), nol, 0, 0, scratch.data_ptr(), need.value,
+                 None, nat.stream())
+        assert bool((scratch[need.value:] == 99).all())
+        assert np.array_equal(job.hits_full().cpu().numpy(), exp)
+    assert len(sizes) == (3 if dense else 2)  # sparse walks take larger bricks in no less scratch
+    nat.call("si_walk_sorted_scratch", cp.Zc, cp.Yc, cp.Xc, n * nbrw, nol, 6, ctypes.byref(need))
+    with pytest.raises(nat.NativeError, match="scratch"):
+        nat.call("si_walk_sorted", job.packed.data_ptr(), 0, cp.Zc, cp.Yc, cp.Xc, job.seeds.data_ptr(),
+                 job.n_seeds.data_ptr(), n, nbrw, 90, 8, job.hits.data_ptr(), nol, 0, 0, scratch.data_ptr(),
+                 need.value - 1, None, nat.stream())
