@@ -717,14 +717,16 @@ constexpr uint64_t kBatchWalks = 1ull << 25;  // default walks per seed range of
 // Sort bricks. Their labels follow one another in the sorted order, so walkers that
 // run at the same time share records and add to different maps (label by label the
 // same bricks came round again for every label, and all walkers of a moment added
-// to one map: 128^3 41.5 ms, now 41.0). Default edge: about kBrickWalks walks per
-// brick, 4 to 8. Smaller bricks keep a dense set of walkers closer together, of a
-// sparse one a CTA then spans too many: 176x224x208 with 2.4 walks a voxel, edge
-// 4 / 6 / 8 309 / 317 / 333 ms, 128^3 with 1.0 41.4 / 41.0 / 41.3, 419x492x462 with
-// 0.45 854 / 828 / 820.
+// to one map: 128^3 41.5 ms, now 41.0). Default edge, 4 to 8: about kBrickWalks walks
+// per brick, but no fewer than kBucketWalks live ones per bucket. Smaller bricks keep
+// a dense set of walkers closer together; of a sparse one a CTA then spans too many,
+// and counting and scanning buckets that hold a walker or two costs more than it
+// orders. Walks in ms at edges 4 / 6 / 8: 176x224x208, 9 labels, 2.4 walks a voxel 309 /
+// 317 / 333, 400x512x512, 9 labels, 2.1 a voxel in seven ranges 4268 / 4164 / 4140, 128^3,
+// 3 labels, 1.0 41.4 / 41.0 / 41.3, 419x492x462, 3 labels, 0.5 713 / 698 / 692.
 constexpr int kSortEdge = 6;  // of batches
 constexpr int kMinSortEdge = 4, kMaxSortEdge = 8;
-constexpr double kBrickWalks = 160.0;
+constexpr double kBrickWalks = 160.0, kBucketWalks = 20.0;
 // Default sweep length: 32 steps, 128 for walks of kLongWalk steps and more.
 // Longer sweeps share the sort's cost among more steps, but let the walkers
 // spread further between sorts. Walks of 4000 steps, 48 / 64 / 96 / 128 / 256
@@ -1063,8 +1065,9 @@ uint64_t sort_bytes(int Zc, int Yc, int Xc, uint64_t walks, int nol, int edge) {
 // many buckets or does not fit in `bytes`. More walks prefer no larger edge, so what
 // si_walk_sorted_scratch asks for is enough for any fewer.
 int default_sort_edge(int Zc, int Yc, int Xc, uint64_t walks, int nol, unsigned long long bytes) {
-  const double per_voxel = (double)std::max<uint64_t>(walks, 1) / ((double)Zc * Yc * Xc);
-  const double want = std::cbrt(kBrickWalks / per_voxel);
+  const double V = (double)Zc * Yc * Xc, n = (double)std::max<uint64_t>(walks, 1);
+  const double live = std::min(n, (double)range_walks());
+  const double want = std::cbrt(std::max(kBrickWalks * V / n, kBucketWalks * nol * V / live));
   const int edge = want >= kMaxSortEdge ? kMaxSortEdge : std::max(kMinSortEdge, (int)std::lround(want));
   const bool counts = (uint64_t)make_geom(Zc, Yc, Xc, edge).nb * (uint64_t)nol < 0xFFFFFFFFull;
   return counts && sort_bytes(Zc, Yc, Xc, walks, nol, edge) <= bytes ? edge : kSortEdge;

@@ -463,7 +463,7 @@ class DeviceJob:
                                       self.hits, nol, self.sweep_steps, self.sort_edge)
             # per sweep: scatter, sweep and the scan's kernels (one of them for up
             # to 16384 buckets, else three); count and scan before the first. The
-            # default edge is 4 to 8 by the walks per voxel
+            # default edge is 4 to 8 by the walks per brick and bucket
             edge = self.sort_edge or 6
             buckets = nol * -(-cp.Zc // edge) * -(-cp.Yc // edge) * -(-cp.Xc // edge)
             scans = 1 if buckets <= 16384 else 3

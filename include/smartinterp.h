@@ -219,7 +219,7 @@ int si_walk_bricks(const void* work, int Zc, int Yc, int Xc,
 
 /* Scratch bytes si_walk_sorted needs (crop dims, max walks = seeds * nbrw,
  * labels, sort brick edge; sort_edge <= 0 selects the default, 4 to 8 by the
- * walks per voxel). Enough for any fewer walks. */
+ * walks per brick and bucket). Enough for any fewer walks. */
 int si_walk_sorted_scratch(int Zc, int Yc, int Xc, uint64_t max_walks, int nol,
                            int sort_edge, unsigned long long* bytes);
 
@@ -229,7 +229,7 @@ int si_walk_sorted_scratch(int Zc, int Yc, int Xc, uint64_t max_walks, int nol,
  * for walks of at least 1000 steps, 256 for those where the device holds a
  * thread for each, else 32);
  * between sweeps the walkers are counting-sorted by (label slot, brick of
- * sort_edge^3 voxels; default when <= 0: 4 to 8 by the walks per voxel, 6 where
+ * sort_edge^3 voxels; default when <= 0: 4 to 8 by the walks per brick and bucket, 6 where
  * the scratch holds no more),
  * so concurrently running walkers share a compact, cache-resident part of
  * the volume and of the hit maps. scratch: si_walk_sorted_scratch bytes;
