@@ -84,7 +84,7 @@ WORKLOADS = {
 }
 
 # one kernel per entry-point call except these (launches per call)
-MULTI_LAUNCH = {"si_extract_seeds": 3, "si_nn_conv3d_wgrad": 2}
+MULTI_LAUNCH = {"si_extract_seeds": 3, "si_nn_conv3d_wgrad": 2, "si_nn_xent": 2}
 
 WALK_SECTORS_L2 = 2  # per walker step at L2: one packed-record sector + one atomic sector
 WALK_BYTES_PAYLOAD_U8 = 10  # 6 neighbour bytes + one 4-byte hit per step

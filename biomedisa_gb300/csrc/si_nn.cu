@@ -810,65 +810,112 @@ __global__ void __launch_bounds__(256) xent_kernel(const float* __restrict__ log
 
 // The same for 16 channels at 16-byte alignment: a voxel's logits stay in
 // registers between the passes over them (one by one they were read four times:
-// 238 us at the 8 x 64^3 training batch; 59 us so), and the loss is summed with
-// compensation per thread and pairwise per CTA before its one atomic addition.
-__global__ void __launch_bounds__(256) xent16_kernel(const float* __restrict__ logits,
-                                                     const float* __restrict__ target,
-                                                     const float* __restrict__ weight, int64_t V, int nol, float scale,
-                                                     __nv_bfloat16* __restrict__ dlogits, float* __restrict__ loss) {
-  __shared__ double s_sum[8];
-  float sum = 0.0f, lost = 0.0f;
-  for (int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; v < V; v += (int64_t)gridDim.x * blockDim.x) {
-    float z[16], p[16];
+// 276 us a call at the 8 x 64^3 training batch; 97 us so, loss kernel included).
+//
+// The gradient takes xent_kernel's operations, bit for bit. The loss takes log1pf
+// (__logf is off by up to 2^-21 where a voxel is sure of its label, and that does
+// not average out), one binary64 addition per voxel, and a fixed order: CTA sums
+// leave through the first eight bytes of the gradient of the CTA's first voxel,
+// where xent16_loss_kernel finds them, adds them up and puts the gradient back.
+// Off the 64-bit sum by at most 1e-7 then; by up to 9e-7, another amount in each run,
+// with the CTAs' sums added to the loss in binary32 (83 us), and by up to 6e-6 with
+// one such addition per warp, as in xent_kernel. Nothing is compensated, so an
+// infinite term leaves an infinite loss.
+__device__ __forceinline__ float xent16_voxel(const float* __restrict__ logits, const float* __restrict__ target,
+                                              float wv, int nol, float scale, uint4 (&grad)[2]) {
+  float z[16], p[16];
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      const float4 q = reinterpret_cast<const float4*>(logits + v * 16)[k];
-      z[4 * k] = q.x; z[4 * k + 1] = q.y; z[4 * k + 2] = q.z; z[4 * k + 3] = q.w;
+  for (int k = 0; k < 4; ++k) {
+    const float4 q = reinterpret_cast<const float4*>(logits)[k];
+    z[4 * k] = q.x; z[4 * k + 1] = q.y; z[4 * k + 2] = q.z; z[4 * k + 3] = q.w;
+  }
+#pragma unroll
+  for (int l = 0; l < 16; ++l) p[l] = l < nol ? target[l] : 0.0f;
+  float m = -INFINITY;
+#pragma unroll
+  for (int l = 0; l < 16; ++l)
+    if (l < nol) m = fmaxf(m, z[l]);
+  float s = 0.0f, others = 0.0f;  // others: without the first largest, whose exponential is 1
+  bool top = false;
+#pragma unroll
+  for (int l = 0; l < 16; ++l)
+    if (l < nol) {
+      const float e = __expf(z[l] - m);
+      s += e;
+      if (z[l] == m && !top)
+        top = true;
+      else
+        others += e;
     }
+  const float lse = m + __logf(s), log_s = log1pf(others);
+  float loss = 0.0f;
+  uint32_t d[8];
 #pragma unroll
-    for (int l = 0; l < 16; ++l) p[l] = l < nol ? target[v * nol + l] : 0.0f;
-    const float wv = weight ? weight[v] : 1.0f;
-    float m = -INFINITY;
+  for (int k = 0; k < 8; ++k) {
+    float g[2];
 #pragma unroll
-    for (int l = 0; l < 16; ++l)
-      if (l < nol) m = fmaxf(m, z[l]);
-    float s = 0.0f;
-#pragma unroll
-    for (int l = 0; l < 16; ++l)
-      if (l < nol) s += __expf(z[l] - m);
-    const float lse = m + __logf(s);
-    float local = 0.0f;
-    uint32_t d[8];
-#pragma unroll
-    for (int k = 0; k < 8; ++k) {
-      float g[2];
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const int l = 2 * k + h;
-        g[h] = 0.0f;
-        if (l < nol) {
-          const float q = __expf(z[l] - lse);
-          local += -wv * p[l] * (z[l] - lse);
-          g[h] = wv * (q - p[l]) * scale;
-        }
+    for (int h = 0; h < 2; ++h) {
+      const int l = 2 * k + h;
+      g[h] = 0.0f;
+      if (l < nol) {
+        loss += wv * p[l] * (log_s - (z[l] - m));
+        g[h] = wv * (__expf(z[l] - lse) - p[l]) * scale;
       }
-      d[k] = pack2(__float2bfloat16(g[0]), __float2bfloat16(g[1]));
     }
-    uint4* o = reinterpret_cast<uint4*>(dlogits + v * 16);
-    o[0] = make_uint4(d[0], d[1], d[2], d[3]);
-    o[1] = make_uint4(d[4], d[5], d[6], d[7]);
-    const float add = __fsub_rn(local, lost), t = __fadd_rn(sum, add);
-    lost = __fsub_rn(__fsub_rn(t, sum), add);
-    sum = t;
+    d[k] = pack2(__float2bfloat16(g[0]), __float2bfloat16(g[1]));
   }
-  double w = sum;
+  grad[0] = make_uint4(d[0], d[1], d[2], d[3]);
+  grad[1] = make_uint4(d[4], d[5], d[6], d[7]);
+  return loss;
+}
+
+// Sum over the CTA, the same in every run; valid in thread 0.
+__device__ __forceinline__ double cta_sum(double w, double* s_warp) {
+#pragma unroll
   for (int o = 16; o; o >>= 1) w += __shfl_xor_sync(0xffffffffu, w, o);
-  if ((threadIdx.x & 31) == 0) s_sum[threadIdx.x >> 5] = w;
+  if ((threadIdx.x & 31) == 0) s_warp[threadIdx.x >> 5] = w;
   __syncthreads();
-  if (threadIdx.x == 0) {
-    for (int k = 1; k < 8; ++k) w += s_sum[k];
-    atomicAdd(loss, (float)w);
+  for (int k = 1; threadIdx.x == 0 && k < (int)(blockDim.x >> 5); ++k) w += s_warp[k];
+  return w;
+}
+
+constexpr int kXentThreads = 256;
+
+__global__ void __launch_bounds__(kXentThreads) xent16_kernel(const float* __restrict__ logits,
+                                                              const float* __restrict__ target,
+                                                              const float* __restrict__ weight, int64_t V, int nol,
+                                                              float scale, __nv_bfloat16* __restrict__ dlogits) {
+  __shared__ double s_warp[kXentThreads / 32];
+  const int64_t first = (int64_t)blockIdx.x * kXentThreads;
+  double sum = 0.0;
+  for (int64_t v = first + threadIdx.x; v < V; v += (int64_t)gridDim.x * kXentThreads) {
+    uint4 grad[2];
+    sum += xent16_voxel(logits + v * 16, target + v * nol, weight ? weight[v] : 1.0f, nol, scale, grad);
+    uint4* o = reinterpret_cast<uint4*>(dlogits + v * 16);
+    o[0] = grad[0];
+    o[1] = grad[1];
   }
+  sum = cta_sum(sum, s_warp);
+  if (threadIdx.x == 0) *reinterpret_cast<double*>(dlogits + first * 16) = sum;
+}
+
+// The sums of the n CTAs, whose first voxels' gradients are restored.
+__global__ void __launch_bounds__(1024) xent16_loss_kernel(const float* __restrict__ logits,
+                                                           const float* __restrict__ target,
+                                                           const float* __restrict__ weight, int n, int nol,
+                                                           float scale, __nv_bfloat16* __restrict__ dlogits,
+                                                           float* __restrict__ loss) {
+  __shared__ double s_warp[32];
+  double sum = 0.0;
+  for (int b = threadIdx.x; b < n; b += blockDim.x) {
+    const int64_t v = (int64_t)b * kXentThreads;
+    sum += *reinterpret_cast<const double*>(dlogits + v * 16);
+    uint4 grad[2];
+    xent16_voxel(logits + v * 16, target + v * nol, weight ? weight[v] : 1.0f, nol, scale, grad);
+    reinterpret_cast<uint4*>(dlogits + v * 16)[0] = grad[0];
+  }
+  sum = cta_sum(sum, s_warp);
+  if (threadIdx.x == 0) atomicAdd(loss, (float)sum);
 }
 
 // AdamW on fp32 master weights; writes the bf16 working copy.
@@ -1151,9 +1198,11 @@ extern "C" int si_nn_xent(const float* logits, const float* target, const float*
   if (!logits || !target || !dlogits || !loss || nol < 1 || nol > C)
     return set_error(SI_ERR_ARG, "si_nn_xent: bad arguments");
   if (C == 16 && ((uintptr_t)logits | (uintptr_t)dlogits) % 16 == 0) {
-    const int64_t want = (V + 255) / 256, most = (int64_t)sm_count() * 4;
-    xent16_kernel<<<(int)std::max<int64_t>(1, std::min(want, most)), 256, 0, as_stream(stream)>>>(
-        logits, target, weight, V, nol, scale, static_cast<__nv_bfloat16*>(dlogits), loss);
+    if (V <= 0) return SI_OK;
+    auto* dl = static_cast<__nv_bfloat16*>(dlogits);
+    const int n = (int)std::min<int64_t>((V + kXentThreads - 1) / kXentThreads, (int64_t)sm_count() * 4);
+    xent16_kernel<<<n, kXentThreads, 0, as_stream(stream)>>>(logits, target, weight, V, nol, scale, dl);
+    xent16_loss_kernel<<<1, 1024, 0, as_stream(stream)>>>(logits, target, weight, n, nol, scale, dl, loss);
     return check_launch("si_nn_xent");
   }
   xent_kernel<<<egrid(V), 256, 0, as_stream(stream)>>>(logits, target, weight, V, C, nol, scale,
