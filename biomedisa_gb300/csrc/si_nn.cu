@@ -596,7 +596,7 @@ __global__ void __launch_bounds__(kWgGroups * 96, 1)
           }
           // compensated (Kahan): the sum of a unit's rows is as good as one rounding
           const float add = __fsub_rn(t, lost[c]), sum = __fadd_rn(bias[c], add);
-          lost[c] = __fsub_rn(__fsub_rn(sum, bias[c]), add);
+          lost[c] = fabsf(sum) < INFINITY ? __fsub_rn(__fsub_rn(sum, bias[c]), add) : 0.0f;  // not inf - inf
           bias[c] = sum;
         }
       }
