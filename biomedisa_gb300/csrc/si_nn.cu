@@ -448,6 +448,9 @@ __device__ __forceinline__ void copy_async16(uint32_t dst, const void* src, bool
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(ok ? 16 : 0) : "memory");
 }
 
+// kRagged: W is no multiple of 64, so a row's last chunk is shorter. (Compiled apart for
+// the full rows' sake: 102 and 98 us at 8 x 64^3.)
+template <bool kRagged>
 __global__ void __launch_bounds__(kWgGroups * 96, 1)
     wgrad16_columns_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ dy,
                            float* __restrict__ dw, float* __restrict__ db, float* __restrict__ partials,
@@ -465,7 +468,7 @@ __global__ void __launch_bounds__(kWgGroups * 96, 1)
   // unit), with the dY row i + 1 below it.
   unsigned u = u0, r = 0, r1 = 0;  // unit; first row behind the segment; end of the unit
   int i = 0, jn = 0, yi = 0;  // yi: the input row's y
-  bool empty = false, zin = false;
+  bool empty = false, zin = false, ragged = false;  // ragged: in the row's last chunk
   unsigned okx = 0, okd = 0;  // this lane's pieces that lie inside the row
   const char *xp = nullptr, *dp = nullptr;  // its first piece of the input row, of the dY row
   const int64_t step = (int64_t)g.dil * g.W * 32;
@@ -475,6 +478,7 @@ __global__ void __launch_bounds__(kWgGroups * 96, 1)
     const int yph = (int)(c % (unsigned)g.dil);
     c /= (unsigned)g.dil;
     const int xb = (int)(c % (unsigned)g.xchunks) * 64;
+    ragged = kRagged && xb + 64 > g.W;
     c /= (unsigned)g.xchunks;
     const int z = (int)(c % (unsigned)g.D), n = (int)(c / (unsigned)g.D);
     const int most = (int)min((unsigned)(g.nt - j0), r1 - r);
@@ -506,14 +510,14 @@ __global__ void __launch_bounds__(kWgGroups * 96, 1)
     enter();
   };
   if (u < u1) bounds();
-  // per slot: 1 a step, 2 input row, 4 dY row, 8 first of a segment, 16 last of a unit
+  // per slot: 1 a step, 2 input row, 4 dY row, 8 first of a segment, 16 last of a unit, 32 ragged
   unsigned flags = 0;
   bool first = true;
   auto stage = [&](int slot) {
     unsigned f = 0;
     if (u < u1) {
       const uint32_t at = base + slot * kWgStage;
-      f = 1u | (first ? 8u : 0u);
+      f = 1u | (first ? 8u : 0u) | (ragged ? 32u : 0u);
       first = false;
       // pieces of 16 bytes, 32 or 96 of them apart: 16 or 48 voxels, whole turns of the swizzle
       if (i + 1 < jn && !empty) {
@@ -545,7 +549,7 @@ __global__ void __launch_bounds__(kWgGroups * 96, 1)
         }
       }
     }
-    flags = (flags & ~(31u << (5 * slot))) | (f << (5 * slot));
+    flags = (flags & ~(63u << (6 * slot))) | (f << (6 * slot));
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
 
@@ -565,7 +569,7 @@ __global__ void __launch_bounds__(kWgGroups * 96, 1)
   stage(1);
   int slot = 0;
   while (true) {
-    const unsigned f = (flags >> (5 * slot)) & 31u;
+    const unsigned f = (flags >> (6 * slot)) & 63u;
     if (!(f & 1u)) break;
     asm volatile("cp.async.wait_group 1;" ::: "memory");
     // the step's rows have landed; the slot staged below was last read a step ago
@@ -601,13 +605,21 @@ __global__ void __launch_bounds__(kWgGroups * 96, 1)
         }
       }
     }
+    // A zero of dY behind the row's end may not meet the row's last voxels, of which one
+    // may be infinite: the left tap reads the zero behind them there.
+    const int len = f & 32u ? g.W & 63 : 64;
+    const uint32_t zero = sx + swz(len + g.dil, 0);
     // dY row i - 1 + k meets the input row at 1 - k along y
     auto multiply = [&](auto all) {
 #pragma unroll
       for (int ks = 0; ks < 4; ++ks) {
         uint32_t b[3][4];
 #pragma unroll
-        for (int dx = 0; dx < 3; ++dx) ldsm_x4_trans(b[dx], sx + swz(ks * 16 + vb + dx * g.dil, hb));
+        for (int dx = 0; dx < 3; ++dx) {
+          uint32_t row = sx + swz(ks * 16 + vb + dx * g.dil, hb);
+          if (kRagged && dx == 0 && ks * 16 + vb >= len) row = zero;
+          ldsm_x4_trans(b[dx], row);
+        }
 #pragma unroll
         for (int k = 0; k < 3; ++k)
           if (decltype(all)::value || (have & (1u << k)))
@@ -1132,14 +1144,15 @@ extern "C" int si_nn_conv3d_wgrad(const void* x, const void* dy, float* dw, floa
     const int64_t want = (int64_t)sm_count() * 8;
     // staged rows hold a dilation up to kWgMaxDil, and rows are counted in 32 bits
     if (dil <= kWgMaxDil && columns * nt < (int64_t)1 << 31) {
-      static std::atomic<bool> set[64];
+      static std::atomic<bool> set[2][64];
+      const bool ragged = W % 64 != 0;
+      const auto kernel = ragged ? wgrad16_columns_kernel<true> : wgrad16_columns_kernel<false>;
       int dev = 0;
       if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) dev = 0;
-      if (!set[dev].load(std::memory_order_acquire)) {
-        if (cudaFuncSetAttribute(wgrad16_columns_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kWgSmem) !=
-            cudaSuccess)
+      if (!set[ragged][dev].load(std::memory_order_acquire)) {
+        if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kWgSmem) != cudaSuccess)
           return check_launch("si_nn_conv3d_wgrad (shared memory)");
-        set[dev].store(true, std::memory_order_release);
+        set[ragged][dev].store(true, std::memory_order_release);
       }
       // units: as many sums per weight as 8 blocks per SM had (fewer, longer sums are
       // less accurate), and no more than the buffer holds
@@ -1149,7 +1162,7 @@ extern "C" int si_nn_conv3d_wgrad(const void* x, const void* dy, float* dw, floa
       const int per_group = (int)((units + groups - 1) / groups);
       const int64_t ctas = (units + (int64_t)per_group * kWgGroups - 1) / ((int64_t)per_group * kWgGroups);
       const WgGeom wg{N, D, H, W, dil, xchunks, (int)nt, (unsigned)(columns * nt), (unsigned)units};
-      wgrad16_columns_kernel<<<(unsigned)ctas, kWgGroups * 96, kWgSmem, st>>>(xb, db16, dw, db, partials, wg, per_group);
+      kernel<<<(unsigned)ctas, kWgGroups * 96, kWgSmem, st>>>(xb, db16, dw, db, partials, wg, per_group);
       if (partials) reduce_wgrad_kernel<<<(kWgOut + 31) / 32, 1024, 0, st>>>(partials, (int)units, dw, db);
       return check_launch("si_nn_conv3d_wgrad");
     }

@@ -35,3 +35,23 @@ def test_infinite_bias_gradient(shape, partials, cuda):
     d = dy.double().reshape(-1, 16)[:, rest]
     # fp32 sums of n terms: 2^-24 sqrt(n) and a factor of eight for their order
     assert bool(((gb.double()[rest] - d.sum(0)).abs() <= 8 * 2.0 ** -24 * len(d) ** 0.5 * d.abs().sum(0)).all())
+
+
+@pytest.mark.parametrize("partials", [True, False], ids=["deterministic", "atomics"])
+@pytest.mark.parametrize("shape,dil", [((1, 3, 5, 70), 1), ((2, 3, 9, 63), 2), ((1, 2, 3, 129), 8),
+                                       ((1, 4, 20, 112), 4)], ids=str)
+def test_infinite_end_of_a_row(shape, dil, partials, cuda):
+    """The tap to the left meets none of a row's last dil voxels: its sums are those
+    of a row that ends in zeros, bit for bit (but for the atomics' order)."""
+    x, dy = _bf((*shape, 16), 3), _bf((*shape, 16), 4)
+    x[..., -dil:, 6] = 0.0
+    exp, _ = _grads(x, dy, dil, partials)
+    x[..., -dil:, 6] = torch.tensor([INF, -INF, float("nan")], device="cuda").repeat(8)[:dil].to(torch.bfloat16)
+    got, _ = _grads(x, dy, dil, partials)
+    left = [t for t in range(27) if t % 3 == 0]
+    if partials:
+        assert torch.equal(got[left], exp[left])
+    else:
+        assert torch.allclose(got[left], exp[left], rtol=1e-4, atol=1e-3)
+    other = [c for c in range(16) if c != 6]
+    assert bool(torch.isfinite(got[..., other]).all()) and not bool(torch.isfinite(got[13, :, 6]).any())
