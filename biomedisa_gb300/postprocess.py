@@ -22,8 +22,9 @@ def _scratch(shape, device):
 
 
 def present_labels(labels: torch.Tensor) -> list[int]:
-    """Ascending label values present in a uint8 volume (the reference's unique())."""
-    if not labels.is_cuda:
+    """Ascending label values present in a volume (the reference's unique()). uint8
+    on the device: the histogram kernel."""
+    if not labels.is_cuda or labels.dtype != torch.uint8 or labels.numel() == 0:
         return [int(v) for v in torch.nonzero(torch.bincount(labels.reshape(-1).to(torch.int64))).flatten().tolist()]
     labels = labels.contiguous()
     hist = torch.zeros(258, dtype=torch.int64, device=labels.device)
