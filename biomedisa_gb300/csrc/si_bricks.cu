@@ -1189,8 +1189,12 @@ extern "C" int si_walk_sorted(const void* packed, int work_is_float, int Zc, int
     // do not fill the SMs once go out in small CTAs, spread more evenly; where a
     // thread for each is resident at once, each gets one, as two in a thread wait
     // for the slower of their loads: 40x36x33, 95 thousand walks, pairs in CTAs of
-    // 256 4.5 ms, of 64 4.2 ms (3.78 with the later sweeps), single 3.39 ms.
-    const bool single = mode == 1 && n0 <= resident;
+    // 256 4.5 ms, of 64 4.2 ms (3.78 with the later sweeps), single 3.39 ms. One a
+    // thread as well where walks or sweeps are no multiple of four steps: walkers off
+    // the blocks of four random words do not advance together, so two of a thread
+    // follow one another (128^3, 999 steps: uint8 24.2 and 20.7 ms, uint16 28.5 and 21.4).
+    const bool unaligned = (((uint32_t)sorw | K) & 3u) != 0u;
+    const bool single = mode == 1 && (n0 <= resident || unaligned);
     const bool few = mode == 1 && !single && n0 <= 2 * resident;
     const uint64_t per = single ? 1u : (uint64_t)mode + 1;
     const int tpb = few ? 64 : mode == 3 || single ? 128 : mode == 1 && work_is_float ? kFloatThreads : 256;
