@@ -4,8 +4,8 @@ The walker's results do not depend on these parameters (integer hit sums), only
 its speed does: the sort-brick edge (walkers are bucketed by label and brick of
 edge^3 voxels between sweeps) and the sweep length (steps per sweep launch).
 The tuner times every candidate on the caller's own volumes with shortened
-walks (2 sweeps of every walk), keeps the fastest, and caches the choice per
-workload signature in a JSON file ($SI_AUTOTUNE_CACHE or
+walks (the first PROBE_STEPS steps of every walk, the same for all), keeps the
+fastest, and caches the choice per workload signature in a JSON file ($SI_AUTOTUNE_CACHE or
 ~/.cache/biomedisa_gb300/autotune.json).
 """
 from __future__ import annotations
@@ -23,6 +23,13 @@ import torch
 from . import _native as nat
 
 CANDIDATES = ((6, 128), (8, 128), (6, 96), (6, 64))
+SHORT_WALK_DEFAULT = (6, 32)  # what the library takes for walks below 1000 steps
+PROBE_STEPS = 256
+
+
+def candidates(sorw: int) -> tuple:
+    """What is timed for walks of sorw steps: the library's own default first."""
+    return CANDIDATES if sorw >= 1000 else (SHORT_WALK_DEFAULT,) + CANDIDATES
 
 
 def cache_path() -> Path:
@@ -36,7 +43,7 @@ def signature(vols, nbrw: int, sorw: int, walks: int) -> str:
     dev = torch.cuda.get_device_name()
     kinds = sorted({int(v.work_is_float) for v in vols})
     vox = sum(v.Zc * v.Yc * v.Xc for v in vols)
-    return json.dumps([dev, CANDIDATES, kinds, len(vols), nbrw, sorw, int(math.log2(max(walks, 1))),
+    return json.dumps([dev, candidates(sorw), kinds, len(vols), nbrw, sorw, int(math.log2(max(walks, 1))),
                        int(math.log2(max(vox, 1)))])
 
 
@@ -88,8 +95,8 @@ def tune(vol_array, n_vols: int, hits: list, nbrw: int, sorw: int, key: int, wal
             return int(hit["sort_edge"]), int(hit["sweep_steps"]), {"cached": True, **hit}
     stream = torch.cuda.current_stream()
     results = []
-    for edge, steps in CANDIDATES:
-        probe = min(sorw, 2 * steps)
+    probe = min(sorw, PROBE_STEPS)
+    for edge, steps in candidates(sorw):
         need = ctypes.c_ulonglong(0)
         nat.call("si_walk_sorted_batch_scratch", vol_array, n_vols, nbrw, edge, ctypes.byref(need))
         scratch = torch.empty(max(int(need.value), 1), dtype=torch.uint8, device="cuda")
