@@ -1172,7 +1172,7 @@ extern "C" int si_walk_sorted(const void* packed, int work_is_float, int Zc, int
   const ScanArgs a{w.counts, nbt, w.offsets, w.ctrs, limit, 0, {}};
   const uint32_t K = (uint32_t)sweep_steps;
   if (cudaMemsetAsync(w.ctrs, 0, kCtrWords * sizeof(uint32_t), st) != cudaSuccess ||
-      cudaMemsetAsync(w.counts, 0, ((size_t)nbt + 1) * sizeof(uint32_t), st) != cudaSuccess)
+      cudaMemsetAsync(w.counts, 0, (size_t)nbt * sizeof(uint32_t), st) != cudaSuccess)
     return set_error(SI_ERR_CUDA, "si_walk_sorted: memset failed");
   std::vector<cudaGraphExec_t> execs;
   int rc = SI_OK;
@@ -1565,7 +1565,7 @@ extern "C" int si_walk_sorted_batch(const si_volume_t* vols, int n_vols, int nbr
   const uint32_t limit = round_limit();
   const ScanArgs a{w.counts, P.nbt, w.offsets, w.ctrs, limit, 0, {}};
   if (cudaMemsetAsync(w.ctrs, 0, kCtrWords * sizeof(uint32_t), st) != cudaSuccess ||
-      cudaMemsetAsync(w.counts, 0, ((size_t)P.nbt + 1) * sizeof(uint32_t), st) != cudaSuccess)
+      cudaMemsetAsync(w.counts, 0, (size_t)P.nbt * sizeof(uint32_t), st) != cudaSuccess)
     return set_error(SI_ERR_CUDA, "si_walk_sorted_batch: memset failed");
   std::vector<cudaGraphExec_t> execs;
   rc = run_range(
