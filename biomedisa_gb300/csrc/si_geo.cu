@@ -213,6 +213,23 @@ __host__ __device__ inline void geo_tile_row(const GeoTiling& g, int Y, int X, i
                                            floor_div(t + kTileP - 1 - vlo, step)));
 }
 
+// What tile-wavefront S launches: its rows of tiles that can hold voxels, from ir0 to
+// ir1, and the longest of them. False: no such row, and no launch.
+inline bool geo_tile_wave(const GeoTiling& g, int Y, int X, int S, int* ir0, int* ir1, int* width) {
+  *ir0 = g.ntr;
+  *ir1 = -1;
+  *width = 0;
+  for (int ir = 0; ir < g.ntr; ++ir) {
+    int lo, hi;
+    geo_tile_row(g, Y, X, S, ir, &lo, &hi);
+    if (hi < lo) continue;
+    *ir0 = imin(*ir0, ir);
+    *ir1 = ir;
+    *width = imax(*width, hi - lo + 1);
+  }
+  return *ir1 >= 0;
+}
+
 // Volume coordinates of transformed (p, q, r).
 __host__ __device__ inline void geo_unskew(const GeoTiling& g, int p, int q, int r, int* z, int* y, int* x) {
   *z = g.s * r;
@@ -727,17 +744,8 @@ int geo_launch_scan(const GeoScanArgs& a, bool lamb1, int iterations, bool tiled
       for (int fwd = 1; fwd >= 0; --fwd) {
         const GeoTiling g = geo_tiling(a.Z, a.Y, a.X, fwd);
         for (int S = 0; S <= g.ntp + g.ntq + g.ntr - 3; ++S) {
-          // rows of tiles with voxels on this wavefront, and the longest of them
-          int ir0 = g.ntr, ir1 = -1, width = 0;
-          for (int ir = 0; ir < g.ntr; ++ir) {
-            int lo, hi;
-            geo_tile_row(g, a.Y, a.X, S, ir, &lo, &hi);
-            if (hi < lo) continue;
-            ir0 = imin(ir0, ir);
-            ir1 = ir;
-            width = imax(width, hi - lo + 1);
-          }
-          if (ir1 < 0) continue;  // no voxel of the domain
+          int ir0, ir1, width;
+          if (!geo_tile_wave(g, a.Y, a.X, S, &ir0, &ir1, &width)) continue;
           if (ir1 - ir0 >= 65535) return set_error(SI_ERR_LIMIT, "si_geo_scan: too many tiles");
           // The first launch follows whatever wrote the image in full; the
           // others may read the image before the wavefront before has ended.
@@ -889,7 +897,10 @@ extern "C" int si_geo_scan_launches(int Z, int Y, int X, double lamb, int iterat
   for (int fwd = 1; fwd >= 0; --fwd) {
     if (mode == 0 || mode == 4 || mode == 5) {
       const GeoTiling g = geo_tiling(Z, Y, X, fwd);
-      n += g.ntp + g.ntq + g.ntr - 2;
+      for (int S = 0; S <= g.ntp + g.ntq + g.ntr - 3; ++S) {
+        int ir0, ir1, width;
+        n += geo_tile_wave(g, Y, X, S, &ir0, &ir1, &width);
+      }
       continue;
     }
     int t0, t1, step;

@@ -527,8 +527,8 @@ int si_geo_tile_visit_order(int Z, int Y, int X, int fwd, int32_t* wave,
 /* No counterpart in the reference (measurement).
  * Host only: *launches = the kernel launches one si_geo_scan call with these
  * arguments makes: 1 in cluster mode (which queries the current device), one
- * per tile-wavefront in the tiled modes (0, 4, 5), one per non-empty
- * wavefront in modes 1 and 3; all times `iterations` and both passes. */
+ * per tile-wavefront with a row of tiles that can hold voxels in the tiled modes
+ * (0, 4, 5), one per non-empty wavefront in modes 1 and 3; all times `iterations` and both passes. */
 int si_geo_scan_launches(int Z, int Y, int X, double lamb, int iterations,
                          int mode, long long* launches);
 
