@@ -535,6 +535,25 @@ int smooth_planes(int columns, int Zc) {
   return planes;
 }
 
+// Pairs per thread: 128-wide columns only when selected and the rows are long enough.
+int smooth_pairs(int Xc) { return g_smooth_pairs.load(std::memory_order_relaxed) == 1 || Xc <= 64 ? 1 : 2; }
+
+// The last column of a row is as narrow as what is left of the row lets it be, so
+// that a volume just above a multiple of 64 (a power of two with its padding) does
+// not pay for one of 64. A step: 130^3 16.2 and 12.7 us, 119x143x135 15.8 and 12.4,
+// 178x226x210 37.7 and 32.2, 402x514x514 294 and 258.
+SmoothColumns smooth_columns(int Yc, int Xc, int kp) {
+  SmoothColumns c{(Xc + 64 * kp - 1) / (64 * kp), (Yc + 7) / 8, 0, 0};
+  const int left = Xc % 64;
+  if (kp == 1 && left && left <= kNarrow[0]) {
+    c.kind = left <= kNarrow[1] ? 1 : 0;
+    c.nx = Xc / 64;
+    const int rows = 512 / kNarrow[c.kind];
+    c.nn = (Yc + rows - 1) / rows;
+  }
+  return c;
+}
+
 // One smoothing step, allowed to start while the step before it drains: its
 // CTAs set up their barriers and wait (griddepcontrol.wait) before they touch
 // the maps. 42x38x35 7.8 -> 5.4 us a step, 130^3 20.0 -> 17.2.
@@ -565,21 +584,8 @@ int smooth_maps(void* maps, float* tmp0, float* tmp1, int nol, int Zc, int Yc, i
   float* tmp1v = tmp1 + kHeadFloats;
   if (iters > 0 && ((reinterpret_cast<uintptr_t>(tmp0) | reinterpret_cast<uintptr_t>(tmp1)) & 15u))
     return set_error(SI_ERR_ARG, "%s: tmp0/tmp1 must be 16-byte aligned", what);
-  // pairs per thread: 128-wide columns only when selected and the rows are long enough
-  const int kp = g_smooth_pairs.load(std::memory_order_relaxed) == 1 || Xc <= 64 ? 1 : 2;
-  const int sx = 64 * kp;
-  // The last column of a row is as narrow as what is left of the row lets it be, so
-  // that a volume just above a multiple of 64 (a power of two with its padding) does
-  // not pay for one of 64. A step: 130^3 16.2 and 12.7 us, 119x143x135 15.8 and 12.4,
-  // 178x226x210 37.7 and 32.2, 402x514x514 294 and 258.
-  SmoothColumns c{(Xc + sx - 1) / sx, (Yc + 7) / 8, 0, 0};
-  const int left = Xc % 64;
-  if (kp == 1 && left && left <= kNarrow[0]) {
-    c.kind = left <= kNarrow[1] ? 1 : 0;
-    c.nx = Xc / 64;
-    const int rows = 512 / kNarrow[c.kind];
-    c.nn = (Yc + rows - 1) / rows;
-  }
+  const int kp = smooth_pairs(Xc), sx = 64 * kp;
+  const SmoothColumns c = smooth_columns(Yc, Xc, kp);
   CUtensorMap map0{}, map1{}, nmap0{}, nmap1{};
   if (iters > 0) {
     int rc = encode_volume_map(&map0, tmp0, Zc, Yc, Xc, sx + 8, 10, what);
@@ -674,6 +680,14 @@ extern "C" int si_smooth_f32(float* maps, float* tmp0, float* tmp1, int nol, int
   const int rc = smooth_args(maps, tmp0, tmp1, nol, Zc, Yc, Xc, iters, update, "si_smooth_f32");
   if (rc) return rc;
   return smooth_maps<false>(maps, tmp0, tmp1, nol, Zc, Yc, Xc, iters, update, as_stream(stream), "si_smooth_f32");
+}
+
+extern "C" int si_smooth_planes(int Zc, int Yc, int Xc, int* planes) {
+  clear_error();
+  if (!planes || Zc < 1 || Yc < 1 || Xc < 1) return set_error(SI_ERR_ARG, "si_smooth_planes: bad arguments");
+  const SmoothColumns c = smooth_columns(Yc, Xc, smooth_pairs(Xc));
+  *planes = smooth_planes(c.nx * c.ny + c.nn, Zc);
+  return SI_OK;
 }
 
 extern "C" int si_smooth_set_pairs(int pairs) {

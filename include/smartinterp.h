@@ -364,6 +364,11 @@ int si_smooth_f32(float* maps, float* tmp0, float* tmp1, int nol, int Zc,
  * the reference. */
 int si_smooth_status(int* status, void* stream);
 
+/* *planes = the planes of a map that a CTA of one smoothing step marches through on
+ * the current device (2, 4, 8, 16 or 32, by the number of columns and planes). No
+ * counterpart in the reference (measurement). */
+int si_smooth_planes(int Zc, int Yc, int Xc, int* planes);
+
 /* Voxels per thread of the smoothing kernel: pairs = 1 (default) gives each
  * thread two voxels of a 64-wide column, 2 four voxels of a 128-wide one
  * (faster on dense maps, slower on sparse hit maps). Process-wide; speed
