@@ -42,8 +42,37 @@ struct CcInfo {
 struct Words {
   int Z, Y, X, W;
   uint32_t n;  // Z * Y * W, at most 2^31 - 1
+  int lanes, lg;  // lanes (a power of two) of a warp that take a word together
   FastDiv by_W, by_Y;
 };
+
+// A lane's place among words that a warp takes `lanes` lanes each: 32, and so one
+// word a warp, but for rows of 16 voxels and less (kShort), of which it takes
+// several (clean of 3000x700x3 noise took 1.60 ms a word a warp, 0.55 ms so).
+template <bool kShort>
+struct WordLane {
+  int sub, first;  // lane within the word, first lane of the word
+  int lg;
+  unsigned low;    // the word's bits
+  __device__ __forceinline__ explicit WordLane(const Words& g) {
+    const int lane = threadIdx.x & 31, lanes = kShort ? g.lanes : 32;
+    lg = kShort ? g.lg : 5;
+    sub = lane & (lanes - 1);
+    first = lane - sub;
+    low = 0xFFFFFFFFu >> (32 - lanes);
+  }
+  __device__ __forceinline__ unsigned ballot(bool p) const { return (__ballot_sync(0xffffffffu, p) >> first) & low; }
+};
+
+// f(i, i < g.n) for the words of a warp, whole warps together.
+template <bool kShort, class F>
+__device__ __forceinline__ void for_word_lanes(const Words& g, const WordLane<kShort>& l, F f) {
+  const uint32_t stride = (gridDim.x * blockDim.x) >> l.lg;
+  for (uint32_t i0 = ((blockIdx.x * blockDim.x + threadIdx.x) & ~31u) >> l.lg; i0 < g.n; i0 += stride) {
+    const uint32_t i = i0 + ((uint32_t)l.first >> l.lg);
+    f(i, !kShort || i < g.n);
+  }
+}
 
 __device__ __forceinline__ int uf_find(const int* L, int p) {
   const volatile int* vl = L;
@@ -110,58 +139,57 @@ __device__ __forceinline__ int start_of(const unsigned* __restrict__ row, int w,
   return 32 * w + 31 - __clz(m);
 }
 
-// One warp per word.
+template <bool kShort>
 __global__ void __launch_bounds__(256) clean_starts_kernel(const uint8_t* __restrict__ lab, Words g, int skip,
                                                            unsigned* __restrict__ starts, int* __restrict__ L,
                                                            unsigned* __restrict__ size) {
-  const int lane = threadIdx.x & 31;
-  const uint32_t stride = gridDim.x * (blockDim.x >> 5);
-  for (uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < g.n; i += stride) {
-    const int64_t r = g.by_W(i);
-    const int w = (int)(i - (uint32_t)r * (uint32_t)g.W), x = 32 * w + lane;
+  const WordLane<kShort> l(g);
+  for_word_lanes(g, l, [&](uint32_t i, bool has) {
+    const int64_t r = has ? g.by_W(i) : 0u;
+    const int w = (int)(i - (uint32_t)r * (uint32_t)g.W), x = 32 * w + l.sub;
     const int64_t v = r * g.X + x;
-    const bool in = x < g.X;
+    const bool in = has && x < g.X;
     const int c = in ? lab[v] : -1;
     int left = __shfl_up_sync(0xffffffffu, c, 1);
-    if (lane == 0) left = w ? lab[v - 1] : -1;
+    if (l.sub == 0) left = in && w ? lab[v - 1] : -1;
     const bool first = in && c != left;
-    const unsigned m = __ballot_sync(0xffffffffu, first);
-    if (lane == 0) starts[i] = m;
+    const unsigned m = l.ballot(first);
+    if (l.sub == 0 && has) starts[i] = m;
     if (first && c != skip) {
       L[v] = (int)v;
       size[v] = 0u;
     }
-  }
+  });
 }
 
-// One warp per word: a lane merges where its run and the neighbouring row's
-// begin to overlap.
+// A lane merges where its run and the neighbouring row's begin to overlap.
+template <bool kShort>
 __global__ void __launch_bounds__(256) clean_merge_kernel(const uint8_t* __restrict__ lab, Words g, int skip,
                                                           const unsigned* __restrict__ starts, int* L) {
-  const int lane = threadIdx.x & 31;
-  const uint32_t stride = gridDim.x * (blockDim.x >> 5);
-  for (uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < g.n; i += stride) {
-    const int64_t r = g.by_W(i);
-    const int w = (int)(i - (uint32_t)r * (uint32_t)g.W), x = 32 * w + lane;
+  const WordLane<kShort> l(g);
+  for_word_lanes(g, l, [&](uint32_t i, bool has) {
+    const int64_t r = has ? g.by_W(i) : 0u;
+    const int w = (int)(i - (uint32_t)r * (uint32_t)g.W), x = 32 * w + l.sub;
     const int64_t v = r * g.X + x;
-    const bool in = x < g.X;
+    const bool in = has && x < g.X;
     const int c = in ? lab[v] : skip;
-    const unsigned m = starts[i];
+    const unsigned m = has ? starts[i] : 0u;
     const int y = (int)((uint32_t)r - g.by_Y((uint32_t)r) * (uint32_t)g.Y);
 #pragma unroll
     for (int dir = 0; dir < 2; ++dir) {
-      if (dir == 0 ? y == 0 : r < g.Y) continue;  // the same for the whole warp
+      const bool row = dir == 0 ? y > 0 : r >= g.Y;
+      if (!__any_sync(0xffffffffu, row)) continue;
       const int64_t dr = dir == 0 ? 1 : g.Y, dv = dr * g.X;
-      const bool eq = in && c != skip && lab[v - dv] == c;
-      const unsigned e = __ballot_sync(0xffffffffu, eq);
-      bool left = lane ? (e >> (lane - 1)) & 1u : false;
-      // lane 0 of a run that comes from the word before
-      if (lane == 0 && eq && !(m & 1u)) left = lab[v - dv - 1] == c;
-      if (eq && (((m >> lane) & 1u) || !left))
-        uf_merge(L, (int)(r * g.X) + start_of(starts + r * g.W, w, lane),
-                 (int)((r - dr) * g.X) + start_of(starts + (r - dr) * g.W, w, lane));
+      const bool eq = in && row && c != skip && lab[v - dv] == c;
+      const unsigned e = l.ballot(eq);
+      bool left = l.sub ? (e >> (l.sub - 1)) & 1u : false;
+      // the first voxel of a word, in a run that comes from the word before
+      if (l.sub == 0 && eq && !(m & 1u)) left = lab[v - dv - 1] == c;
+      if (eq && (((m >> l.sub) & 1u) || !left))
+        uf_merge(L, (int)(r * g.X) + start_of(starts + r * g.W, w, l.sub),
+                 (int)((r - dr) * g.X) + start_of(starts + (r - dr) * g.W, w, l.sub));
     }
-  }
+  });
 }
 
 // One thread per word.
@@ -222,28 +250,28 @@ __global__ void __launch_bounds__(256) clean_max_kernel(const uint8_t* __restric
 }
 
 // remove_outlier.py:85-97: keep components with size > threshold * largest
-// (one warp per word)
+template <bool kShort>
 __global__ void __launch_bounds__(256) clean_write_kernel(const uint8_t* __restrict__ lab, Words g, int skip,
                                                           const unsigned* __restrict__ starts,
                                                           const int* __restrict__ L,
                                                           const unsigned* __restrict__ size,
                                                           const unsigned* __restrict__ big, double threshold,
                                                           uint8_t* __restrict__ out) {
-  const int lane = threadIdx.x & 31;
-  const uint32_t stride = gridDim.x * (blockDim.x >> 5);
-  for (uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < g.n; i += stride) {
+  const WordLane<kShort> l(g);
+  for_word_lanes(g, l, [&](uint32_t i, bool has) {
+    if (!has) return;
     const int64_t r = g.by_W(i);
-    const int w = (int)(i - (uint32_t)r * (uint32_t)g.W), x = 32 * w + lane;
-    if (x >= g.X) continue;
+    const int w = (int)(i - (uint32_t)r * (uint32_t)g.W), x = 32 * w + l.sub;
+    if (x >= g.X) return;
     const int64_t v = r * g.X + x;
     const int c = lab[v];
     bool keep = true;
     if (c != skip) {
-      const int root = L[(int)(r * g.X) + start_of(starts + r * g.W, w, lane)];
+      const int root = L[(int)(r * g.X) + start_of(starts + r * g.W, w, l.sub)];
       keep = (double)size[root] > threshold * (double)big[c];
     }
     out[v] = keep ? (uint8_t)c : (uint8_t)0;
-  }
+  });
 }
 
 // ---- fill: one label at a time inside its grown bounding box ----
@@ -520,12 +548,22 @@ __global__ void __launch_bounds__(256) fill_write_kernel(uint8_t* img, Words g, 
 }
 
 Words words_of(int Z, int Y, int X) {
+  // One voxel a row: the rows of a plane are a row (same voxels in the same order,
+  // same neighbours), and so for planes of one row.
+  for (int k = 0; k < 2 && X == 1; ++k) {
+    X = Y;
+    Y = Z;
+    Z = 1;
+  }
   Words g{};
   g.Z = Z;
   g.Y = Y;
   g.X = X;
   g.W = (X + 31) / 32;
   g.n = (uint32_t)((int64_t)Z * Y * g.W);
+  g.lg = 5;
+  while (g.lg > 0 && (1 << (g.lg - 1)) >= X) --g.lg;
+  g.lanes = 1 << g.lg;
   g.by_W = FastDiv((uint32_t)g.W);
   g.by_Y = FastDiv((uint32_t)Y);
   return g;
@@ -582,14 +620,18 @@ extern "C" int si_clean(const uint8_t* labels, uint8_t* out, int Z, int Y, int X
   const Words g = words_of(Z, Y, X);
   const CcScratch c(scratch, g);
   cudaStream_t st = as_stream(stream);
-  const int per_warp = grid_for((int64_t)g.n * 32), per_thread = grid_for(g.n);
+  const int per_warp = grid_for((int64_t)g.n * g.lanes), per_thread = grid_for(g.n);
   if (cudaMemsetAsync(c.big, 0, 256 * sizeof(unsigned), st) != cudaSuccess)
     return set_error(SI_ERR_CUDA, "si_clean: memset failed");
-  clean_starts_kernel<<<per_warp, 256, 0, st>>>(labels, g, skip_label, c.words, c.L, c.size);
-  clean_merge_kernel<<<per_warp, 256, 0, st>>>(labels, g, skip_label, c.words, c.L);
+  const bool sh = g.lanes < 32;
+  (sh ? clean_starts_kernel<true> : clean_starts_kernel<false>)<<<per_warp, 256, 0, st>>>(labels, g, skip_label,
+                                                                                          c.words, c.L, c.size);
+  (sh ? clean_merge_kernel<true> : clean_merge_kernel<false>)<<<per_warp, 256, 0, st>>>(labels, g, skip_label, c.words,
+                                                                                        c.L);
   clean_count_kernel<<<per_thread, 256, 0, st>>>(labels, g, skip_label, c.words, c.L, c.size);
   clean_max_kernel<<<per_thread, 256, 0, st>>>(labels, g, skip_label, c.words, c.L, c.size, c.big);
-  clean_write_kernel<<<per_warp, 256, 0, st>>>(labels, g, skip_label, c.words, c.L, c.size, c.big, threshold, out);
+  (sh ? clean_write_kernel<true> : clean_write_kernel<false>)<<<per_warp, 256, 0, st>>>(
+      labels, g, skip_label, c.words, c.L, c.size, c.big, threshold, out);
   return check_launch("si_clean");
 }
 
@@ -601,7 +643,7 @@ extern "C" int si_fill(uint8_t* img, int Z, int Y, int X, double threshold, cons
   const Words g = words_of(Z, Y, X);
   const CcScratch c(scratch, g);
   cudaStream_t st = as_stream(stream);
-  const int mask_grid = std::min(grid_for((int64_t)Z * Y * 32), sm_count() * 8), per_thread = grid_for(g.n);
+  const int mask_grid = std::min(grid_for((int64_t)g.Z * g.Y * 32), sm_count() * 8), per_thread = grid_for(g.n);
   for (int i = 0; i < n_labels; ++i) {
     const int k = label_list[i];
     if (k < 0 || k > 255) return set_error(SI_ERR_ARG, "si_fill: label %d outside 0..255", k);
