@@ -6,6 +6,7 @@
 // coordinates outside it as zero.
 #include <cfloat>
 #include <climits>
+#include <type_traits>
 
 #include "si_common.cuh"
 #include "si_internal.h"
@@ -129,33 +130,36 @@ __device__ __forceinline__ bool survives(const V& lv, int z, int y, int x, int r
   return ones1(lv, z - cz, y - cy, x - cx, rz, ry, rx) || ones1(lv, z + cz, y + cy, x + cx, rz, ry, rx);
 }
 
-template <typename T>
+template <typename T, bool kShort>
 __global__ void __launch_bounds__(256) slice_flags_kernel(const T* __restrict__ lab, int Z0, int Y0, int X0,
                                                           const uint8_t* __restrict__ nz_lut_g, int allaxis,
                                                           uint8_t* __restrict__ fz, uint8_t* __restrict__ fy,
-                                                          uint8_t* __restrict__ fx, int32_t* __restrict__ bbox) {
+                                                          uint8_t* __restrict__ fx, int32_t* __restrict__ bbox,
+                                                          int lg_short) {
   __shared__ uint8_t lut[256];
   for (int i = threadIdx.x; i < 256; i += blockDim.x) lut[i] = nz_lut_g[i];
   __syncthreads();
   LabelView<T> lv{lab, lut, Z0, Y0, X0, allaxis != 2};
   int bmin[3] = {INT_MAX, INT_MAX, INT_MAX};
   int bmax[3] = {-1, -1, -1};
-  // a warp per x-row, four loads in flight a lane (a thread per voxel spent its
+  // a warp per x-row, or 2^lg_short lanes (compiled apart: 694 and 742 us for the analysis
+  // of 64x1024x1024 int32 with all axes), four loads in flight a lane (a thread per voxel spent its
   // time on the divisions of a 64-bit index: 88 us on 192x256x250 uint8)
+  const int lg = kShort ? lg_short : 5;
   const uint64_t rows = (uint64_t)Z0 * Y0;
-  const uint64_t stride = (uint64_t)gridDim.x * (blockDim.x >> 5);
-  const int lane = threadIdx.x & 31;
-  for (uint64_t row = (uint64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); row < rows; row += stride) {
+  const uint64_t stride = (uint64_t)gridDim.x * (blockDim.x >> lg);
+  const int lane = threadIdx.x & ((1 << lg) - 1);
+  for (uint64_t row = (uint64_t)blockIdx.x * (blockDim.x >> lg) + (threadIdx.x >> lg); row < rows; row += stride) {
     const int z = (int)(row / (unsigned)Y0), y = (int)(row - (uint64_t)z * Y0);
     const int pz = z + 1, py = y + 1;  // padded coordinates
     const T* at = lab + row * X0;
-    for (int x0 = lane; x0 < X0; x0 += 128) {
+    for (int x0 = lane; x0 < X0; x0 += 4 << lg) {
       int v[4];
 #pragma unroll
-      for (int k = 0; k < 4; ++k) v[k] = x0 + 32 * k < X0 ? load_label(at, (uint64_t)(x0 + 32 * k)) : 256;
+      for (int k = 0; k < 4; ++k) v[k] = x0 + (k << lg) < X0 ? load_label(at, (uint64_t)(x0 + (k << lg))) : 256;
 #pragma unroll
       for (int k = 0; k < 4; ++k) {
-        const int x = x0 + 32 * k, px = x + 1;
+        const int x = x0 + (k << lg), px = x + 1;
         if (!lv.set(v[k])) continue;
         bmin[0] = min(bmin[0], pz); bmax[0] = max(bmax[0], pz);
         bmin[1] = min(bmin[1], py); bmax[1] = max(bmax[1], py);
@@ -388,20 +392,26 @@ extern "C" int si_slice_flags(const void* labels, int dtype, int Z0, int Y0, int
   if (allaxis < 0 || allaxis > 2) return set_error(SI_ERR_ARG, "si_slice_flags: allaxis must be 0, 1 or 2");
   if (allaxis && (!flags_y || !flags_x)) return set_error(SI_ERR_ARG, "si_slice_flags: allaxis needs flags_y/flags_x");
   if (Z0 <= 0 || Y0 <= 0 || X0 <= 0) return set_error(SI_ERR_ARG, "si_slice_flags: bad dims");
-  const int block = 256, grid = grid_for((uint64_t)Z0 * Y0, block / 32);
+  // a warp per row; fewer lanes for rows shorter than 17 voxels, most of a warp idling
+  // on them (3000x700x3, all axes: the job's analysis 0.92 ms, 0.38 so)
+  int lg = 5;
+  while (lg > 0 && (1 << (lg - 1)) >= X0) --lg;
+  const int block = 256, grid = grid_for((uint64_t)Z0 * Y0, block >> lg);
   cudaStream_t st = as_stream(stream);
+  const auto run = [&](auto* lab) {
+    using T = std::remove_const_t<std::remove_pointer_t<decltype(lab)>>;
+    (lg < 5 ? slice_flags_kernel<T, true> : slice_flags_kernel<T, false>)<<<grid, block, 0, st>>>(
+        lab, Z0, Y0, X0, nz_lut, allaxis, flags_z, flags_y, flags_x, bbox, lg);
+  };
   switch (dtype) {
     case SI_U8:
-      slice_flags_kernel<<<grid, block, 0, st>>>(static_cast<const uint8_t*>(labels), Z0, Y0, X0, nz_lut, allaxis,
-                                                 flags_z, flags_y, flags_x, bbox);
+      run(static_cast<const uint8_t*>(labels));
       break;
     case SI_I16:
-      slice_flags_kernel<<<grid, block, 0, st>>>(static_cast<const int16_t*>(labels), Z0, Y0, X0, nz_lut, allaxis,
-                                                 flags_z, flags_y, flags_x, bbox);
+      run(static_cast<const int16_t*>(labels));
       break;
     case SI_I32:
-      slice_flags_kernel<<<grid, block, 0, st>>>(static_cast<const int32_t*>(labels), Z0, Y0, X0, nz_lut, allaxis,
-                                                 flags_z, flags_y, flags_x, bbox);
+      run(static_cast<const int32_t*>(labels));
       break;
     default:
       return set_error(SI_ERR_ARG, "si_slice_flags: unsupported label dtype %d", dtype);
