@@ -318,13 +318,6 @@ __global__ void __launch_bounds__(kTileThreads) geo_tile_kernel(GeoScanArgs a, G
   int iq, iq_hi;
   geo_tile_row(g, a.Y, a.X, S, ir, &iq, &iq_hi);
   iq += (int)blockIdx.x;
-  // Every CTA waits for the wavefront before, those without a voxel too: a wavefront of
-  // a thin volume may have no others (12x3x3, S = 1), and the one after it waits for
-  // this grid alone, so this grid must not end before the one before it.
-  if (iq > iq_hi) {  // uniform over the CTA
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    return;
-  }
   const int ip = S - iq - ir;
   float* cl = a.c + (long long)blockIdx.z * a.V;
   const int cq = threadIdx.x % kTileQ, cr = threadIdx.x / kTileQ;
@@ -334,15 +327,16 @@ __global__ void __launch_bounds__(kTileThreads) geo_tile_kernel(GeoScanArgs a, G
   int k_lo = g.s > 0 ? 1 - x0 : x0 - (a.X - 2), k_hi = g.s > 0 ? a.X - 2 - x0 : x0 - 1;
   k_lo = imax(k_lo, 0);
   k_hi = imin(k_hi, kTileP - 1);
-  if (z < g.zlo || z > g.zhi || y < 1 || y > a.Y - 2) k_hi = -1;
-  if (!__syncthreads_or(k_lo <= k_hi)) {  // no voxel of the domain in this tile
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    return;
-  }
+  if (iq > iq_hi || z < g.zlo || z > g.zhi || y < 1 || y > a.Y - 2) k_hi = -1;
+  const bool any = __syncthreads_or(k_lo <= k_hi);
   const int p0 = g.pb + ip * kTileP - 7, q0 = g.qb + iq * kTileQ - 3, r0 = g.rb + ir * kTileR - 1;
-  geo_stage_box(a, g, a.img, si, p0, q0, r0);
-  // the wavefront before has written its distances; the next may start on its image
+  if (any) geo_stage_box(a, g, a.img, si, p0, q0, r0);
+  // The wavefront before has written its distances; the next may start on its image.
+  // Tiles without a voxel of the domain wait too: a wavefront of a thin volume may have
+  // no others (12x3x3, S = 1), and the one after it waits for this grid alone, so this
+  // grid must not end before the one before it.
   asm volatile("griddepcontrol.wait;" ::: "memory");
+  if (!any) return;
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   geo_stage_box(a, g, cl, sc, p0, q0, r0);
   asm volatile("cp.async.wait_all;" ::: "memory");
