@@ -86,7 +86,11 @@ WORKLOADS = {
 # one kernel per entry-point call except these (launches per call)
 MULTI_LAUNCH = {"si_extract_seeds": 3, "si_nn_conv3d_wgrad": 2, "si_nn_xent": 2}
 
-WALK_SECTORS_L2 = 2  # per walker step at L2: one packed-record sector + one atomic sector
+# Per walker step at L2, from the committed ncu summary of a sweep: 0.58 sectors read
+# (records that miss L1) and 1.21 added to (0.84 hit atomics: returns are merged;
+# an addition to the far die's half of L2 passes both)
+WALK_SECTORS_L2 = 1.79
+WALK_ATOMICS = 0.84
 WALK_BYTES_PAYLOAD_U8 = 10  # 6 neighbour bytes + one 4-byte hit per step
 
 
@@ -459,12 +463,13 @@ def main():
         "gpu_launches": launches // max(args.steps, 1),
         "roofline": {"bound": "l2", "achieved": achieved_l2, "peak": l2_gbs, "unit": "GB/s",
                      "frac": achieved_l2 / l2_gbs if l2_gbs else None, "traffic": traffic,
-                     "atomics_per_s": walk_rate, "atomic_peak_per_s": l2["atomics_per_s"],
-                     "atomic_frac": walk_rate / l2["atomics_per_s"] if l2.get("atomics_per_s") else None,
+                     "atomics_per_s": WALK_ATOMICS * walk_rate, "atomic_peak_per_s": l2["atomics_per_s"],
+                     "atomic_frac": WALK_ATOMICS * walk_rate / l2["atomics_per_s"] if l2.get("atomics_per_s") else None,
                      "note": f"walker (sorted-sweep kernel, two walkers per thread, {sweeps} sweeps per job on "
                              "the device-side loop), issue- and L2-bound: "
-                             f"{WALK_SECTORS_L2} x 32 B sectors per step at L2 (one packed neighbourhood record "
-                             "+ one hit atomic) x steps / CUDA-event walk duration; peak = L2 read ceiling "
+                             f"{WALK_SECTORS_L2} x 32 B sectors per step at L2 (records that miss L1, and hit "
+                             f"atomics: {WALK_ATOMICS} per step, most of them passing both halves of L2; from the "
+                             "committed ncu summary) x steps / CUDA-event walk duration; peak = L2 read ceiling "
                              "measured in this run by si_probe_l2_read over a 48 MiB L2-resident buffer (no L2 "
                              "figure in the measured-peaks file); atomic peak = si_probe_l2_atomics; traffic = "
                              f"DRAM bytes per sweep launch from the committed ncu summary ({traffic_per_step} "

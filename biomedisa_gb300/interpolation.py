@@ -461,13 +461,9 @@ class DeviceJob:
             self.rounds = walk_sorted(self.packed, self.work_is_float, cp.Zc, cp.Yc, cp.Xc, self.seeds,
                                       self.n_seeds, self.seed_capacity, self.nbrw, self.sorw, self.rng_seed,
                                       self.hits, nol, self.sweep_steps, self.sort_edge)
-            # per sweep: scatter, sweep and the scan's kernels (one of them for up
-            # to 16384 buckets, else three); count and scan before the first. The
-            # default edge is 4 to 8 by the walks per brick and bucket
-            edge = self.sort_edge or 6
-            buckets = nol * -(-cp.Zc // edge) * -(-cp.Yc // edge) * -(-cp.Xc // edge)
-            scans = 1 if buckets <= 16384 else 3
-            self.launches += (2 + scans) * self.rounds + 1 + scans
+            # at least: per sweep a scatter, a sweep and the scan, which is one kernel or,
+            # above 16384 buckets, three; a count and a scan before the first
+            self.launches += 3 * self.rounds + 2
             return
         nat.call("si_walk", _ptr(self.packed), int(self.work_is_float), cp.Zc, cp.Yc, cp.Xc, _ptr(self.seeds),
                  _ptr(self.n_seeds), self.seed_capacity, self.nbrw, self.sorw, self.rng_seed, _ptr(self.hits), nol,
