@@ -727,11 +727,17 @@ constexpr uint64_t kBatchWalks = 1ull << 25;  // default walks per seed range of
 constexpr int kSortEdge = 6;  // of batches
 constexpr int kMinSortEdge = 4, kMaxSortEdge = 8;
 constexpr double kBrickWalks = 160.0, kBucketWalks = 20.0;
-// Default sweep length: 32 steps, 128 for walks of kLongWalk steps and more.
-// Longer sweeps share the sort's cost among more steps, but let the walkers
+// Default sweep length: 128 steps for walks of kLongWalk steps and more, 32 for shorter
+// ones. Longer sweeps share the sort's cost among more steps, but let the walkers
 // spread further between sorts. Walks of 4000 steps, 48 / 64 / 96 / 128 / 256
 // steps a sweep: 128^3 44.4 / 43.2 / 42.0 / 41.4 / 42.0 ms, 419x492x462 873 /
-// 855 / 838 / 834 / 843 ms.
+// 855 / 838 / 834 / 843 ms. Speed does not put the line at kLongWalk: 128 steps are the
+// fastest at every length. 32 / 64 / 128 / 256 steps a sweep, 240x250x230 uint8: walks of
+// 252 steps 18.3 / 17.2 / 16.6 / 17.0 ms, 500 36.1 / 33.5 / 32.4 / 33.0, 1000 71.9 / 66.9 /
+// 64.3 / 65.4, 2000 143 / 133 / 128 / 130 (uint16 alike; 40x36x33, 500 steps 0.58 / 0.48 /
+// 0.45 / 0.42). Below it the default stays the 32 steps that callers who count sweeps or
+// limit their number (si_walk_sorted_set_round_limit) know; sweep_steps = 128 gains 8 to
+// 11 % there, and the batch tuner tries it.
 constexpr int kLongWalk = 1000;
 int default_sweep_steps(int sorw) { return sorw >= kLongWalk ? 128 : 32; }
 std::atomic<unsigned long long> g_range_walks{0};  // 0 = kBatchWalks (si_walk_sorted_set_range)

@@ -306,9 +306,9 @@ __device__ __forceinline__ void geo_stage_box(const GeoScanArgs& a, const GeoTil
 // other ten neighbours are values that moved through registers (three per
 // neighbour column, one new load per column and plane); their minimum is formed
 // before the barrier. Boxes come by asynchronous copies, the image's while the
-// wavefront before still runs (programmatic launch). 7.3 us per tile-wavefront;
-// 23.5 us with 26 loads and the index arithmetic of every voxel behind the
-// barrier. Both loops are unrolled in full (8.3 us by three and four).
+// wavefront before still runs (programmatic launch). 6.6 us per tile-wavefront in a
+// replayed graph; 23.5 us with 26 loads and the index arithmetic of every voxel behind the
+// barrier. Both loops are unrolled in full (a microsecond more by three and four).
 template <bool kLamb1>
 __global__ void __launch_bounds__(kTileThreads) geo_tile_kernel(GeoScanArgs a, GeoTiling g, int S, int ir0) {
   extern __shared__ float smem[];

@@ -163,7 +163,8 @@ __global__ void __launch_bounds__(256) remap_kernel(uint8_t* __restrict__ out, P
 // a plane step loads 9 values per voxel from shared memory. Instructions bound
 // it on large volumes (issue 79 % busy at 139 per voxel); unrolled by three, so
 // that the planes' registers change roles instead of being moved, 121 per voxel:
-// 402x514x514 441 -> 422 us dense, 373 -> 361 us on a hit map.
+// 402x514x514 441 -> 422 us dense, 373 -> 361 us on a hit map (258 us with the narrow last
+// columns and 16 planes of now: 93 per voxel of a sparse map, issue 66 % busy).
 //
 // Support box: values outside the box of non-(+0) source values grown by
 // one voxel per iteration are exactly +0 (all differences +0, kappa =
