@@ -827,8 +827,8 @@ __global__ void __launch_bounds__(256) xent_kernel(const float* __restrict__ log
 // The gradient takes xent_kernel's operations, bit for bit. The loss takes log1pf
 // (__logf is off by up to 2^-21 where a voxel is sure of its label, and that does
 // not average out), one binary64 addition per voxel, and a fixed order: CTA sums
-// leave through the first eight bytes of the gradient of the CTA's first voxel,
-// where xent16_loss_kernel finds them, adds them up and puts the gradient back.
+// leave through the first half of the gradient of the CTA's first voxel, where
+// xent16_loss_kernel finds them, adds them up and puts the gradient back.
 // Off the 64-bit sum by at most 1e-7 then; by up to 9e-7, another amount in each run,
 // with the CTAs' sums added to the loss in binary32 (83 us), and by up to 6e-6 with
 // one such addition per warp, as in xent_kernel. Nothing is compensated, so an
@@ -908,7 +908,9 @@ __global__ void __launch_bounds__(kXentThreads) xent16_kernel(const float* __res
     o[1] = grad[1];
   }
   sum = cta_sum(sum, s_warp);
-  if (threadIdx.x == 0) *reinterpret_cast<double*>(dlogits + first * 16) = sum;
+  if (threadIdx.x == 0)  // as uint4, like the gradient that it takes the place of
+    *reinterpret_cast<uint4*>(dlogits + first * 16) =
+        make_uint4((uint32_t)__double2loint(sum), (uint32_t)__double2hiint(sum), 0u, 0u);
 }
 
 // The sums of the n CTAs, whose first voxels' gradients are restored.
@@ -921,10 +923,11 @@ __global__ void __launch_bounds__(1024) xent16_loss_kernel(const float* __restri
   double sum = 0.0;
   for (int b = threadIdx.x; b < n; b += blockDim.x) {
     const int64_t v = (int64_t)b * kXentThreads;
-    sum += *reinterpret_cast<const double*>(dlogits + v * 16);
+    uint4* half = reinterpret_cast<uint4*>(dlogits + v * 16);
+    sum += __hiloint2double((int)half->y, (int)half->x);
     uint4 grad[2];
     xent16_voxel(logits + v * 16, target + v * nol, weight ? weight[v] : 1.0f, nol, scale, grad);
-    reinterpret_cast<uint4*>(dlogits + v * 16)[0] = grad[0];
+    *half = grad[0];
   }
   sum = cta_sum(sum, s_warp);
   if (threadIdx.x == 0) atomicAdd(loss, (float)sum);
