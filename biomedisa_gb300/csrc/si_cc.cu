@@ -151,7 +151,7 @@ __global__ void __launch_bounds__(256) clean_starts_kernel(const uint8_t* __rest
     const bool in = has && x < g.X;
     const int c = in ? lab[v] : -1;
     int left = __shfl_up_sync(0xffffffffu, c, 1);
-    if (l.sub == 0) left = in && w ? lab[v - 1] : -1;
+    if (l.sub == 0) left = w ? lab[v - 1] : -1;  // short rows have one word
     const bool first = in && c != left;
     const unsigned m = l.ballot(first);
     if (l.sub == 0 && has) starts[i] = m;
@@ -178,7 +178,7 @@ __global__ void __launch_bounds__(256) clean_merge_kernel(const uint8_t* __restr
 #pragma unroll
     for (int dir = 0; dir < 2; ++dir) {
       const bool row = dir == 0 ? y > 0 : r >= g.Y;
-      if (!__any_sync(0xffffffffu, row)) continue;
+      if (kShort ? !__any_sync(0xffffffffu, row) : !row) continue;  // the same for the whole warp
       const int64_t dr = dir == 0 ? 1 : g.Y, dv = dr * g.X;
       const bool eq = in && row && c != skip && lab[v - dv] == c;
       const unsigned e = l.ballot(eq);
