@@ -25,7 +25,7 @@
 // falls in the ring (results do not depend on the grid). The regions of consecutive
 // inputs overlap, and no wait lies between their MMAs: one thread's MMAs keep their
 // order there too (promised by PTX for the same accumulator and shape only; no
-// different bit in 1.5 million convolutions, and waiting for each input's MMAs changed
+// different bit in 3.4 million convolutions, and waiting for each input's MMAs changed
 // nothing and cost 5 to 7 %). Every MMA accumulates; the epilogue zeroes a position's slot (tcgen05.st) after
 // reading it and before releasing it, and all slots start zeroed.
 //
@@ -652,7 +652,7 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm)
       // the fence orders the reads before the copy that refills it. (Released with the
       // position, its loads still on their way, the slot was refilled under them once in
       // some thousand convolutions: up to 32 voxels of a row with another row's residual.
-      // None in 800 thousand so, at the same speed.)
+      // None in 2.7 million so, at the same speed.)
       if (has_res) {
         fence_proxy_async_shared();
         __syncwarp();
